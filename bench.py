@@ -79,9 +79,7 @@ COMPULSORY_B = 288  # bytes per cell-update: Q[7] + pi[10] + Pi, read + write
 # matter (nactive, read from the device every step).
 KERNEL_BYTES = {
     "k_update_m": 48,       # m[3] in, m[3] out
-    "k_face_x": 120,        # Q or Qh [7] + m in, face flux [7] out
-    "k_face_y": 120,
-    "k_face_z": 120,
+    "k_face": 360,          # per direction Q or Qh [7] + m in, face flux [7] out
     "k_update": 336,        # 3 face fluxes [21] + Q/Qh [7] in, 2 x [7] out
     "k_ghost": 0,           # boundary planes only
     "k_visc_prims": 152,    # Qh [7] in, prims [8] + [4] out

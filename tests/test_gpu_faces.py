@@ -1,0 +1,111 @@
+"""The face and con2prim kernels at the sizes and states where their splits
+end: grids whose sides and cell counts leave remainders of a block's faces,
+the smallest sides, and the root find and the table's nb = 0 row over states
+and energies at their borders.  Everything is compared bit for bit."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import pyoracle as P
+from helpers import compare_states, gpu_state_as_oracle
+from vhlle_b200 import capi
+from vhlle_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+# (2, 2): one face per direction; 64 and 65 cells: a block's faces, one more
+@pytest.mark.parametrize("nx,ny,nz", [(2, 2, 1), (3, 2, 2), (4, 4, 4), (5, 13, 1), (8, 8, 1), (16, 5, 3),
+                                      (33, 7, 2), (64, 3, 5), (65, 31, 1)])
+@pytest.mark.parametrize("nb", [0.0, 0.3])
+def test_steps_on_ragged_grids_equal_oracle(nx, ny, nz, nb):
+    if nz > 1:
+        s = W.glauber3d_setup(nx=nx, ny=ny, nz=nz, xmax=6.0, etamax=4.0, b=2.0, nb_peak=nb)
+    else:
+        s = W.batch_event(0, nz=1)
+        g = W.Grid(nx, ny, 1, -6., 6., -6., 6., -0.5, 0.5)
+        x, y, _ = g.coords()
+        prof, _ = W.glauber_profile(3, 2.0, x, y)
+        e = np.where(prof < 1e-3, 0., 40. * prof)[None]
+        z = np.zeros_like(e)
+        s.grid, s.m = g, (e.reshape(-1) > 0).astype(float)
+        s.Q = W.conserved_from_primitive(s.tau0, e, z, nb * prof[None] * (e > 0), z, z, z).reshape(7, -1)
+        s.zetaSparam = 0
+    h, o = capi.GpuHydro(s), P.OracleRun(s)
+    for _ in range(3):
+        h.step(1)
+        assert o.step(1) == 0
+        bad = compare_states(gpu_state_as_oracle(h.get_state()), o.get_state())
+        assert not bad, bad
+    h.close()
+
+
+def _axis(kind, n):
+    if kind == "log":
+        return np.exp(np.linspace(np.log(1e-4), np.log(1e3), n))
+    if kind == "linear":
+        return np.linspace(0.01, 50., n)
+    if kind == "from_zero":
+        return np.linspace(0., 50., n)
+    return np.sort(np.random.default_rng(5).uniform(1e-3, 80., n))  # searched, not guessed
+
+
+@pytest.mark.parametrize("kind", ["log", "linear", "from_zero", "irregular"])
+@pytest.mark.parametrize("nbaxis", ["two", "many", "symmetric", "above_zero", "off_zero"])
+def test_pressure_at_zero_charge(kind, nbaxis):
+    """EoS::p (which the root find calls) at nb = 0 equals EoS::eos's p, which
+    always takes the table's four corners, and the oracle's."""
+    eg = _axis(kind, 301)
+    ng = {"two": np.array([0., 1.]), "many": np.linspace(0., 1., 40), "symmetric": np.linspace(-1., 1., 41),
+          "above_zero": np.linspace(0.1, 1., 7), "off_zero": np.linspace(-0.95, 1., 40)}[nbaxis]
+    E, B = np.meshgrid(eg, ng)  # [in][ie]
+    p = (0.3 * E - 0.01 + 0.02 * B * B).reshape(-1)
+    eos = W.EosTable(kind=1, egrid=eg, ngrid=ng, p=p, T=(0.1 + 0.05 * E ** 0.25).reshape(-1), mub=B.reshape(-1))
+    s = W.small_glauber3d(5, 5)
+    s.eos = eos
+    rng = np.random.default_rng(2)
+    e = np.concatenate([eg, np.nextafter(eg, 0), np.nextafter(eg, 1e9), rng.uniform(-1e-3, 100., 2000),
+                        10. ** rng.uniform(-300, 9, 2000), [0., -0., 1e-308, 5e-324, 1e12, 1e300]])
+    h, o = capi.GpuHydro(s), P.OracleRun(s)
+    for nb in (0., -0.):
+        nbs = np.full_like(e, nb)
+        got = h.eos6(e, nbs)
+        assert np.array_equal(got[:, 4], got[:, 0], equal_nan=True)
+        ok = e >= 0  # (EoS1f's eos does not return for e < 0)
+        assert np.array_equal(got[ok, 4], o.eos6(e, nbs)[ok, 4], equal_nan=True)
+    h.close()
+
+
+@pytest.mark.parametrize("eos", ["table", "nb_table", "conformal", "chiral"])
+def test_root_find_equals_oracle(eos):
+    """transformPV from vacuum and rest to |M| > Q_t, over 24 decades, with and
+    without charge."""
+    torch = pytest.importorskip("torch")
+    s = W.small_glauber3d(5, 5)
+    s.eos = {"table": W.make_cs2_table, "nb_table": lambda: W.nb_table(400, 21), "chiral": W.chiral_eos,
+             "conformal": lambda: W.EosTable(kind=0)}[eos]()
+    rng = np.random.default_rng(11)
+    n = 20000
+    T = 10. ** rng.uniform(-20, 4, n)
+    d = rng.normal(size=(n, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    M = T * np.where(rng.random(n) < 0.5, rng.uniform(0., 1.2, n), 1. - 10. ** rng.uniform(-16, 0, n))
+    Q = np.zeros((n, 7))
+    Q[:, 0] = T
+    Q[:, 1:4] = M[:, None] * d
+    Q[n // 2:, 4] = T[n // 2:] * 10. ** rng.uniform(-6, 0, n - n // 2)
+    Q[n // 2:, 5] = 0.4 * Q[n // 2:, 4]
+    Q[::11, 1:4] = 0.           # at rest
+    Q[::13, 3] = 0.
+    Q[::17, 0] = 0.             # vacuum
+    Q[::19, 0] *= -1.
+    Q[::23, 4] = -0.
+    h, o = capi.GpuHydro(s), P.OracleRun(s)
+    dQ = torch.from_numpy(np.ascontiguousarray(Q.T)).cuda()
+    out = torch.empty((8, n), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    h._check(h.L.vh_transform_pv(h.h, ctypes.c_void_p(dQ.data_ptr()), n, ctypes.c_void_p(out.data_ptr())))
+    h.sync()
+    assert np.array_equal(out.cpu().numpy().T, o.transform_pv(Q), equal_nan=True)
+    h.close()

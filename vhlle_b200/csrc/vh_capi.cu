@@ -333,6 +333,35 @@ static vh_status upload_eos(vh_ctx* c, const vh_eos* eos, vh::EosDev& E) {
       }
       rdev += r.size();
     }
+    // the row of nb = 0 (eos1f_row0): its bracket as the binary search finds
+    // it, where the bracket starts at 0 exactly and no term of the next row
+    // can be anything but +-0
+    E.row0 = nullptr;
+    if (E.erinv && E.emode != vh::GRID_BSEARCH) {
+      int k1 = 0, k2 = nn - 1;
+      while (k2 - k1 > 1) {
+        const int k = (k1 + k2) / 2;
+        (0. < eos->ngrid[k] ? k2 : k1) = k;
+      }
+      bool ok = eos->ngrid[k1] == 0. && eos->ngrid[k2] > 0. && eos->egrid[0] >= 0x1p-800;
+      const double *p0 = eos->p + (size_t)ne * k1, *p1 = p0 + ne;
+      for (int k = 0; k < ne; k++) ok = ok && std::isfinite(p0[k]) && std::isfinite(p1[k]);
+      if (ok) {
+        std::vector<double> row((size_t)6 * (ne - 1));
+        for (int k = 0; k + 1 < ne; k++) {
+          const double den = eos->egrid[k + 1] - eos->egrid[k];
+          const double v[6] = {eos->egrid[k], eos->egrid[k + 1], 1.0 / den, den, p0[k], p0[k + 1]};
+          std::copy(v, v + 6, row.begin() + (size_t)6 * k);
+        }
+        double* dev = nullptr;
+        if ((st = dalloc(c, &dev, row.size())) != VH_OK) return st;
+        if ((e = cudaMemcpy(dev, row.data(), row.size() * sizeof(double), cudaMemcpyHostToDevice))) {
+          cuda_fail(c, e, "vh_create: EoS upload");
+          return VH_ERR_CUDA;
+        }
+        E.row0 = reinterpret_cast<const double2*>(dev);
+      }
+    }
   }
   if (eos->kind == VH_EOS_TABLE3) {
     const int ne = eos->ne, nn = eos->nn;
@@ -1287,10 +1316,10 @@ vh_status vh_sync(vh_ctx* ctx) {
 
 vh_status vh_launches_per_step(vh_ctx* ctx, int* n) {
   if (!ctx || !n) return VH_ERR_ARG;
-  // update_m, 2 x (faces + update), 2 ghost, the viscous five (prims, the
+  // update_m, 2 x (faces, update), 2 ghost, the viscous five (prims, the
   // relaxation's list and relaxation, advection, update) and the six of the
   // vorticity, the MLP guess, the clock
-  int k = 1 + 2 * (2 + (ctx->g.nz > 1 ? 1 : 0) + 1) + 1 + (ctx->viscous ? 5 : 0) + 1 +
+  int k = 1 + 2 * (1 + 1) + 1 + (ctx->viscous ? 5 : 0) + 1 +
           (ctx->viscous && ctx->vort_on ? 6 : 0) + (ctx->mlp ? 1 : 0) + 1;
   *n = k;
   return VH_OK;

@@ -79,6 +79,11 @@ struct EosDev {
   // interpolation weights then take crm::mk_div instead of a divide
   const double* __restrict__ erinv;
   const double* __restrict__ nrinv;
+  // kind 1: the lookup at nb = 0 where that is one row of the table (its nb
+  // bracket starts at 0 and the row's and the next row's p are finite), per
+  // e interval {g[k], g[k+1]}, {RN(1/(g[k+1]-g[k])), g[k+1]-g[k]},
+  // {p[k], p[k+1]}; or null (eos1f_row0)
+  const double2* __restrict__ row0;
   // con2prim policy (not part of the EoS proper, but passed everywhere with
   // it): stop when |dv| < tol (the reference's 0.00001 by default); vguess,
   // when set, holds a start point in (0, 1) per cell for the root find; stats,
@@ -312,6 +317,39 @@ __device__ __forceinline__ void eos1f(const EosDev& E, double e, double nb,
     T = sT;
     mub = sm;
   }
+}
+
+// eos1f's p at nb = +-0 from the table's row there: with a zero nb weight
+// the other row's terms are +-0 and add nothing, so this is eos1f's sum bit
+// for bit.  A baryon-free run makes nothing but such lookups; one has 12
+// instead of 27 FP64 operations and reads three 16-byte pairs next to one
+// another instead of ten doubles in six places.
+//
+// The weight's division needs no range test (crm::mk_div): with every grid
+// point at least 2^-800, e - g is +0 or at least 2^-853, and where it is so
+// large that the quotient overflows the sum is NaN either way.
+__device__ __forceinline__ double eos1f_row0(const EosDev& E, double e) {
+  const int ne = E.ne;
+  const float fx = (float)e;
+  const float t0 = (E.emode == GRID_LOG ? __log2f(fx) - E.e0 : fx - E.e0) * E.einv;
+  int k = (int)fminf(fmaxf(t0, 0.f), (float)(ne - 2));  // NaN: 0, and p NaN
+  const double2* t = E.row0 + 3 * k;
+  double2 g = __ldg(t), d = __ldg(t + 1), pp = __ldg(t + 2);
+  // a guess is a step or two off at most, and rarely
+  while ((k > 0 && e < g.x) || (k < ne - 2 && e >= g.y)) {
+    k += e < g.x ? -1 : 1;
+    t = E.row0 + 3 * k;
+    g = __ldg(t);
+    d = __ldg(t + 1);
+    pp = __ldg(t + 2);
+  }
+  const double num = e - g.x;
+  const double q0 = num * d.x;
+  const double ue = fma(fma(-q0, d.y, num), d.x, q0);
+  double sp = 0.;
+  sp += (1. - ue) * pp.x;
+  sp += ue * pp.y;
+  return sp < 0. ? 0. : sp;
 }
 
 // EoSaux::get / EoSaux::p, src/eoChiral.cpp:99-151: the bracket is the
@@ -757,6 +795,7 @@ __device__ __forceinline__ double eos_p(const EosDev& E, double e, double nb) {
     return p;
   }
   if (E.kind == 0) return ddivp(e, 3.);
+  if (E.row0 && nb == 0.) return eos1f_row0(E, e);
   eos1f<false>(E, e, nb, T, mub, p);
   return p;
 }
@@ -832,25 +871,24 @@ __device__ __forceinline__ double eos_s(const EosDev& E, double e, double nb,
 // (a learned guess) the iteration starts there instead of at 0.5 and the
 // bracket is narrowed by the sign of f at g; the safeguarded Newton /
 // bisection then runs as in the reference until |dv| < E.tol.
+//
+// One loop holds the only EoS lookup: the start point's, each iterate's and
+// the final state's pressure are its trips, so the final lookup of a lane
+// that is done shares a trip with the others' next iterates, and the
+// kernels' code is a third of the unrolled form's (the face kernels spent
+// most of their issue slots waiting for instructions: 5.6 of 14 cycles per
+// issue, at 101x101x51).
 template <int EK = EK_ANY>
 __device__ __forceinline__ void transform_pv(const EosDev& E, double Q[7], Prim& o,
                                              float g = -1.f) {
   const int MAXIT = 100;
   const double dpe = 1. / 3.;
   const double corrf = 0.9999;
-  double v, vl = 0., vh = 1., dvold, dv, f, df;
   double M = sqrtz(Q[X_] * Q[X_] + Q[Y_] * Q[Y_] + Q[Z_] * Q[Z_]);
   if (Q[T_] <= 0.) {
     o.e = 0.; o.p = 0.;
     o.vx = o.vy = o.vz = 0.;
     o.nb = o.nq = o.ns = 0.;
-    return;
-  }
-  if (M == 0.) {
-    o.e = Q[T_];
-    o.vx = 0.; o.vy = 0.; o.vz = 0.;
-    o.nb = Q[NB_]; o.nq = Q[NQ_]; o.ns = Q[NS_];
-    o.p = eos_p<EK>(E, o.e, o.nb);
     return;
   }
   if (M > Q[T_]) {
@@ -859,17 +897,11 @@ __device__ __forceinline__ void transform_pv(const EosDev& E, double Q[7], Prim&
     Q[Z_] *= corrf * Q[T_] / M;
     M = Q[T_] * corrf;
   }
-  double e, p, nb, nq, ns;
+  const bool rest = M == 0.;  // v = 0: one trip, for p(Q_t, Q_nb)
   const bool guessed = g > 0.f && g < 1.f;
-  v = guessed ? (double)g : 0.5 * (vl + vh);
-  e = Q[T_] - M * v;
-  if (e < 0.) e = 0.;
-  {
-    const double sq = sqrt(1 - v * v);
-    nb = Q[NB_] * sq;
-    nq = Q[NQ_] * sq;
-    ns = Q[NS_] * sq;
-  }
+  double vl = 0., vh = 1., dvold = 1., dv = 1.;
+  double v = guessed ? (double)g : 0.5;
+  double e, p, nb = Q[NB_];
   // The table-slope variant (ek_slope) takes f' = (Q_t + p) - v (M dp/de +
   // dp/dnb Q_nb v / sqrt(1 - v^2)) with the EoS's own derivatives, so the
   // Newton steps converge quadratically inside a table cell, and stops when
@@ -877,31 +909,45 @@ __device__ __forceinline__ void transform_pv(const EosDev& E, double Q[7], Prim&
   // into bisection).  Not the reference's iteration: for a tight tolerance
   // only, where the result does not depend on the path to the root.
   constexpr bool SL = ek_slope(EK);
-  double dpde = 0., dpdn = 0.;
-  auto slope = [&](double vv, double sq) {
-    const double dn = sq > 0. ? dpdn * Q[NB_] * vv / sq : 0.;
-    return (Q[T_] + p) - vv * (M * dpde + dn);
-  };
-  double sq0 = sqrt(1 - v * v);
-  if (SL) {
-    p = eos_p_d<EK>(E, e, nb, dpde, dpdn);
-  } else {
-    p = eos_p<EK>(E, e, nb);
-  }
-  f = (Q[T_] + p) * v - M;
-  df = SL ? slope(v, sq0) : (Q[T_] + p) - M * v * dpe;
-  if (guessed) {
-    if (f > 0.)
-      vh = v;
-    else
-      vl = v;
-  }
-  dvold = vh - vl;
-  dv = dvold;
+  // Q_nb = +-0 stays Q_nb times any square root of a number in [0, 1]
+  const bool nb0 = !SL && Q[NB_] == 0.;
+  bool done = rest, keep_nb = rest;
   int it = 0;
-  const bool at_root = SL && f == 0.;  // a start point that is the root
-  for (int i = 0; i < MAXIT && !at_root; i++) {
-    it = i + 1;
+#pragma unroll 1
+  while (true) {
+    e = Q[T_] - M * v;
+    double sq = 0.;
+    if (!keep_nb && !(nb0 && fabs(v) <= 1.)) {
+      sq = sqrt(1 - v * v);
+      nb = Q[NB_] * sq;
+    }
+    if (!done && e < 0.) e = 0.;
+    double dpde = 0., dpdn = 0.;
+    if (SL) {
+      p = eos_p_d<EK>(E, e, nb, dpde, dpdn);
+    } else {
+      p = eos_p<EK>(E, e, nb);
+    }
+    if (done) break;  // p of the state at v, with the last iterate's nb, as the reference
+    const double f = (Q[T_] + p) * v - M;
+    if (SL && f == 0.) {
+      done = keep_nb = true;
+      continue;
+    }
+    double df;
+    if (SL) {
+      const double dn = sq > 0. ? dpdn * Q[NB_] * v / sq : 0.;
+      df = (Q[T_] + p) - v * (M * dpde + dn);
+    } else {
+      df = (Q[T_] + p) - M * v * dpe;
+    }
+    if (it > 0 || guessed) {
+      if (f > 0.)
+        vh = v;
+      else
+        vl = v;
+      if (it == 0) dvold = dv = vh - vl;
+    }
     if ((f + df * (vh - v)) * (f + df * (vl - v)) >= 0. ||
         fabs(2. * f) > fabs(dvold * df)) {
       dvold = dv;
@@ -909,28 +955,19 @@ __device__ __forceinline__ void transform_pv(const EosDev& E, double Q[7], Prim&
       v = vl + dv;
     } else {
       dvold = dv;
-      dv = ddiv(f, df);
+      dv = f / df;  // a zero f is rare here, and df is not: no ddiv
       v -= dv;
     }
-    if (fabs(dv) < E.tol) break;
-    e = Q[T_] - M * v;
-    if (e < 0.) e = 0.;
-    const double sq = sqrt(1 - v * v);
-    nb = Q[NB_] * sq;
-    nq = Q[NQ_] * sq;
-    ns = Q[NS_] * sq;
-    if (SL) {
-      p = eos_p_d<EK>(E, e, nb, dpde, dpdn);
-    } else {
-      p = eos_p<EK>(E, e, nb);
-    }
-    f = (Q[T_] + p) * v - M;
-    if (SL && f == 0.) break;
-    df = SL ? slope(v, sq) : (Q[T_] + p) - M * v * dpe;
-    if (f > 0.)
-      vh = v;
-    else
-      vl = v;
+    it++;
+    keep_nb = fabs(dv) < E.tol;
+    done = keep_nb || it == MAXIT;
+  }
+  if (rest) {
+    o.e = Q[T_];
+    o.p = p;
+    o.vx = 0.; o.vy = 0.; o.vz = 0.;
+    o.nb = Q[NB_]; o.nq = Q[NQ_]; o.ns = Q[NS_];
+    return;
   }
   if (E.stats) {
     atomicAdd(&E.stats[0], 1ull);
@@ -951,8 +988,8 @@ __device__ __forceinline__ void transform_pv(const EosDev& E, double Q[7], Prim&
       o.vz = ddivp(nz, M);
     }
   }
-  o.e = Q[T_] - M * v;
-  o.p = eos_p<EK>(E, o.e, nb);  // the last iterate's nb, as the reference
+  o.e = e;
+  o.p = p;
   const double sq = sqrt(1 - o.vx * o.vx - o.vy * o.vy - o.vz * o.vz);
   o.nb = Q[NB_] * sq;
   o.nq = Q[NQ_] * sq;
@@ -1059,14 +1096,15 @@ __device__ __forceinline__ bool hlle_face(int dir, bool predict, double tau, dou
                                           double dxdir, Prim l, Prim r, double mL,
                                           double mR, double flux[7], unsigned& err) {
   const double dta = predict ? dt / 2. : dt;
-  const double El = ddiv(l.e + l.p, 1 - l.vx * l.vx - l.vy * l.vy - l.vz * l.vz);
-  const double Er = ddiv(r.e + r.p, 1 - r.vx * r.vx - r.vy * r.vy - r.vz * r.vz);
+  const double hl = l.e + l.p, hr = r.e + r.p;  // before the cut of negative e
   const double tauFactor = predict ? tau + 0.25 * dt : tau + 0.5 * dt;
   if (l.e < 0.) { l.e = 0.; l.p = 0.; }
   if (r.e < 0.) { r.e = 0.; r.p = 0.; }
   if (l.e > 1e10) { err |= ERR_E_HUGE; return false; }
   if (l.e == 0. && r.e == 0.) return false;
   if (mL < 1. && mR < 1.) return false;
+  const double El = ddiv(hl, 1 - l.vx * l.vx - l.vy * l.vy - l.vz * l.vz);
+  const double Er = ddiv(hr, 1 - r.vx * r.vx - r.vy * r.vy - r.vz * r.vz);
   const double cs2 = 1. / 3.;
   const double cs = sqrt(1. / 3.);
   const double gammal = 1. / sqrt(1 - l.vx * l.vx - l.vy * l.vy - l.vz * l.vz);

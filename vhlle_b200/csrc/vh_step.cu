@@ -21,6 +21,12 @@
 
 namespace vh {
 
+// resident blocks of 128 threads per SM, from sweeps on the 101x101x51 event
+// (us per step at the stated counts): the face kernel 6 / 7 / 8 / 10 blocks
+// 369 / 341 / 330 / 364; the update 6 / 8 / 10 / 12: 112 / 113 / 124 / 129;
+// the viscous primitives 6 / 7 / 8 / 10: 57.3 / 55.5 / 57.3 / 60.9
+constexpr int kFaceMinBlocks = 8, kUpdateMinBlocks = 6, kPrimsMinBlocks = 7;
+
 // -------------------------------------------------------------- updateM
 // Fluid::updateM, src/fld.cpp:384-423 (both passes; out of place).
 __device__ __forceinline__ void d_update_m(const Geo& g, const double* __restrict__ m,
@@ -68,80 +74,100 @@ __global__ void k_update_m(Geo g, const double* __restrict__ m, double* __restri
 
 
 // ------------------------------------------------------------ face flux
-// One HLLE face between cell i and its +DIR neighbour (Hydro::hlle_flux with
-// Cell::getPrimVarRight / getPrimVarLeft or their H variants,
-// src/cll.cpp:106-204).  F[c*N + i] holds the flux of the face on the +DIR
-// side of cell i (0 where the reference adds nothing).
-// Occupancy (measured over 100 steps of the 101x101x51 event): 8 blocks of
-// 128 threads per SM (64 registers, a few spills) are 11 % faster than the
-// unbounded build (80 registers, 6 blocks); 10 blocks are slower.  The
-// same sweep set k_update to 12 blocks (-14 %), k_visc_prims to 8 (-14 %),
-// k_visc_update to 8 (-10 %); k_is_advect stays unbounded (8 blocks: +52 %).
-template <int DIR, bool PRED, int EK>
-// 7 blocks of 128 per SM (72 registers): measured against 6 and 8 blocks on
-// the 300-step event, 3 % faster than 8 (64 registers, more spills)
-__device__ __forceinline__ void d_face(const Geo& g, const EosDev& E,
+// One HLLE face between cell i and its neighbour on the + side along `dir`
+// (Hydro::hlle_flux with Cell::getPrimVarRight / getPrimVarLeft or their H
+// variants, src/cll.cpp:106-204).  F[c*N + i] holds the flux of the face on
+// the + side of cell i (0 where the reference adds nothing).
+//
+// A block of B threads takes B / 2 faces: thread t < B/2 reconstructs and
+// solves the left state of face t, thread t + B/2 its right state, the
+// primitives meet in shared memory, and the first half of the block forms
+// the fluxes.  One launch holds the faces of every direction (the direction
+// of a block a run-time number), so the directions share one instruction
+// stream, and there is one ragged end per pass instead of three.
+// A thread that solved both states of a face (three kernels of 16 thousand
+// warps) spent 5.6 of 14 cycles per issue waiting for instructions; in this
+// form it is 0.5 of 9, and 101x101x51 takes 280 us of faces per step instead
+// of 492 (2 passes, baryon-free, 20 % of the cells with matter).
+static inline unsigned face_blocks(long long N, int bs) {
+  return (unsigned)((N + bs / 2 - 1) / (bs / 2));
+}
+template <int EK>
+__device__ __forceinline__ void d_face(const Geo& g, const EosDev& E, bool predict, int dir,
                                        const double* __restrict__ QQ,
                                        const double* __restrict__ m, double* __restrict__ F,
                                        const double* __restrict__ clk, unsigned* err,
                                        long long blk) {
+  __shared__ double sp[8][128];
+  const int half = blockDim.x >> 1, t = threadIdx.x;
+  const bool right = t >= half;
   const double tau = clk[0], dt = clk[1];  // the step's clock (device)
-  const long long i = blk * blockDim.x + threadIdx.x;
-  if (i >= g.N) return;
-  int ix, iy, iz;
-  coords(g, i, ix, iy, iz);
+  const long long i = blk * half + (right ? t - half : t);
   const long long N = g.N;
-  long long L = i, Lm, R, Rp;
-  if (DIR == X_) {
-    if (ix >= g.nx - 1) return;
-    Lm = cidx(g, ix - 1, iy, iz);
-    R = cidx(g, ix + 1, iy, iz);
-    Rp = cidx(g, ix + 2, iy, iz);
-  } else if (DIR == Y_) {
-    if (iy >= g.ny - 1) return;
-    Lm = cidx(g, ix, iy - 1, iz);
-    R = cidx(g, ix, iy + 1, iz);
-    Rp = cidx(g, ix, iy + 2, iz);
-  } else {
-    if (iz >= g.nz - 1) return;
-    Lm = cidx(g, ix, iy, iz - 1);
-    R = cidx(g, ix, iy, iz + 1);
-    Rp = cidx(g, ix, iy, iz + 2);
+  const long long st = dir == X_ ? 1 : (dir == Y_ ? g.nx : (long long)g.nx * g.ny);
+  bool face = false;  // a face of the grid
+  int c = 0, n = 0;
+  if (i < N) {
+    int ix, iy, iz;
+    coords(g, i, ix, iy, iz);
+    c = dir == X_ ? ix : (dir == Y_ ? iy : iz);
+    n = dir == X_ ? g.nx : (dir == Y_ ? g.ny : g.nz);
+    face = c < n - 1;
   }
-  double qlr[14];  // the two reconstructed states, then divided by tau as one batch
+  if (face) {
+    // the cell whose edge this is, and its neighbours (clamped as getCell)
+    if (right) c++;
+    const long long cell = i + (right ? st : 0);
+    const long long lo = cell - (c > 0 ? st : 0), hi = cell + (c < n - 1 ? st : 0);
+    // the reconstructed state, then divided by tau as one batch; the state
+    // of vacuum (Q_t <= 0, transform_pv's first test) needs no more than Q_t
+    double q[7];
+    auto edge = [&](int k) {
+      const double x0 = QQ[k * N + lo], x1 = QQ[k * N + cell], x2 = QQ[k * N + hi];
+      const double dQ = minmod((x2 - x1) / 2., (x1 - x0) / 2.);
+      return x1 + (right ? -dQ : dQ);
+    };
+    Prim p{0., 0., 0., 0., 0., 0., 0., 0.};
+    q[0] = edge(0);
+    if (!(q[0] <= 0.)) {
 #pragma unroll
-  for (int k = 0; k < 7; k++) {
-    const double a = QQ[k * N + Lm], b = QQ[k * N + L], c = QQ[k * N + R], d = QQ[k * N + Rp];
-    const double dQl = minmod((c - b) / 2., (b - a) / 2.);
-    qlr[k] = b + dQl;
-    const double dQr = minmod((d - c) / 2., (c - b) / 2.);
-    qlr[7 + k] = c - dQr;
+      for (int k = 1; k < 7; k++) q[k] = edge(k);
+      div_batch<7>(q, tau, 1.0 / tau, crm::mk_den_ok(tau));
+      transform_pv<EK>(E, q, p, c2p_guess(E, cell));
+    }
+    sp[0][t] = p.e;
+    sp[1][t] = p.p;
+    sp[2][t] = p.nb;
+    sp[3][t] = p.nq;
+    sp[4][t] = p.ns;
+    sp[5][t] = p.vx;
+    sp[6][t] = p.vy;
+    sp[7][t] = p.vz;
   }
-  div_batch<14>(qlr, tau, 1.0 / tau, crm::mk_den_ok(tau));
-  double ql[7], qr[7];
-#pragma unroll
-  for (int k = 0; k < 7; k++) {
-    ql[k] = qlr[k];
-    qr[k] = qlr[7 + k];
-  }
-  Prim pl, pr;
-  transform_pv<EK>(E, ql, pl, c2p_guess(E, L));
-  transform_pv<EK>(E, qr, pr, c2p_guess(E, R));
-  const double dxdir = DIR == X_ ? g.dx : (DIR == Y_ ? g.dy : g.dz);
+  __syncthreads();
+  if (right || !face) return;
+  auto prim = [&](int s) {
+    return Prim{sp[0][s], sp[1][s], sp[2][s], sp[3][s], sp[4][s], sp[5][s], sp[6][s], sp[7][s]};
+  };
+  const double dxdir = dir == X_ ? g.dx : (dir == Y_ ? g.dy : g.dz);
   double fl[7];
   unsigned e = 0;
-  const bool ok = hlle_face(DIR, PRED, tau, dt, dxdir, pl, pr, m[(DIR - 1) * N + L],
-                            m[(DIR - 1) * N + R], fl, e);
+  const bool ok = hlle_face(dir, predict, tau, dt, dxdir, prim(t), prim(t + half),
+                            m[(dir - 1) * N + i], m[(dir - 1) * N + i + st], fl, e);
   if (e) atomicOr(err, e);
 #pragma unroll
   for (int k = 0; k < 7; k++) F[k * N + i] = ok ? fl[k] : 0.;
 }
-template <int DIR, bool PRED, int EK>
-__global__ void __launch_bounds__(128, 7) k_face(Geo g, EosDev E, const double* __restrict__ QQ,
-                                              const double* __restrict__ m,
-                                              double* __restrict__ F, const double* __restrict__ clk,
-                                              unsigned* err) {
-  d_face<DIR, PRED, EK>(g, E, QQ, m, F, clk, err, blockIdx.x);
+// nbd blocks per direction, X first
+template <int EK>
+__global__ void __launch_bounds__(128, kFaceMinBlocks) k_face(
+    Geo g, EosDev E, bool predict, unsigned nbd, const double* __restrict__ QQ,
+    const double* __restrict__ m, double* __restrict__ Fx, double* __restrict__ Fy,
+    double* __restrict__ Fz, const double* __restrict__ clk, unsigned* err) {
+  const unsigned b = blockIdx.x;
+  const int dir = b < nbd ? X_ : (b < 2 * nbd ? Y_ : Z_);
+  d_face<EK>(g, E, predict, dir, QQ, m, dir == X_ ? Fx : (dir == Y_ ? Fy : Fz), clk, err,
+             b - (dir - 1) * nbd);
 }
 
 
@@ -241,7 +267,7 @@ __device__ __forceinline__ void d_update(const Geo& g, const EosDev& E, double* 
   }
 }
 template <bool PRED, int EK>
-__global__ void __launch_bounds__(128, 12) k_update(Geo g, EosDev E, double* __restrict__ Q,
+__global__ void __launch_bounds__(128, kUpdateMinBlocks) k_update(Geo g, EosDev E, double* __restrict__ Q,
                                                 double* __restrict__ Qh,
                                                 double* __restrict__ Qprev,
                                                 const double* __restrict__ Fx,
@@ -426,7 +452,7 @@ __device__ __forceinline__ void d_visc_prims(const Geo& g, const EosDev& E, cons
   }
 }
 template <int EK>
-__global__ void __launch_bounds__(128, 8) k_visc_prims(Geo g, EosDev E, TrDev tr,
+__global__ void __launch_bounds__(128, kPrimsMinBlocks) k_visc_prims(Geo g, EosDev E, TrDev tr,
                                                     const double* __restrict__ Q,
                                                     const double* __restrict__ Qprev,
                                                     const double* __restrict__ Qh,
@@ -1186,7 +1212,7 @@ __global__ void k_transform_pv(EosDev E, const double* __restrict__ Q, long long
 static inline unsigned nblk(long long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
 const char* const kKernelNames[KK_COUNT] = {
-    "k_update_m", "k_face_x", "k_face_y", "k_face_z", "k_update", "k_ghost",
+    "k_update_m", "k_face", "k_update", "k_ghost",
     "k_visc_prims", "k_is_relax", "k_is_advect", "k_visc_update",
     "vorticity (k_vort_*, 6 kernels)"};
 
@@ -1210,31 +1236,17 @@ static int launch_step_ek(const StepArgs& a, cudaStream_t s, LaunchMarker* mk) {
   for (int pass = 0; pass < 2; pass++) {
     const bool pred = pass == 0;
     const double* QQ = pred ? F.Q : F.Qh;
-    if (pred) {
-      k_face<X_, true, EK><<<nb, bs, 0, s>>>(g, a.eos, QQ, m, F.Fx, a.clk, F.err);
-      done(KK_FACE_X);
-      k_face<Y_, true, EK><<<nb, bs, 0, s>>>(g, a.eos, QQ, m, F.Fy, a.clk, F.err);
-      done(KK_FACE_Y);
-      if (g.nz > 1) {
-        k_face<Z_, true, EK><<<nb, bs, 0, s>>>(g, a.eos, QQ, m, F.Fz, a.clk, F.err);
-        done(KK_FACE_Z);
-      }
-      k_update<true, EK><<<nb, bs, 0, s>>>(g, a.eos, F.Q, F.Qh, F.Qprev, F.Fx, F.Fy, F.Fz, a.clk, F.err,
-                                       a.viscous ? F.pBC : nullptr, nullptr);
-      done(KK_UPDATE);
-    } else {
-      k_face<X_, false, EK><<<nb, bs, 0, s>>>(g, a.eos, QQ, m, F.Fx, a.clk, F.err);
-      done(KK_FACE_X);
-      k_face<Y_, false, EK><<<nb, bs, 0, s>>>(g, a.eos, QQ, m, F.Fy, a.clk, F.err);
-      done(KK_FACE_Y);
-      if (g.nz > 1) {
-        k_face<Z_, false, EK><<<nb, bs, 0, s>>>(g, a.eos, QQ, m, F.Fz, a.clk, F.err);
-        done(KK_FACE_Z);
-      }
-      k_update<false, EK><<<nb, bs, 0, s>>>(g, a.eos, F.Q, F.Qh, F.Qprev, F.Fx, F.Fy, F.Fz, a.clk, F.err,
-                                        nullptr, a.viscous ? F.pA : nullptr);
-      done(KK_UPDATE);
-    }
+    const unsigned nbd = face_blocks(g.N, bs);
+    k_face<EK><<<nbd * (g.nz > 1 ? 3 : 2), bs, 0, s>>>(g, a.eos, pred, nbd, QQ, m, F.Fx, F.Fy, F.Fz,
+                                                       a.clk, F.err);
+    done(KK_FACE);
+    if (pred)
+      k_update<true, EK><<<nb, bs, 0, s>>>(g, a.eos, F.Q, F.Qh, F.Qprev, F.Fx, F.Fy, F.Fz, a.clk,
+                                           F.err, a.viscous ? F.pBC : nullptr, nullptr);
+    else
+      k_update<false, EK><<<nb, bs, 0, s>>>(g, a.eos, F.Q, F.Qh, F.Qprev, F.Fx, F.Fy, F.Fz, a.clk,
+                                            F.err, nullptr, a.viscous ? F.pA : nullptr);
+    done(KK_UPDATE);
   }
   k_ghost<false><<<nb, bs, 0, s>>>(g, F.gsrc, F.gdst, F.Q, F.Qh, F.pi, F.Pi);
   done(KK_GHOST);
@@ -1360,17 +1372,25 @@ __global__ void kb_update_m(const StepDev* __restrict__ evs, const BItem* __rest
   d_update_m(g, A.f.m, A.f.m2, A.clk, blk);
 }
 
-template <int DIR, bool PRED, int EK>
-__global__ void __launch_bounds__(128, 7) kb_face(const StepDev* __restrict__ evs,
-                                               const BItem* __restrict__ items) {
-  VH_ITEM
+// the faces of a work item's kBatchBlock cells take two blocks per direction
+// (grid.y: X, Y, Z)
+template <int EK>
+__global__ void __launch_bounds__(128, kFaceMinBlocks) kb_face(const StepDev* __restrict__ evs,
+                                                               const BItem* __restrict__ items,
+                                                               bool predict) {
+  const BItem it = items[blockIdx.x >> 1];
+  const StepDev& A = evs[it.ev];
+  const Geo g = A.g;
+  const int dir = X_ + blockIdx.y;
+  if (dir == Z_ && g.nz == 1) return;
   const EosDev E = A.eos;
-  double* F = DIR == X_ ? A.f.Fx : (DIR == Y_ ? A.f.Fy : A.f.Fz);
-  d_face<DIR, PRED, EK>(g, E, PRED ? A.f.Q : A.f.Qh, A.f.m2, F, A.clk, A.f.err, blk);
+  double* F = dir == X_ ? A.f.Fx : (dir == Y_ ? A.f.Fy : A.f.Fz);
+  d_face<EK>(g, E, predict, dir, predict ? A.f.Q : A.f.Qh, A.f.m2, F, A.clk, A.f.err,
+             2LL * it.blk + (blockIdx.x & 1));
 }
 
 template <bool PRED, int EK>
-__global__ void __launch_bounds__(128, 12) kb_update(const StepDev* __restrict__ evs,
+__global__ void __launch_bounds__(128, kUpdateMinBlocks) kb_update(const StepDev* __restrict__ evs,
                                                  const BItem* __restrict__ items) {
   VH_ITEM
   const EosDev E = A.eos;
@@ -1387,7 +1407,7 @@ __global__ void kb_ghost(const StepDev* __restrict__ evs, const BItem* __restric
 }
 
 template <int EK>
-__global__ void __launch_bounds__(128, 8) kb_visc_prims(const StepDev* __restrict__ evs,
+__global__ void __launch_bounds__(128, kPrimsMinBlocks) kb_visc_prims(const StepDev* __restrict__ evs,
                                                      const BItem* __restrict__ items) {
   VH_ITEM
   const EosDev E = A.eos;
@@ -1455,16 +1475,13 @@ static int launch_step_batched_ek(bool viscous, const StepDev* evs, int nev, con
   kb_update_m<<<nb, kBatchBlock, 0, s>>>(evs, items);
   launches++;
   // predictor and corrector; z faces of 2+1D events return at once
-  kb_face<X_, true, EK><<<nb, kBatchBlock, 0, s>>>(evs, items);
-  kb_face<Y_, true, EK><<<nb, kBatchBlock, 0, s>>>(evs, items);
-  kb_face<Z_, true, EK><<<nb, kBatchBlock, 0, s>>>(evs, items);
+  const dim3 fgrid(2 * nb, 3);
+  kb_face<EK><<<fgrid, kBatchBlock, 0, s>>>(evs, items, true);
   kb_update<true, EK><<<nb, kBatchBlock, 0, s>>>(evs, items);
-  kb_face<X_, false, EK><<<nb, kBatchBlock, 0, s>>>(evs, items);
-  kb_face<Y_, false, EK><<<nb, kBatchBlock, 0, s>>>(evs, items);
-  kb_face<Z_, false, EK><<<nb, kBatchBlock, 0, s>>>(evs, items);
+  kb_face<EK><<<fgrid, kBatchBlock, 0, s>>>(evs, items, false);
   kb_update<false, EK><<<nb, kBatchBlock, 0, s>>>(evs, items);
   kb_ghost<false><<<nb, kBatchBlock, 0, s>>>(evs, items);
-  launches += 9;
+  launches += 5;
   if (viscous) {
     kb_visc_prims<EK><<<nb, kBatchBlock, 0, s>>>(evs, items);
     kb_nactive_zero<<<ne, 128, 0, s>>>(evs, nev);

@@ -18,14 +18,33 @@ struct Geo {
   // in [zt0, zt1), and where these planes sit in the whole grid (plane 0 is
   // plane zoff of nzg); the whole grid by default ([2, nz - 2), 0, nz)
   int zc0, zc1, zt0, zt1, zoff, nzg;
+  // x / nx and x / ny of a 31-bit x as a multiply and a shift: (umulhi(mul,
+  // x) + x) >> shift (geo_divisors); mulx 0: N above that range
+  unsigned mulx, muly;
+  int shx, shy;
 };
 
-// the default window of a whole grid
+// Granlund and Montgomery's invariant division (PLDI 1994): s = ceil(log2
+// d), mul = floor(2^32 (2^s - d) / d) + 1; exact for every x < 2^31 (and
+// umulhi(mul, x) + x stays below 2^32 there)
+inline void geo_divisor(unsigned d, unsigned* mul, int* sh) {
+  int s = 0;
+  while ((1ull << s) < d) s++;
+  *sh = s;
+  *mul = (unsigned)((((1ull << s) - d) << 32) / d + 1);
+}
+
+// the default window of a whole grid, and the divisors of its sides
 inline void geo_whole(Geo& g) {
   g.zc0 = g.zt0 = 2;
   g.zc1 = g.zt1 = g.nz - 2;
   g.zoff = 0;
   g.nzg = g.nz;
+  g.mulx = 0;
+  if (g.N < (1LL << 31)) {
+    geo_divisor((unsigned)g.nx, &g.mulx, &g.shx);
+    geo_divisor((unsigned)g.ny, &g.muly, &g.shy);
+  }
 }
 
 // Fluid::getCell index with clamping (src/fld.h:70-78)
@@ -39,7 +58,19 @@ __device__ __forceinline__ long long cidx(const Geo& g, int ix, int iy, int iz) 
   return (long long)ix + (long long)g.nx * iy + (long long)g.nx * g.ny * iz;
 }
 
+// ix, iy, iz of cell i.  The 64-bit divisions of the general form are a
+// call of over a hundred instructions, more than the rest of the index
+// arithmetic of any step kernel.
 __device__ __forceinline__ void coords(const Geo& g, long long i, int& ix, int& iy, int& iz) {
+  if (g.mulx) {
+    const unsigned x = (unsigned)i;
+    const unsigned r = (__umulhi(g.mulx, x) + x) >> g.shx;
+    const unsigned z = (__umulhi(g.muly, r) + r) >> g.shy;
+    ix = (int)(x - r * (unsigned)g.nx);
+    iy = (int)(r - z * (unsigned)g.ny);
+    iz = (int)z;
+    return;
+  }
   ix = (int)(i % g.nx);
   const long long r = i / g.nx;
   iy = (int)(r % g.ny);
@@ -131,7 +162,7 @@ int launch_vorticity(const StepArgs& a, cudaStream_t s);
 
 // Kernel kinds, for per-kernel timing.
 enum KernelKind {
-  KK_UPDATE_M = 0, KK_FACE_X, KK_FACE_Y, KK_FACE_Z, KK_UPDATE, KK_GHOST, KK_VISC_PRIMS,
+  KK_UPDATE_M = 0, KK_FACE, KK_UPDATE, KK_GHOST, KK_VISC_PRIMS,
   KK_IS_RELAX, KK_IS_ADVECT, KK_VISC_UPDATE, KK_VORT, KK_COUNT
 };
 extern const char* const kKernelNames[KK_COUNT];

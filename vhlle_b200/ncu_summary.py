@@ -9,7 +9,7 @@ table of the launch list.
 CSV is ncu's `--csv --log-file` output of a capture of bench.py's timed
 region (`--nvtx --nvtx-include timed/`); GRID is the workload's nx,ny,nz.
 Launches are grouped under the kernel names bench.py's per-kernel profile
-uses (k_face_x/y/z by direction, k_relax_list counted with k_is_relax, the
+uses (k_relax_list counted with k_is_relax, the
 freeze-out kernels as "surface"), each kind's values in launch order.
 """
 from __future__ import annotations
@@ -33,9 +33,6 @@ def kind_of(name: str) -> str:
     base = re.sub(r"^void\s+", "", name).split("(")[0]
     base = base.replace("vh::", "")
     short = base.split("<")[0]
-    if short == "k_face":
-        d = re.search(r"<\s*(\d)", base)
-        return "k_face_" + {"1": "x", "2": "y", "3": "z"}.get(d.group(1) if d else "", "?")
     if short == "k_relax_list":
         return "k_is_relax"
     if any(short.startswith(p) for p in SURFACE):
