@@ -109,3 +109,32 @@ def test_root_find_equals_oracle(eos):
     h.sync()
     assert np.array_equal(out.cpu().numpy().T, o.transform_pv(Q), equal_nan=True)
     h.close()
+
+
+# the faces that can carry a flux are listed where they fill the chip (more
+# than 1184 blocks of 64 faces): sizes on both sides of the line, mostly
+# vacuum, with a filled event and with cells not filled yet (m < 1)
+@pytest.mark.parametrize("nx,ny,nz", [(29, 30, 29), (31, 29, 29), (33, 64, 32), (197, 191, 1), (200, 199, 1)])
+@pytest.mark.parametrize("nb", [0.0, 0.3])
+def test_listed_faces_equal_oracle(nx, ny, nz, nb):
+    if nz > 1:
+        s = W.glauber3d_setup(nx=nx, ny=ny, nz=nz, xmax=14.0, etamax=7.0, b=9.0, nb_peak=nb)
+    else:
+        if nb:
+            pytest.skip("one 2+1D form")
+        s = W.gubser_setup(nx, ny)
+        s.dt = 0.2 * min(s.grid.dx, s.grid.dy)
+        x, y, _ = s.grid.coords()
+        far = (np.hypot(*np.meshgrid(x, y)) > 2.5).reshape(-1)
+        s.Q = s.Q.reshape(7, -1).copy()
+        s.Q[:, far] = 0.
+        s.m = np.where(far, 0., s.m.reshape(-1))
+    rng = np.random.default_rng(4)
+    s.m = np.where((s.m > 0) & (rng.random(s.m.shape) < 0.02), 0.4, s.m)  # matter in cells not filled
+    h, o = capi.GpuHydro(s), P.OracleRun(s)
+    for _ in range(3):
+        h.step(1)
+        assert o.step(1) == 0
+        bad = compare_states(gpu_state_as_oracle(h.get_state()), o.get_state())
+        assert not bad, bad
+    h.close()

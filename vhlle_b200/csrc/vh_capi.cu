@@ -608,6 +608,9 @@ vh_status vh_create(const vh_grid* grid, const vh_eos* eos, const vh_trcoeff* tr
   ALLOC(f.Fx, 7 * N);
   ALLOC(f.Fy, 7 * N);
   ALLOC(f.Fz, 7 * N);
+  ALLOC(f.fact, N);
+  ALLOC(f.flist, 3 * N);
+  ALLOC(f.fcount, 6);
   if (c->viscous) {
     ALLOC(f.flux, 4 * N);
     ALLOC(f.pA, 8 * N);
@@ -1316,10 +1319,10 @@ vh_status vh_sync(vh_ctx* ctx) {
 
 vh_status vh_launches_per_step(vh_ctx* ctx, int* n) {
   if (!ctx || !n) return VH_ERR_ARG;
-  // update_m, 2 x (faces, update), 2 ghost, the viscous five (prims, the
-  // relaxation's list and relaxation, advection, update) and the six of the
+  // update_m, 2 x (face list, faces, update), 2 ghost, the viscous four
+  // (prims, relaxation, advection, update) and the six of the
   // vorticity, the MLP guess, the clock
-  int k = 1 + 2 * (1 + 1) + 1 + (ctx->viscous ? 5 : 0) + 1 +
+  int k = 1 + 2 * (vh::face_lists(ctx->g, 128) ? 3 : 2) + 1 + (ctx->viscous ? 4 : 0) + 1 +
           (ctx->viscous && ctx->vort_on ? 6 : 0) + (ctx->mlp ? 1 : 0) + 1;
   *n = k;
   return VH_OK;

@@ -31,9 +31,10 @@ namespace {
 
 constexpr long long kMaxCells = VH_NOALLOC_MAX_CELLS;
 constexpr int kMaxDim = VH_NOALLOC_MAX_DIM;
-constexpr long long kDoublesPerCell = 81;  // m2 3, Fx/Fy/Fz 21, flux 4, pA 8, pD 4,
+constexpr long long kDoublesPerCell = 83;  // m2 3, Fx/Fy/Fz 21, flux 4, pA 8, pD 4,
                                            // pTh 9, pBC 9, pi0/piH0 20, Pi0/PiH0 2,
-                                           // the active-cell list (ints) 1
+                                           // the active-cell list (ints) 1, the
+                                           // face lists and flags 2
 constexpr size_t kHeaderBytes = 256 + 3 * kMaxDim * sizeof(int) + 3 * kMaxDim;  // err, maps
 constexpr size_t kHeaderAligned = (kHeaderBytes + 255) / 256 * 256;
 constexpr size_t kScratchBytes = kHeaderAligned + (size_t)kDoublesPerCell * kMaxCells * sizeof(double);
@@ -200,7 +201,7 @@ extern "C" vh_status vh_step_noalloc(const vh_grid* grid, const vh_eos* eos_dev,
                    tr->zetaSWidthT};
   a.viscous = tr->etaS0 > 0. || tr->zetaS0 > 0. || tr->etaSparam > 0 || tr->zetaSparam > 0;
 
-  // scratch layout: [err, clock, active count | ghost src maps | ghost dst
+  // scratch layout: [err, clock, active and face counts | ghost src maps | ghost dst
   // flags | pad][doubles...]
   vh::Fields& f = a.f;
   f.err = reinterpret_cast<unsigned*>(base);
@@ -237,6 +238,10 @@ extern "C" vh_status vh_step_noalloc(const vh_grid* grid, const vh_eos* eos_dev,
   f.PiH0 = d;
   d += N;
   f.active = reinterpret_cast<int*>(d);
+  d += N;
+  f.flist = reinterpret_cast<int*>(d);
+  f.fact = reinterpret_cast<unsigned char*>(f.flist + 3 * N);
+  f.fcount = reinterpret_cast<int*>(base + 64);
   f.Q = s->Q;
   f.Qh = s->Qh;
   f.Qprev = s->Qprev;

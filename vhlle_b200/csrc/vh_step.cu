@@ -31,9 +31,13 @@ constexpr int kFaceMinBlocks = 8, kUpdateMinBlocks = 6, kPrimsMinBlocks = 7;
 // Fluid::updateM, src/fld.cpp:384-423 (both passes; out of place).
 __device__ __forceinline__ void d_update_m(const Geo& g, const double* __restrict__ m,
                                            double* __restrict__ mo, const double* __restrict__ clk,
+                                           int* __restrict__ fcount, int* __restrict__ nactive,
                                            long long blk) {
   const double tau = clk[0], dt = clk[1];  // the step's clock (device)
   const long long i = blk * blockDim.x + threadIdx.x;
+  // the step's list counters, filled by later kernels
+  if (i < 6) fcount[i] = 0;
+  if (i == 0 && nactive) *nactive = 0;
   if (i >= g.N) return;
   int ix, iy, iz;
   coords(g, i, ix, iy, iz);
@@ -68,46 +72,139 @@ __device__ __forceinline__ void d_update_m(const Geo& g, const double* __restric
   mo[2 * N + i] = a2;
 }
 __global__ void k_update_m(Geo g, const double* __restrict__ m, double* __restrict__ mo,
-                           const double* __restrict__ clk) {
-  d_update_m(g, m, mo, clk, blockIdx.x);
+                           const double* __restrict__ clk, int* __restrict__ fcount,
+                           int* __restrict__ nactive) {
+  d_update_m(g, m, mo, clk, fcount, nactive, blockIdx.x);
 }
 
+
+// ------------------------------------------------------------ face lists
+// The faces that can carry a flux, one list per direction (cell i for its
+// face on the + side).  Most of a grid is vacuum (80 to 92 % of the cells of
+// the 3D events in their first steps, 30 % late), and a face between two
+// empty edges, or between two cells that are not filled yet, adds nothing
+// (src/hdo.cpp:118-144): with the faces taken in grid order the root finds
+// ran on 39 to 51 % of their warps' lanes, on packed lists on 87 %.  A face
+// off the list has no flux in memory either (fact), so its 56 bytes are
+// neither written nor read.
+//
+// Exact: an edge with Q_t <= 0 is vacuum to transform_pv; hlle_flux returns
+// for two vacuum edges, and for two unfilled cells unless it stops the run
+// for e > 1e10, which e <= Q_t / tau rules out.  Lists are in block order,
+// which varies; no face's flux depends on it.
+__device__ __forceinline__ void d_face_list(const Geo& g, const double* __restrict__ QT,
+                                            const double* __restrict__ m,
+                                            unsigned char* __restrict__ fact,
+                                            int* __restrict__ flist, int* __restrict__ fcount,
+                                            const double* __restrict__ clk, long long blk) {
+  __shared__ int wcnt[3][4], base[3];
+  const long long i = blk * blockDim.x + threadIdx.x;
+  const long long N = g.N;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  unsigned act = 0;
+  if (i < N) {
+    int ix, iy, iz;
+    coords(g, i, ix, iy, iz);
+    const int cc[3] = {ix, iy, iz}, nn[3] = {g.nx, g.ny, g.nz};
+    const long long ss[3] = {1, g.nx, (long long)g.nx * g.ny};
+    const double x1 = QT[i], huge = 0.9e10 * clk[0];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      if (cc[d] >= nn[d] - 1) continue;
+      const long long st = ss[d];
+      const double x2 = QT[i + st];
+      const double x0 = cc[d] > 0 ? QT[i - st] : x1, x3 = cc[d] < nn[d] - 2 ? QT[i + 2 * st] : x2;
+      const double el = x1 + minmod((x2 - x1) / 2., (x1 - x0) / 2.);
+      const double er = x2 - minmod((x3 - x2) / 2., (x2 - x1) / 2.);
+      if (el <= 0. && er <= 0.) continue;
+      if (m[d * N + i] < 1. && m[d * N + i + st] < 1. && el <= huge) continue;
+      act |= 1u << d;
+    }
+    fact[i] = (unsigned char)act;
+  }
+  unsigned bal[3];
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    bal[d] = __ballot_sync(0xffffffffu, (act >> d) & 1u);
+    if (lane == 0) wcnt[d][warp] = __popc(bal[d]);
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    int n = 0;
+    for (int w = 0; w < nw; w++) n += wcnt[threadIdx.x][w];
+    base[threadIdx.x] = n ? atomicAdd(fcount + threadIdx.x, n) : 0;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    if (!((act >> d) & 1u)) continue;
+    int at = base[d] + __popc(bal[d] & ((1u << lane) - 1u));
+    for (int w = 0; w < warp; w++) at += wcnt[d][w];
+    flist[d * N + at] = (int)i;
+  }
+}
+__global__ void __launch_bounds__(128) k_face_list(Geo g, const double* __restrict__ QT,
+                                                   const double* __restrict__ m,
+                                                   unsigned char* __restrict__ fact,
+                                                   int* __restrict__ flist,
+                                                   int* __restrict__ fcount,
+                                                   const double* __restrict__ clk) {
+  d_face_list(g, QT, m, fact, flist, fcount, clk, blockIdx.x);
+}
 
 // ------------------------------------------------------------ face flux
-// One HLLE face between cell i and its neighbour on the + side along `dir`
-// (Hydro::hlle_flux with Cell::getPrimVarRight / getPrimVarLeft or their H
-// variants, src/cll.cpp:106-204).  F[c*N + i] holds the flux of the face on
-// the + side of cell i (0 where the reference adds nothing).
+// One HLLE face between cell i and its neighbour on the + side along a
+// direction (Hydro::hlle_flux with Cell::getPrimVarRight / getPrimVarLeft or
+// their H variants, src/cll.cpp:106-204), for the listed faces.  F[c*N + i]
+// holds the flux of the face on the + side of cell i (0 where the reference
+// adds nothing).
 //
-// A block of B threads takes B / 2 faces: thread t < B/2 reconstructs and
-// solves the left state of face t, thread t + B/2 its right state, the
-// primitives meet in shared memory, and the first half of the block forms
-// the fluxes.  One launch holds the faces of every direction (the direction
-// of a block a run-time number), so the directions share one instruction
-// stream, and there is one ragged end per pass instead of three.
+// A block of B threads takes B / 2 faces of one direction: thread t < B/2
+// reconstructs and solves the left state of face t, thread t + B/2 its right
+// state, the primitives meet in shared memory, and the first half of the
+// block forms the fluxes.  One launch holds the faces of every direction
+// (the direction of a block a run-time number), so the directions share one
+// instruction stream, and there is one ragged end per pass instead of three.
 // A thread that solved both states of a face (three kernels of 16 thousand
 // warps) spent 5.6 of 14 cycles per issue waiting for instructions; in this
-// form it is 0.5 of 9, and 101x101x51 takes 280 us of faces per step instead
-// of 492 (2 passes, baryon-free, 20 % of the cells with matter).
-static inline unsigned face_blocks(long long N, int bs) {
-  return (unsigned)((N + bs / 2 - 1) / (bs / 2));
+// form it is 0.5 of 9.  101x101x51, two passes, 20 % of the cells with
+// matter: 492 us a step in that form, 280 in this one over the whole grid,
+// 153 over the lists (with the list kernels).
+struct FaceBatch {
+  int cnt[3], blocks[3];  // listed faces, and blocks of B / 2 of them, per direction
+};
+// without lists every cell stands for its faces
+__device__ __forceinline__ FaceBatch face_batch(const Geo& g, const int* __restrict__ fcount) {
+  FaceBatch b;
+  const int half = blockDim.x >> 1;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    b.cnt[d] = fcount ? fcount[d] : (d < 2 || g.nz > 1 ? (int)g.N : 0);
+    b.blocks[d] = (b.cnt[d] + half - 1) / half;
+  }
+  return b;
 }
 template <int EK>
-__device__ __forceinline__ void d_face(const Geo& g, const EosDev& E, bool predict, int dir,
-                                       const double* __restrict__ QQ,
-                                       const double* __restrict__ m, double* __restrict__ F,
-                                       const double* __restrict__ clk, unsigned* err,
-                                       long long blk) {
+__device__ __forceinline__ void d_face(const Geo& g, const EosDev& E, bool predict,
+                                       const FaceBatch& fb, const double* __restrict__ QQ,
+                                       const double* __restrict__ m, double* __restrict__ Fx,
+                                       double* __restrict__ Fy, double* __restrict__ Fz,
+                                       const int* __restrict__ flist,
+                                       const double* __restrict__ clk, unsigned* err, int b) {
   __shared__ double sp[8][128];
   const int half = blockDim.x >> 1, t = threadIdx.x;
   const bool right = t >= half;
+  const int dir = b < fb.blocks[0] ? X_ : (b < fb.blocks[0] + fb.blocks[1] ? Y_ : Z_);
+  const int first = dir == X_ ? 0 : (dir == Y_ ? fb.blocks[0] : fb.blocks[0] + fb.blocks[1]);
+  const int at = (b - first) * half + (right ? t - half : t);
+  const int cnt = dir == X_ ? fb.cnt[0] : (dir == Y_ ? fb.cnt[1] : fb.cnt[2]);
   const double tau = clk[0], dt = clk[1];  // the step's clock (device)
-  const long long i = blk * half + (right ? t - half : t);
   const long long N = g.N;
   const long long st = dir == X_ ? 1 : (dir == Y_ ? g.nx : (long long)g.nx * g.ny);
-  bool face = false;  // a face of the grid
+  bool face = at < cnt;
+  const long long i = !face ? 0 : (flist ? flist[(dir - 1) * N + at] : at);
   int c = 0, n = 0;
-  if (i < N) {
+  if (face) {
     int ix, iy, iz;
     coords(g, i, ix, iy, iz);
     c = dir == X_ ? ix : (dir == Y_ ? iy : iz);
@@ -150,6 +247,7 @@ __device__ __forceinline__ void d_face(const Geo& g, const EosDev& E, bool predi
     return Prim{sp[0][s], sp[1][s], sp[2][s], sp[3][s], sp[4][s], sp[5][s], sp[6][s], sp[7][s]};
   };
   const double dxdir = dir == X_ ? g.dx : (dir == Y_ ? g.dy : g.dz);
+  double* F = dir == X_ ? Fx : (dir == Y_ ? Fy : Fz);
   double fl[7];
   unsigned e = 0;
   const bool ok = hlle_face(dir, predict, tau, dt, dxdir, prim(t), prim(t + half),
@@ -158,16 +256,20 @@ __device__ __forceinline__ void d_face(const Geo& g, const EosDev& E, bool predi
 #pragma unroll
   for (int k = 0; k < 7; k++) F[k * N + i] = ok ? fl[k] : 0.;
 }
-// nbd blocks per direction, X first
+// resident blocks that walk the listed faces (their number is known on the
+// device only); flist and fcount null: every face
 template <int EK>
 __global__ void __launch_bounds__(128, kFaceMinBlocks) k_face(
-    Geo g, EosDev E, bool predict, unsigned nbd, const double* __restrict__ QQ,
-    const double* __restrict__ m, double* __restrict__ Fx, double* __restrict__ Fy,
-    double* __restrict__ Fz, const double* __restrict__ clk, unsigned* err) {
-  const unsigned b = blockIdx.x;
-  const int dir = b < nbd ? X_ : (b < 2 * nbd ? Y_ : Z_);
-  d_face<EK>(g, E, predict, dir, QQ, m, dir == X_ ? Fx : (dir == Y_ ? Fy : Fz), clk, err,
-             b - (dir - 1) * nbd);
+    Geo g, EosDev E, bool predict, const double* __restrict__ QQ, const double* __restrict__ m,
+    double* __restrict__ Fx, double* __restrict__ Fy, double* __restrict__ Fz,
+    const int* __restrict__ flist, const int* __restrict__ fcount, const double* __restrict__ clk,
+    unsigned* err) {
+  const FaceBatch fb = face_batch(g, fcount);
+  const int nb = fb.blocks[0] + fb.blocks[1] + fb.blocks[2];
+  for (int b = blockIdx.x; b < nb; b += gridDim.x) {
+    d_face<EK>(g, E, predict, fb, QQ, m, Fx, Fy, Fz, flist, clk, err, b);
+    __syncthreads();  // the shared primitives are read
+  }
 }
 
 
@@ -181,6 +283,7 @@ __device__ __forceinline__ void d_update(const Geo& g, const EosDev& E, double* 
                                          const double* __restrict__ Fx,
                                          const double* __restrict__ Fy,
                                          const double* __restrict__ Fz,
+                                         const unsigned char* __restrict__ fact,
                                          const double* __restrict__ clk, unsigned* err,
                                          double* __restrict__ pB, double* __restrict__ pA,
                                          long long blk) {
@@ -191,24 +294,65 @@ __device__ __forceinline__ void d_update(const Geo& g, const EosDev& E, double* 
   coords(g, i, ix, iy, iz);
   const long long N = g.N;
   const long long sy = g.nx, sz = (long long)g.nx * g.ny;
+  const double* field = PRED ? Q : Qh;
+  const double tau1 = PRED ? tau : tau + 0.5 * dt;
+  const double _dt = PRED ? dt / 2. : dt;
+  // which of the six faces carry a flux (d_face_list; without lists all)
+  bool xm = ix > 0, ym = iy > 0, zm = iz > 0;
+  bool xp = ix < g.nx - 1, yp = iy < g.ny - 1, zp = iz < g.nz - 1;
+  if (fact) {
+    const unsigned fi = fact[i];
+    xp = fi & 1u;
+    yp = fi & 2u;
+    zp = fi & 4u;
+    if (xm) xm = fact[i - 1] & 1u;
+    if (ym) ym = fact[i - sy] & 2u;
+    if (zm) zm = fact[i - sz] & 4u;
+  }
+  const bool faces = xm | xp | ym | yp | zm | zp;
+  double q[7], qin[7];
+  qin[T_] = field[i];
+  qin[Z_] = field[3 * N + i];
+  // vacuum that nothing flows into: no flux, no source, the row stays
+  const bool still = !faces && qin[T_] <= 0. && qin[Z_] == 0.;
+  if (!PRED && still) {
+    if (pA) {
+      pA[i] = 0.;  // e and v are read of empty cells too, the rest of none
+#pragma unroll
+      for (int k = 5; k < 8; k++) pA[k * N + i] = 0.;
+    }
+    return;
+  }
+#pragma unroll
+  for (int k = 1; k < 7; k++)
+    if (k != Z_) qin[k] = field[k * N + i];
+  if (PRED && still) {
+#pragma unroll
+    for (int k = 0; k < 7; k++) {
+      Qprev[k * N + i] = qin[k];
+      Qh[k * N + i] = qin[k];
+    }
+    // pB is read of cells with matter at the half step: not of this one,
+    // unless the ghost copy puts matter there
+    if (pB && (ix < 2 || ix >= g.nx - 2 || iy < 2 || iy >= g.ny - 2 || iz < 2 || iz >= g.nz - 2)) {
+      pB[i] = 1.;
+#pragma unroll
+      for (int k = 1; k < 5; k++) pB[k * N + i] = 0.;
+    }
+    return;
+  }
   double fl[7];
 #pragma unroll
   for (int k = 0; k < 7; k++) {
     double a = 0.;
-    if (ix > 0) a += Fx[k * N + i - 1];
-    if (ix < g.nx - 1) a += -Fx[k * N + i];
-    if (iy > 0) a += Fy[k * N + i - sy];
-    if (iy < g.ny - 1) a += -Fy[k * N + i - 0];
-    if (iz > 0) a += Fz[k * N + i - sz];
-    if (iz < g.nz - 1) a += -Fz[k * N + i];
+    if (xm) a += Fx[k * N + i - 1];
+    if (xp) a += -Fx[k * N + i];
+    if (ym) a += Fy[k * N + i - sy];
+    if (yp) a += -Fy[k * N + i];
+    if (zm) a += Fz[k * N + i - sz];
+    if (zp) a += -Fz[k * N + i];
     fl[k] = a;
   }
-  const double* field = PRED ? Q : Qh;
-  const double tau1 = PRED ? tau : tau + 0.5 * dt;
-  const double _dt = PRED ? dt / 2. : dt;
-  double q[7], qin[7];
-#pragma unroll
-  for (int k = 0; k < 7; k++) qin[k] = field[k * N + i];
   q_over(qin, tau1, q);
   Prim pp;
   transform_pv<EK>(E, q, pp, c2p_guess(E, i));
@@ -255,9 +399,8 @@ __device__ __forceinline__ void d_update(const Geo& g, const EosDev& E, double* 
   if (PRED) {
 #pragma unroll
     for (int k = 0; k < 7; k++) {
-      const double qk = Q[k * N + i];
-      Qprev[k * N + i] = qk;
-      Qh[k * N + i] = qk + fl[k];
+      Qprev[k * N + i] = qin[k];
+      Qh[k * N + i] = qin[k] + fl[k];
     }
   } else {
     if (!(Q[i] + fl[0] < 0.)) {
@@ -272,9 +415,11 @@ __global__ void __launch_bounds__(128, kUpdateMinBlocks) k_update(Geo g, EosDev 
                                                 double* __restrict__ Qprev,
                                                 const double* __restrict__ Fx,
                                                 const double* __restrict__ Fy,
-                                                const double* __restrict__ Fz, const double* __restrict__ clk, unsigned* err,
+                                                const double* __restrict__ Fz,
+                                                const unsigned char* __restrict__ fact,
+                                                const double* __restrict__ clk, unsigned* err,
                                                 double* __restrict__ pB, double* __restrict__ pA) {
-  d_update<PRED, EK>(g, E, Q, Qh, Qprev, Fx, Fy, Fz, clk, err, pB, pA, blockIdx.x);
+  d_update<PRED, EK>(g, E, Q, Qh, Qprev, Fx, Fy, Fz, fact, clk, err, pB, pA, blockIdx.x);
 }
 
 
@@ -347,6 +492,19 @@ __global__ void k_ghost(Geo g, const int* __restrict__ src, const unsigned char*
 __device__ __forceinline__ double maxM_at(const Geo& g, const double* __restrict__ m, int ix,
                                           int iy, int iz);
 
+__device__ __forceinline__ Prim loadA(const double* __restrict__ pA, long long N, long long i) {
+  Prim a;
+  a.e = pA[i];
+  a.p = pA[N + i];
+  a.nb = pA[2 * N + i];
+  a.nq = pA[3 * N + i];
+  a.ns = pA[4 * N + i];
+  a.vx = pA[5 * N + i];
+  a.vy = pA[6 * N + i];
+  a.vz = pA[7 * N + i];
+  return a;
+}
+
 template <int EK>
 __device__ __forceinline__ void d_visc_prims(const Geo& g, const EosDev& E, const TrDev& tr,
                                              const double* __restrict__ Q,
@@ -357,49 +515,64 @@ __device__ __forceinline__ void d_visc_prims(const Geo& g, const EosDev& E, cons
                                              double* __restrict__ pBC,
                                              const double* __restrict__ clk,
                                              const unsigned char* __restrict__ isdst,
-                                             long long blk) {
+                                             int* __restrict__ active,
+                                             int* __restrict__ nactive, long long blk) {
   const double dt = clk[1], tau = clk[0] + dt;  // tau_{n+1} (src/hdo.cpp:1095)
   const long long i = blk * blockDim.x + threadIdx.x;
-  if (i >= g.N) return;
   const long long N = g.N;
   double q[7], qh[7];
-#pragma unroll
-  for (int k = 0; k < 7; k++) qh[k] = Qh[k * N + i];
   const double tA = tau - dt / 2.;
-  Prim a;
-  int gx, gy, gz;
-  coords(g, i, gx, gy, gz);
-  // A is the corrector's con2prim (k_update<false> stored it in pA) when
-  // its divisor tau_n + dt/2 equals tA bit for bit and the ghost copy has
-  // not changed this cell's Qh since
-  if (tA == clk[0] + 0.5 * dt && !(isdst[gx] | isdst[g.nx + gy] | isdst[g.nx + g.ny + gz])) {
-    a.e = pA[0 * N + i];
-    a.p = pA[1 * N + i];
-    a.nb = pA[2 * N + i];
-    a.nq = pA[3 * N + i];
-    a.ns = pA[4 * N + i];
-    a.vx = pA[5 * N + i];
-    a.vy = pA[6 * N + i];
-    a.vz = pA[7 * N + i];
-  } else {
-    q_over(qh, tA, q);
-    transform_pv<EK>(E, q, a, c2p_guess(E, i));
-    pA[0 * N + i] = a.e;
-    pA[1 * N + i] = a.p;
-    pA[2 * N + i] = a.nb;
-    pA[3 * N + i] = a.nq;
-    pA[4 * N + i] = a.ns;
-    pA[5 * N + i] = a.vx;
-    pA[6 * N + i] = a.vy;
-    pA[7 * N + i] = a.vz;
+  Prim a{0., 0., 0., 0., 0., 0., 0., 0.};
+  int gx = 0, gy = 0, gz = 0;
+  if (i < N) {
+    coords(g, i, gx, gy, gz);
+    qh[0] = Qh[i];
+    // A is the corrector's con2prim (k_update<false> stored it in pA) when
+    // its divisor tau_n + dt/2 equals tA bit for bit and the ghost copy has
+    // not changed this cell's Qh since
+    if (tA == clk[0] + 0.5 * dt && !(isdst[gx] | isdst[g.nx + gy] | isdst[g.nx + g.ny + gz])) {
+      a = loadA(pA, N, i);
+    } else {
+#pragma unroll
+      for (int k = 1; k < 7; k++) qh[k] = Qh[k * N + i];
+      q_over(qh, tA, q);
+      transform_pv<EK>(E, q, a, c2p_guess(E, i));
+      pA[0 * N + i] = a.e;
+      pA[1 * N + i] = a.p;
+      pA[2 * N + i] = a.nb;
+      pA[3 * N + i] = a.nq;
+      pA[4 * N + i] = a.ns;
+      pA[5 * N + i] = a.vx;
+      pA[6 * N + i] = a.vy;
+      pA[7 * N + i] = a.vz;
+    }
   }
-  q_over(qh, tau, q);
-  Prim d;
-  transform_pv<EK>(E, q, d, c2p_guess(E, i));
-  pD[0 * N + i] = d.e;
-  pD[1 * N + i] = d.vx;
-  pD[2 * N + i] = d.vy;
-  pD[3 * N + i] = d.vz;
+  {
+    // the list of cells with matter, for the relaxation and the advection:
+    // packed in warp order (one atomic per warp; the order between warps
+    // varies, and every cell's result depends on that cell alone)
+    const bool act = i < N && !(a.e <= 0.);
+    const int lane = threadIdx.x & 31;
+    const unsigned bal = __ballot_sync(0xffffffffu, act);
+    int base = 0;
+    if (lane == 0 && bal) base = atomicAdd(nactive, __popc(bal));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (act) active[base + __popc(bal & ((1u << lane) - 1u))] = (int)i;
+  }
+  if (i >= N) return;
+  if (qh[0] <= 0.) {  // vacuum: the neighbours read e first, and stop there
+    pD[i] = 0.;
+  } else {
+#pragma unroll
+    for (int k = 1; k < 7; k++) qh[k] = Qh[k * N + i];
+    q_over(qh, tau, q);
+    Prim d;
+    transform_pv<EK>(E, q, d, c2p_guess(E, i));
+    pD[0 * N + i] = d.e;
+    pD[1 * N + i] = d.vx;
+    pD[2 * N + i] = d.vy;
+    pD[3 * N + i] = d.vz;
+  }
   if (a.e <= 0.) return;
   {
     double T, mub, mus, p;
@@ -420,8 +593,7 @@ __device__ __forceinline__ void d_visc_prims(const Geo& g, const EosDev& E, cons
     pTh[7 * N + i] = tauPi;
     pTh[8 * N + i] = 9. / 70. / p;  // eos_p at the same point is this p
   }
-  int ix, iy, iz;
-  coords(g, i, ix, iy, iz);
+  const int ix = gx, iy = gy, iz = gz;
   const bool vac = maxM_at(g, m, ix + 1, iy, iz) <= 0.9 || maxM_at(g, m, ix, iy + 1, iz) <= 0.9 ||
                    maxM_at(g, m, ix - 1, iy, iz) <= 0.9 || maxM_at(g, m, ix, iy - 1, iz) <= 0.9 ||
                    maxM_at(g, m, ix + 1, iy + 1, iz) <= 0.9 ||
@@ -461,8 +633,11 @@ __global__ void __launch_bounds__(128, kPrimsMinBlocks) k_visc_prims(Geo g, EosD
                                                     double* __restrict__ pD,
                                                     double* __restrict__ pTh,
                                                     double* __restrict__ pBC, const double* __restrict__ clk,
-                                                    const unsigned char* __restrict__ isdst) {
-  d_visc_prims<EK>(g, E, tr, Q, Qprev, Qh, m, pA, pD, pTh, pBC, clk, isdst, blockIdx.x);
+                                                    const unsigned char* __restrict__ isdst,
+                                                    int* __restrict__ active,
+                                                    int* __restrict__ nactive) {
+  d_visc_prims<EK>(g, E, tr, Q, Qprev, Qh, m, pA, pD, pTh, pBC, clk, isdst, active, nactive,
+                   blockIdx.x);
 }
 
 
@@ -471,25 +646,15 @@ __device__ __forceinline__ double maxM_at(const Geo& g, const double* __restrict
   return maxM(m, g.N, cidx(g, ix, iy, iz));
 }
 
-__device__ __forceinline__ Prim loadA(const double* __restrict__ pA, long long N, long long i) {
-  Prim a;
-  a.e = pA[i];
-  a.p = pA[N + i];
-  a.nb = pA[2 * N + i];
-  a.nq = pA[3 * N + i];
-  a.ns = pA[4 * N + i];
-  a.vx = pA[5 * N + i];
-  a.vy = pA[6 * N + i];
-  a.vz = pA[7 * N + i];
-  return a;
-}
-
 // ------------------------------------------------ ISformal, loop #1
 // Hydro::ISformal loop 1 with Hydro::NSquant (src/hdo.cpp:381-652,
 // 690-864): Navier-Stokes shear/bulk from the velocity gradients, then the
 // two-stage Israel-Stewart relaxation with Christoffel and cross terms.
 // Writes pi0/piH0/Pi0/PiH0 and the first flux contribution
-// (+(tau-dt) * delta Q_n).  One thread per cell, every index a compile-time
+// (+(tau-dt) * delta Q_n) of the cells with matter; the zeros of the empty
+// ones (src/hdo.cpp:697-708) are left to their readers, which see e <= 0
+// (writing them, 208 bytes a cell, took 25 us of a 988 us step at 101x101x51
+// with 80 % vacuum).  One thread per cell, every index a compile-time
 // constant; the con2prims and the thermodynamics come precomputed from
 // k_visc_prims.  Four 128-thread blocks per SM (128 registers) hide the FP64
 // latency better than fewer, spill-free ones (measured: 3 and 2 blocks per SM
@@ -503,50 +668,6 @@ constexpr int kRelaxBlock = 128;
 constexpr int kSmPI = 0, kSmSIG = 10, kSmU = 20, kSmH = 24, kSmF = 34, kSmY = 44, kSmRows = 54;
 constexpr size_t kRelaxSmem = sizeof(double) * kSmRows * kRelaxBlock;
 
-// The empty cells' share of ISformal loop 1 (src/hdo.cpp:697-708: zero
-// pi0/piH0/Pi0/PiH0) and the list of the other cells, so that k_is_relax
-// runs full warps: cells with matter are packed in warp order (one atomic
-// per warp; the list's order between warps varies, and every cell's result
-// depends on that cell alone).  *nactive is zero on entry.
-__device__ __forceinline__ void d_relax_list(const Geo& g, const double* __restrict__ pA,
-                                             int* __restrict__ active, int* __restrict__ nactive,
-                                             double* __restrict__ pi0, double* __restrict__ piH0,
-                                             double* __restrict__ Pi0, double* __restrict__ PiH0,
-                                             double* __restrict__ flux, long long blk) {
-  const long long i = blk * blockDim.x + threadIdx.x;
-  const long long N = g.N;
-  const bool in = i < N;
-  const bool act = in && !(pA[i] <= 0.);
-  const int lane = threadIdx.x & 31;
-  const unsigned bal = __ballot_sync(0xffffffffu, act);
-  int base = 0;
-  if (lane == 0 && bal) base = atomicAdd(nactive, __popc(bal));
-  base = __shfl_sync(0xffffffffu, base, 0);
-  if (act) active[base + __popc(bal & ((1u << lane) - 1u))] = (int)i;
-  if (in && !act) {
-#pragma unroll
-    for (int k = 0; k < 10; k++) {
-      piH0[k * N + i] = 0.0;
-      pi0[k * N + i] = 0.0;
-    }
-    PiH0[i] = 0.0;
-    Pi0[i] = 0.0;
-#pragma unroll
-    for (int k = 0; k < 4; k++) flux[k * N + i] = 0.;
-  }
-}
-__global__ void __launch_bounds__(128) k_relax_list(Geo g, const double* __restrict__ pA,
-                                                    int* __restrict__ active,
-                                                    int* __restrict__ nactive,
-                                                    double* __restrict__ pi0,
-                                                    double* __restrict__ piH0,
-                                                    double* __restrict__ Pi0,
-                                                    double* __restrict__ PiH0,
-                                                    double* __restrict__ flux) {
-  d_relax_list(g, pA, active, nactive, pi0, piH0, Pi0, PiH0, flux, blockIdx.x);
-}
-
-
 __device__ __forceinline__ void d_is_relax(
     const Geo& g, const EosDev& E, const TrDev& tr, const double* __restrict__ Q,
     const double* __restrict__ Qprev, const double* __restrict__ m, const double* __restrict__ pA,
@@ -559,7 +680,7 @@ __device__ __forceinline__ void d_is_relax(
   const double dt = clk[1], tau = clk[0] + dt;  // tau_{n+1} (src/hdo.cpp:1095)
   const int idx = (int)(blk * blockDim.x + threadIdx.x);
   if (idx >= *nactive) return;
-  const long long i = active[idx];  // a cell with matter (k_relax_list)
+  const long long i = active[idx];  // a cell with matter (k_visc_prims)
   const long long N = g.N;
   const double e = pA[i];
   int ix, iy, iz;
@@ -966,7 +1087,7 @@ __device__ __forceinline__ void d_is_advect(const Geo& g, const double* __restri
                                             const int* __restrict__ active,
                                             const int* __restrict__ nactive, long long blk) {
   const double dt = clk[1], tau = clk[0] + dt;  // tau_{n+1} (src/hdo.cpp:1095)
-  // the cells with matter only (k_relax_list); the empty ones are left as
+  // the cells with matter only (k_visc_prims); the empty ones are left as
   // they are, as the reference's loop 2 leaves them (e <= 0)
   const int idx = (int)(blk * blockDim.x + threadIdx.x);
   if (idx >= *nactive) return;
@@ -999,6 +1120,7 @@ __device__ __forceinline__ void d_is_advect(const Geo& g, const double* __restri
 #pragma unroll
       for (int jz = 0; jz < 2; jz++) {
         const long long c1 = cidx(g, ix + jx * sx, iy + jy * sy, iz + jz * sz);
+        if (jx + jy + jz > 0 && pA[c1] <= 0.) continue;  // an empty cell: zeros
         const double w = wx[jx] * wy[jy] * wz[jz];
         const double wH = wxH[jx] * wyH[jy] * wzH[jz];
 #pragma unroll
@@ -1126,13 +1248,27 @@ __device__ __forceinline__ void d_visc_update(const Geo& g, const double* __rest
   int ix, iy, iz;
   coords(g, i, ix, iy, iz);
   const long long N = g.N;
-  double fl[4];
-#pragma unroll
-  for (int k = 0; k < 4; k++) fl[k] = flux[k * N + i];
+  // an empty cell has no flux so far, and between unfilled cells none comes
+  const double e = pA[i];
+  const bool empty = e <= 0.;
   double f[4];
   const long long st[3] = {1, g.nx, (long long)g.nx * g.ny};
   const int cc[3] = {ix, iy, iz};
   const int nn[3] = {g.nx, g.ny, g.nz};
+  if (empty) {
+    bool any = false;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      const double* md = m + d * N;
+      const bool own = !(md[i] < 1.);
+      any |= cc[d] > 0 && (own || !(md[i - st[d]] < 1.));
+      any |= cc[d] < nn[d] - 1 && (own || !(md[i + st[d]] < 1.));
+    }
+    if (!any) return;
+  }
+  double fl[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) fl[k] = empty ? 0. : flux[k * N + i];
 #pragma unroll
   for (int d = 0; d < 3; d++) {
     const double dxa = visc_dxa(d + 1, tau, dt, g), rdxa = 1.0 / dxa;
@@ -1146,8 +1282,7 @@ __device__ __forceinline__ void d_visc_update(const Geo& g, const double* __rest
       for (int k = 0; k < 4; k++) fl[k] += -f[k];
     }
   }
-  const double e = pA[i];
-  if (!(e <= 0.)) {
+  if (!empty) {
     const double vx = pA[5 * N + i], vy = pA[6 * N + i], vz = pA[7 * N + i];
     double uuu[4];
     uuu[0] = 1. / sqrt(1. - vx * vx - vy * vy - vz * vz);
@@ -1211,6 +1346,18 @@ __global__ void k_transform_pv(EosDev E, const double* __restrict__ Q, long long
 // ------------------------------------------------------------ launcher
 static inline unsigned nblk(long long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
+static long long face_blocks(const Geo& g, int bs) {
+  return (g.nz > 1 ? 3LL : 2LL) * nblk(g.N, bs / 2);
+}
+static long long face_resident(int bs) { return 148LL * kFaceMinBlocks * (128 / bs); }
+// Where the faces do not fill one resident set of blocks the step is a chain
+// of latencies, and the lists (a kernel more in it, and the emptiest warps
+// of a grid that leaves the chip idle anyway) do not pay: 101x101x1, 320
+// blocks of 1184, 48 us a step with lists and 39 without; 47x61x23, 3093
+// blocks, 192 with and 223 without.
+bool face_lists(const Geo& g, int bs) { return face_blocks(g, bs) > face_resident(bs); }
+
+
 const char* const kKernelNames[KK_COUNT] = {
     "k_update_m", "k_face", "k_update", "k_ghost",
     "k_visc_prims", "k_is_relax", "k_is_advect", "k_visc_update",
@@ -1223,28 +1370,37 @@ static int launch_step_ek(const StepArgs& a, cudaStream_t s, LaunchMarker* mk) {
   const int bs = a.block == 64 ? 64 : 128;
   const unsigned nb = nblk(g.N, bs);
   const unsigned nb128 = nblk(g.N, 128);
+  // one resident set of blocks for the faces
+  const long long fblocks = face_blocks(g, bs), resident = face_resident(bs);
+  const bool lists = face_lists(g, bs);
+  const unsigned nface = (unsigned)std::min(fblocks, resident);
+  const unsigned char* fact = lists ? a.f.fact : nullptr;
   int launches = 0;
   const Fields& F = a.f;
   auto done = [&](int kind) {
     launches++;
     if (mk) mk->after(kind);
   };
-  k_update_m<<<nb, bs, 0, s>>>(g, F.m, F.m2, a.clk);
+  k_update_m<<<nb, bs, 0, s>>>(g, F.m, F.m2, a.clk, F.fcount, a.viscous ? F.nactive : nullptr);
   done(KK_UPDATE_M);
   const double* m = F.m2;  // the updated fill fractions
   // predictor (src/hdo.cpp:1023-1060) and corrector (src/hdo.cpp:1062-1094)
   for (int pass = 0; pass < 2; pass++) {
     const bool pred = pass == 0;
     const double* QQ = pred ? F.Q : F.Qh;
-    const unsigned nbd = face_blocks(g.N, bs);
-    k_face<EK><<<nbd * (g.nz > 1 ? 3 : 2), bs, 0, s>>>(g, a.eos, pred, nbd, QQ, m, F.Fx, F.Fy, F.Fz,
-                                                       a.clk, F.err);
+    int* fcount = lists ? F.fcount + 3 * pass : nullptr;
+    if (lists) {
+      k_face_list<<<nb, bs, 0, s>>>(g, QQ, m, F.fact, F.flist, fcount, a.clk);
+      launches++;
+    }
+    k_face<EK><<<nface, bs, 0, s>>>(g, a.eos, pred, QQ, m, F.Fx, F.Fy, F.Fz,
+                                    lists ? F.flist : nullptr, fcount, a.clk, F.err);
     done(KK_FACE);
     if (pred)
-      k_update<true, EK><<<nb, bs, 0, s>>>(g, a.eos, F.Q, F.Qh, F.Qprev, F.Fx, F.Fy, F.Fz, a.clk,
+      k_update<true, EK><<<nb, bs, 0, s>>>(g, a.eos, F.Q, F.Qh, F.Qprev, F.Fx, F.Fy, F.Fz, fact, a.clk,
                                            F.err, a.viscous ? F.pBC : nullptr, nullptr);
     else
-      k_update<false, EK><<<nb, bs, 0, s>>>(g, a.eos, F.Q, F.Qh, F.Qprev, F.Fx, F.Fy, F.Fz, a.clk,
+      k_update<false, EK><<<nb, bs, 0, s>>>(g, a.eos, F.Q, F.Qh, F.Qprev, F.Fx, F.Fy, F.Fz, fact, a.clk,
                                             F.err, nullptr, a.viscous ? F.pA : nullptr);
     done(KK_UPDATE);
   }
@@ -1252,18 +1408,13 @@ static int launch_step_ek(const StepArgs& a, cudaStream_t s, LaunchMarker* mk) {
   done(KK_GHOST);
   if (a.viscous) {
     k_visc_prims<EK><<<nb, bs, 0, s>>>(g, a.eos, a.tr, F.Q, F.Qprev, F.Qh, m, F.pA, F.pD, F.pTh,
-                                   F.pBC, a.clk, F.gdst);
+                                   F.pBC, a.clk, F.gdst, F.active, F.nactive);
     done(KK_VISC_PRIMS);
     if (a.vort) {
       launches += launch_vorticity(a, s) - 1;
       done(KK_VORT);
     }
-    // the relaxation on full warps of cells with matter (the list kernel's
-    // time is counted with the relaxation's)
-    cudaMemsetAsync(F.nactive, 0, sizeof(int), s);
-    k_relax_list<<<nb128, 128, 0, s>>>(g, F.pA, F.active, F.nactive, F.pi0, F.piH0, F.Pi0,
-                                       F.PiH0, F.flux);
-    launches++;
+    // the relaxation on full warps of cells with matter
     k_is_relax<<<nb128, kRelaxBlock, kRelaxSmem, s>>>(g, a.eos, a.tr, F.Q, F.Qprev, m, F.pA, F.pD, F.pTh,
                                              F.pBC, F.pi, F.Pi, F.pi0, F.piH0, F.Pi0, F.PiH0,
                                              F.flux, a.clk, F.err, F.active, F.nactive);
@@ -1369,24 +1520,32 @@ __global__ void k_clock_op(double* clk, int op, int n) {
 
 __global__ void kb_update_m(const StepDev* __restrict__ evs, const BItem* __restrict__ items) {
   VH_ITEM
-  d_update_m(g, A.f.m, A.f.m2, A.clk, blk);
+  d_update_m(g, A.f.m, A.f.m2, A.clk, A.f.fcount, A.f.nactive, blk);
 }
 
-// the faces of a work item's kBatchBlock cells take two blocks per direction
-// (grid.y: X, Y, Z)
+__global__ void __launch_bounds__(128) kb_face_list(const StepDev* __restrict__ evs,
+                                                    const BItem* __restrict__ items,
+                                                    bool predict) {
+  VH_ITEM
+  d_face_list(g, predict ? A.f.Q : A.f.Qh, A.f.m2, A.f.fact, A.f.flist,
+              A.f.fcount + (predict ? 0 : 3), A.clk, blk);
+}
+
+// a work item of kBatchBlock cells stands for six blocks (grid.y) of its
+// event's listed faces: all there can be
 template <int EK>
 __global__ void __launch_bounds__(128, kFaceMinBlocks) kb_face(const StepDev* __restrict__ evs,
                                                                const BItem* __restrict__ items,
                                                                bool predict) {
-  const BItem it = items[blockIdx.x >> 1];
+  const BItem it = items[blockIdx.x];
   const StepDev& A = evs[it.ev];
+  const FaceBatch fb = face_batch(A.g, A.f.fcount + (predict ? 0 : 3));
+  const int b = 6 * it.blk + blockIdx.y;
+  if (b >= fb.blocks[0] + fb.blocks[1] + fb.blocks[2]) return;
   const Geo g = A.g;
-  const int dir = X_ + blockIdx.y;
-  if (dir == Z_ && g.nz == 1) return;
   const EosDev E = A.eos;
-  double* F = dir == X_ ? A.f.Fx : (dir == Y_ ? A.f.Fy : A.f.Fz);
-  d_face<EK>(g, E, predict, dir, predict ? A.f.Q : A.f.Qh, A.f.m2, F, A.clk, A.f.err,
-             2LL * it.blk + (blockIdx.x & 1));
+  d_face<EK>(g, E, predict, fb, predict ? A.f.Q : A.f.Qh, A.f.m2, A.f.Fx, A.f.Fy, A.f.Fz,
+             A.f.flist, A.clk, A.f.err, b);
 }
 
 template <bool PRED, int EK>
@@ -1396,8 +1555,8 @@ __global__ void __launch_bounds__(128, kUpdateMinBlocks) kb_update(const StepDev
   const EosDev E = A.eos;
   double* pB = PRED && A.viscous ? A.f.pBC : nullptr;
   double* pA = !PRED && A.viscous ? A.f.pA : nullptr;
-  d_update<PRED, EK>(g, E, A.f.Q, A.f.Qh, A.f.Qprev, A.f.Fx, A.f.Fy, A.f.Fz, A.clk, A.f.err, pB,
-                     pA, blk);
+  d_update<PRED, EK>(g, E, A.f.Q, A.f.Qh, A.f.Qprev, A.f.Fx, A.f.Fy, A.f.Fz, A.f.fact, A.clk,
+                     A.f.err, pB, pA, blk);
 }
 
 template <bool FULL>
@@ -1413,19 +1572,7 @@ __global__ void __launch_bounds__(128, kPrimsMinBlocks) kb_visc_prims(const Step
   const EosDev E = A.eos;
   const TrDev tr = A.tr;
   d_visc_prims<EK>(g, E, tr, A.f.Q, A.f.Qprev, A.f.Qh, A.f.m2, A.f.pA, A.f.pD, A.f.pTh,
-                   A.f.pBC, A.clk, A.f.gdst, blk);
-}
-
-__global__ void kb_nactive_zero(const StepDev* __restrict__ evs, int nev) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < nev) *evs[e].f.nactive = 0;
-}
-
-__global__ void __launch_bounds__(128) kb_relax_list(const StepDev* __restrict__ evs,
-                                                     const BItem* __restrict__ items) {
-  VH_ITEM
-  d_relax_list(g, A.f.pA, A.f.active, A.f.nactive, A.f.pi0, A.f.piH0, A.f.Pi0, A.f.PiH0,
-               A.f.flux, blk);
+                   A.f.pBC, A.clk, A.f.gdst, A.f.active, A.f.nactive, blk);
 }
 
 __global__ void __launch_bounds__(kRelaxBlock, kRelaxMinBlocks) kb_is_relax(
@@ -1470,26 +1617,25 @@ __global__ void kb_clock_op(const StepDev* __restrict__ evs, int nev, int op,
 template <int EK>
 static int launch_step_batched_ek(bool viscous, const StepDev* evs, int nev, const BItem* items,
                                   int nitems, cudaStream_t s) {
-  const unsigned nb = (unsigned)nitems, ne = nblk(nev, 128);
+  const unsigned nb = (unsigned)nitems;
   int launches = 0;
   kb_update_m<<<nb, kBatchBlock, 0, s>>>(evs, items);
   launches++;
-  // predictor and corrector; z faces of 2+1D events return at once
-  const dim3 fgrid(2 * nb, 3);
+  const dim3 fgrid(nb, 6);
+  kb_face_list<<<nb, kBatchBlock, 0, s>>>(evs, items, true);
   kb_face<EK><<<fgrid, kBatchBlock, 0, s>>>(evs, items, true);
   kb_update<true, EK><<<nb, kBatchBlock, 0, s>>>(evs, items);
+  kb_face_list<<<nb, kBatchBlock, 0, s>>>(evs, items, false);
   kb_face<EK><<<fgrid, kBatchBlock, 0, s>>>(evs, items, false);
   kb_update<false, EK><<<nb, kBatchBlock, 0, s>>>(evs, items);
   kb_ghost<false><<<nb, kBatchBlock, 0, s>>>(evs, items);
-  launches += 5;
+  launches += 7;
   if (viscous) {
     kb_visc_prims<EK><<<nb, kBatchBlock, 0, s>>>(evs, items);
-    kb_nactive_zero<<<ne, 128, 0, s>>>(evs, nev);
-    kb_relax_list<<<nb, kBatchBlock, 0, s>>>(evs, items);
     kb_is_relax<<<nb, kRelaxBlock, kRelaxSmem, s>>>(evs, items);
     kb_is_advect<<<nb, kBatchBlock, 0, s>>>(evs, items);
     kb_visc_update<<<nb, kBatchBlock, 0, s>>>(evs, items);
-    launches += 6;
+    launches += 4;
   }
   kb_ghost<true><<<nb, kBatchBlock, 0, s>>>(evs, items);
   return launches + 1;

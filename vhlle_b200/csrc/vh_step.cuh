@@ -87,7 +87,11 @@ struct Fields {
   double *pi, *piH;              // [10][N]
   double *Pi, *PiH, *vcc;        // [N]
   double *m, *m2;                // [3][N] fill fractions (double-buffered)
-  double *Fx, *Fy, *Fz;          // [7][N] face fluxes on the +dir side
+  double *Fx, *Fy, *Fz;          // [7][N] face fluxes on the +dir side, where
+                                 // fact has the direction's bit
+  unsigned char *fact;           // [N] bit d: the +d face may carry a flux
+  int *flist;                    // [3][N] the cells whose +d face may
+  int *fcount;                   // [6] their numbers: predictor, corrector
   double *flux;                  // [4][N] viscous flux accumulator
   double *pA;                    // [8][N] prims of Qh at tau_{n+1} - dt/2
   double *pD;                    // [4][N] e, v of Qh at tau_{n+1}
@@ -178,6 +182,9 @@ struct LaunchMarker {
 // there and outside any stream capture.
 cudaError_t step_kernels_setup();
 
+// Whether launch_step lists the faces that can carry a flux (two launches
+// more) on this grid, with bs threads per block.
+bool face_lists(const Geo& g, int bs);
 // Enqueues one performStep on stream s; returns the number of launches.
 // Leaves the updated fill fractions in f.m2 (the caller swaps m and m2).
 int launch_step(const StepArgs& a, cudaStream_t s, LaunchMarker* mk = nullptr);
