@@ -138,3 +138,32 @@ def test_listed_faces_equal_oracle(nx, ny, nz, nb):
         bad = compare_states(gpu_state_as_oracle(h.get_state()), o.get_state())
         assert not bad, bad
     h.close()
+
+
+@pytest.mark.parametrize("form", ["ordinary", "tiny", "mixed", "zero", "no_shear", "bump", "large_dt"])
+def test_relaxation_ranges_equal_oracle(form):
+    """Shear and bulk stresses inside and outside the ranges in which the
+    relaxation divides without tests (2^+-140), exact zeros, eta/s = 0 and a
+    zeta/s that falls off to 1e-200."""
+    s = W.glauber3d_setup(nx=17, ny=15, nz=9, xmax=7.0, etamax=4.0, b=2.0, dt=0.2 if form == "large_dt" else 0.05)
+    rng = np.random.default_rng(8)
+    N = s.grid.ncells
+    e = s.Q.reshape(7, N)[0] / s.tau0
+    mag = {"ordinary": 0., "tiny": -60., "mixed": None, "zero": 0.}.get(form, 0.)
+    ex = rng.uniform(-220., 0., (10, N)) if mag is None else np.full((10, N), mag)
+    s.pi = 0.05 * e * rng.normal(size=(10, N)) * 10. ** ex
+    s.Pi = 0.02 * e * rng.normal(size=N) * 10. ** ex[0]
+    if form == "zero":
+        s.pi[rng.random((10, N)) < 0.7] = 0.
+        s.Pi[:] = 0.
+    if form == "no_shear":
+        s.tr = dict(s.tr, etaS0=0.0, zetaS0=0.1)
+    if form == "bump":
+        s = W.with_zeta_bump(s, width_T=0.008)
+    h, o = capi.GpuHydro(s), P.OracleRun(s, crmath=form == "bump")
+    for _ in range(3):
+        h.step(1)
+        assert o.step(1) == 0
+        bad = compare_states(gpu_state_as_oracle(h.get_state()), o.get_state())
+        assert not bad, bad
+    h.close()

@@ -614,7 +614,7 @@ vh_status vh_create(const vh_grid* grid, const vh_eos* eos, const vh_trcoeff* tr
   if (c->viscous) {
     ALLOC(f.flux, 4 * N);
     ALLOC(f.pA, 8 * N);
-    ALLOC(f.pD, 4 * N);
+    ALLOC(f.pD, 5 * N);
     ALLOC(f.pTh, 9 * N);
     ALLOC(f.pBC, 9 * N);
     ALLOC(f.pi0, 10 * N);

@@ -31,7 +31,7 @@ namespace {
 
 constexpr long long kMaxCells = VH_NOALLOC_MAX_CELLS;
 constexpr int kMaxDim = VH_NOALLOC_MAX_DIM;
-constexpr long long kDoublesPerCell = 83;  // m2 3, Fx/Fy/Fz 21, flux 4, pA 8, pD 4,
+constexpr long long kDoublesPerCell = 84;  // m2 3, Fx/Fy/Fz 21, flux 4, pA 8, pD 5,
                                            // pTh 9, pBC 9, pi0/piH0 20, Pi0/PiH0 2,
                                            // the active-cell list (ints) 1, the
                                            // face lists and flags 2
@@ -224,7 +224,7 @@ extern "C" vh_status vh_step_noalloc(const vh_grid* grid, const vh_eos* eos_dev,
   f.pA = d;
   d += 8 * N;
   f.pD = d;
-  d += 4 * N;
+  d += 5 * N;
   f.pTh = d;
   d += 9 * N;
   f.pBC = d;

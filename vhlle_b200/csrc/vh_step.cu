@@ -481,7 +481,7 @@ __global__ void k_ghost(Geo g, const int* __restrict__ src, const unsigned char*
 // Per-cell inputs of the viscous stages, one thread per cell:
 //  A  = con2prim(Qh / (tau - dt/2))  (getPrimVarHCenter in ISformal, NSquant,
 //                                     visc_flux, visc_source_step),
-//  D  = con2prim(Qh / tau)           (the six NSquant neighbour velocities),
+//  D  = con2prim(Qh / tau), e and u  (the six NSquant neighbour velocities),
 //  thermodynamics at A: T, muB, p, s, eta/s, zeta/s, tau_pi, tau_Pi, 9/70/p
 //                                    (src/hdo.cpp:427-432, 727-749),
 //  B  = con2prim(Qprev / (tau - dt)), C = con2prim(Q / tau) as four-velocities
@@ -524,6 +524,7 @@ __device__ __forceinline__ void d_visc_prims(const Geo& g, const EosDev& E, cons
   const double tA = tau - dt / 2.;
   Prim a{0., 0., 0., 0., 0., 0., 0., 0.};
   int gx = 0, gy = 0, gz = 0;
+  bool vac = false;
   if (i < N) {
     coords(g, i, gx, gy, gz);
     qh[0] = Qh[i];
@@ -548,16 +549,23 @@ __device__ __forceinline__ void d_visc_prims(const Geo& g, const EosDev& E, cons
     }
   }
   {
-    // the list of cells with matter, for the relaxation and the advection:
+    // the list of cells with matter, for the relaxation and the advection
+    // (the complement of a cell next to vacuum, which NSquant leaves alone):
     // packed in warp order (one atomic per warp; the order between warps
     // varies, and every cell's result depends on that cell alone)
     const bool act = i < N && !(a.e <= 0.);
+    if (act)
+      vac = maxM_at(g, m, gx + 1, gy, gz) <= 0.9 || maxM_at(g, m, gx, gy + 1, gz) <= 0.9 ||
+            maxM_at(g, m, gx - 1, gy, gz) <= 0.9 || maxM_at(g, m, gx, gy - 1, gz) <= 0.9 ||
+            maxM_at(g, m, gx + 1, gy + 1, gz) <= 0.9 ||
+            maxM_at(g, m, gx + 1, gy - 1, gz) <= 0.9 ||
+            maxM_at(g, m, gx - 1, gy + 1, gz) <= 0.9 || maxM_at(g, m, gx - 1, gy - 1, gz) <= 0.9;
     const int lane = threadIdx.x & 31;
     const unsigned bal = __ballot_sync(0xffffffffu, act);
     int base = 0;
     if (lane == 0 && bal) base = atomicAdd(nactive, __popc(bal));
     base = __shfl_sync(0xffffffffu, base, 0);
-    if (act) active[base + __popc(bal & ((1u << lane) - 1u))] = (int)i;
+    if (act) active[base + __popc(bal & ((1u << lane) - 1u))] = vac ? ~(int)i : (int)i;
   }
   if (i >= N) return;
   if (qh[0] <= 0.) {  // vacuum: the neighbours read e first, and stop there
@@ -568,10 +576,12 @@ __device__ __forceinline__ void d_visc_prims(const Geo& g, const EosDev& E, cons
     q_over(qh, tau, q);
     Prim d;
     transform_pv<EK>(E, q, d, c2p_guess(E, i));
+    const double ut = 1.0 / sqrt(1.0 - d.vx * d.vx - d.vy * d.vy - d.vz * d.vz);
     pD[0 * N + i] = d.e;
-    pD[1 * N + i] = d.vx;
-    pD[2 * N + i] = d.vy;
-    pD[3 * N + i] = d.vz;
+    pD[1 * N + i] = ut;
+    pD[2 * N + i] = ut * d.vx;
+    pD[3 * N + i] = ut * d.vy;
+    pD[4 * N + i] = ut * d.vz;
   }
   if (a.e <= 0.) return;
   {
@@ -593,13 +603,6 @@ __device__ __forceinline__ void d_visc_prims(const Geo& g, const EosDev& E, cons
     pTh[7 * N + i] = tauPi;
     pTh[8 * N + i] = 9. / 70. / p;  // eos_p at the same point is this p
   }
-  const int ix = gx, iy = gy, iz = gz;
-  const bool vac = maxM_at(g, m, ix + 1, iy, iz) <= 0.9 || maxM_at(g, m, ix, iy + 1, iz) <= 0.9 ||
-                   maxM_at(g, m, ix - 1, iy, iz) <= 0.9 || maxM_at(g, m, ix, iy - 1, iz) <= 0.9 ||
-                   maxM_at(g, m, ix + 1, iy + 1, iz) <= 0.9 ||
-                   maxM_at(g, m, ix + 1, iy - 1, iz) <= 0.9 ||
-                   maxM_at(g, m, ix - 1, iy + 1, iz) <= 0.9 ||
-                   maxM_at(g, m, ix - 1, iy - 1, iz) <= 0.9;
   if (vac) return;
   // B is the predictor's con2prim when the divisors agree bit for bit
   // (k_update<true> stored it in pBC); otherwise computed here
@@ -668,19 +671,15 @@ constexpr int kRelaxBlock = 128;
 constexpr int kSmPI = 0, kSmSIG = 10, kSmU = 20, kSmH = 24, kSmF = 34, kSmY = 44, kSmRows = 54;
 constexpr size_t kRelaxSmem = sizeof(double) * kSmRows * kRelaxBlock;
 
-__device__ __forceinline__ void d_is_relax(
-    const Geo& g, const EosDev& E, const TrDev& tr, const double* __restrict__ Q,
-    const double* __restrict__ Qprev, const double* __restrict__ m, const double* __restrict__ pA,
-    const double* __restrict__ pD, const double* __restrict__ pTh,
-    const double* __restrict__ pBC, const double* __restrict__ pi, const double* __restrict__ Pi,
-    double* __restrict__ pi0, double* __restrict__ piH0, double* __restrict__ Pi0,
-    double* __restrict__ PiH0, double* __restrict__ flux, const double* __restrict__ clk,
-    unsigned* err, const int* __restrict__ active, const int* __restrict__ nactive,
-    long long blk) {
+// The relaxation of one cell with every division checked for its range
+// (div_batch, ddiv): the form for cells that relax_fast gives back.
+__device__ __noinline__ void relax_general(
+    const Geo& g, const double* __restrict__ pA, const double* __restrict__ pD,
+    const double* __restrict__ pTh, const double* __restrict__ pBC, const double* __restrict__ pi,
+    const double* __restrict__ Pi, double* __restrict__ pi0, double* __restrict__ piH0,
+    double* __restrict__ Pi0, double* __restrict__ PiH0, double* __restrict__ flux,
+    const double* __restrict__ clk, unsigned* err, long long i, bool vac) {
   const double dt = clk[1], tau = clk[0] + dt;  // tau_{n+1} (src/hdo.cpp:1095)
-  const int idx = (int)(blk * blockDim.x + threadIdx.x);
-  if (idx >= *nactive) return;
-  const long long i = active[idx];  // a cell with matter (k_visc_prims)
   const long long N = g.N;
   const double e = pA[i];
   int ix, iy, iz;
@@ -717,14 +716,6 @@ __device__ __forceinline__ void d_is_relax(
   // ------------------------------------------------------ NSquant
   double piNS[10], PiNS, du;
   double dmu[4][4];
-  const bool vac = maxM(m, N, cidx(g, ix + 1, iy, iz)) <= 0.9 ||
-                   maxM(m, N, cidx(g, ix, iy + 1, iz)) <= 0.9 ||
-                   maxM(m, N, cidx(g, ix - 1, iy, iz)) <= 0.9 ||
-                   maxM(m, N, cidx(g, ix, iy - 1, iz)) <= 0.9 ||
-                   maxM(m, N, cidx(g, ix + 1, iy + 1, iz)) <= 0.9 ||
-                   maxM(m, N, cidx(g, ix + 1, iy - 1, iz)) <= 0.9 ||
-                   maxM(m, N, cidx(g, ix - 1, iy + 1, iz)) <= 0.9 ||
-                   maxM(m, N, cidx(g, ix - 1, iy - 1, iz)) <= 0.9;
   if (vac) {
 #pragma unroll
     for (int a = 0; a < 4; a++)
@@ -767,16 +758,8 @@ __device__ __forceinline__ void d_is_relax(
       }
       const double ep = pD[ip], em = pD[im];
       if (ep > 0. && em > 0.) {
-        const double vx1 = pD[N + ip], vy1 = pD[2 * N + ip], vz1 = pD[3 * N + ip];
-        const double vx0 = pD[N + im], vy0 = pD[2 * N + im], vz0 = pD[3 * N + im];
-        ut0 = 1.0 / sqrt(1.0 - vx0 * vx0 - vy0 * vy0 - vz0 * vz0);
-        ux0 = ut0 * vx0;
-        uy0 = ut0 * vy0;
-        uz0 = ut0 * vz0;
-        ut1 = 1.0 / sqrt(1.0 - vx1 * vx1 - vy1 * vy1 - vz1 * vz1);
-        ux1 = ut1 * vx1;
-        uy1 = ut1 * vy1;
-        uz1 = ut1 * vz1;
+        ut0 = pD[N + im], ux0 = pD[2 * N + im], uy0 = pD[3 * N + im], uz0 = pD[4 * N + im];
+        ut1 = pD[N + ip], ux1 = pD[2 * N + ip], uy1 = pD[3 * N + ip], uz1 = pD[4 * N + ip];
         if (d < 3) {
           const double h = d == 1 ? g.dx : g.dy;
           dmu[d][0] = ddivp(ddivp(0.25 * (ut1 * ut1 - ut0 * ut0), uuu[0]), h);
@@ -1052,16 +1035,415 @@ __device__ __forceinline__ void d_is_relax(
 #undef SIG
 #undef H
 }
+
+// y / b by crm::mk_div's three operations for operands known to be in its
+// range (a zero y may lose its sign)
+__device__ __forceinline__ double mk_raw(double y, double b, double r) {
+  const double q0 = y * r;
+  return fma(fma(-q0, b, y), r, q0);
+}
+// x = +-0 or 2^-B <= |x| < 2^(B+1): integer operations on the exponent
+template <int B>
+__device__ __forceinline__ bool exp_ok(double x) {
+  const unsigned h = crm::mk_hi(x) & 0x7fffffffu;
+  return h - ((1023u - B) << 20) < ((2u * B + 1u) << 20) || (h | crm::mk_lo(x)) == 0u;
+}
+
+// The relaxation of one cell, or false (with nothing but flux written) for a
+// cell that has a nonzero quantity outside the ranges below, which
+// relax_general then takes.
+//
+// The relaxation is bound by the number of instructions it issues (57 % of
+// them were not FP64: range tests of the ~600 quotients, sign fixes,
+// shared-memory reads), so the ranges are tested once, on the quantities the
+// quotients are made of.  With pi, u, dmu, phi7, piNS, sigma and h0 zero or
+// in 2^+-140 (pi and h0 in 2^+-300 where the second-order terms are off,
+// as in the dilute cells at the edge), and eta zero or in 2^+-100, every
+// numerator below is zero or in [2^-860, 2^710]: a product of n such factors
+// is above 2^-140n, a difference of two of them is zero or a multiple of the
+// smaller one's last bit, and no numerator has more than five factors and two
+// differences.  Every quotient is then Markstein's without a test.  The same
+// ranges make these rewritings exact, value for value:
+//   x * 0.5 * dt = x * (0.5 dt), and Z * dmu * 2 = (2 Z) * dmu;
+//   NSquant's terms with Z = 0, and those of lamPipi = 8/5 (1/3 - 1/3) = 0,
+//   are +-0 and left out;
+//   the terms pi^{kl} Y^{kl} of (k, l) and (l, k) are one value, +- the sign
+//   of g_kk g_ll, divided once;
+//   |a / b| > 3 as |a| - 3 |b| > 2^-52 |b| (the difference is exact near 3).
+__device__ __forceinline__ bool relax_fast(
+    const Geo& g, const double* __restrict__ pA, const double* __restrict__ pD,
+    const double* __restrict__ pTh, const double* __restrict__ pBC, const double* __restrict__ pi,
+    const double* __restrict__ Pi, double* __restrict__ pi0, double* __restrict__ piH0,
+    double* __restrict__ Pi0, double* __restrict__ PiH0, double* __restrict__ flux,
+    const double* __restrict__ clk, long long i, bool vac) {
+  const double dt = clk[1], tau = clk[0] + dt;  // tau_{n+1} (src/hdo.cpp:1095)
+  const long long N = g.N;
+  const double e = pA[i];
+  double cpi[10];
+#pragma unroll
+  for (int k = 0; k < 10; k++) cpi[k] = pi[k * N + i];
+  const double cPi = Pi[i];
+#define PI(a, b) cpi[index44(a, b)]
+  const double vx = pA[5 * N + i], vy = pA[6 * N + i], vz = pA[7 * N + i];
+  const double gamma = 1.0 / sqrt(1.0 - vx * vx - vy * vy - vz * vz);
+  const double rg = 1.0 / gamma;
+  double u[4];
+  u[0] = gamma;
+  u[1] = u[0] * vx;
+  u[2] = u[0] * vy;
+  u[3] = u[0] * vz;
+  {
+    double f[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) f[k] = (tau - dt) * (PI(0, k) + cPi * u[0] * u[k]);
+    f[0] += -(tau - dt) * cPi;
+#pragma unroll
+    for (int k = 0; k < 4; k++) flux[k * N + i] = 0. + f[k];
+  }
+  const double s = pTh[3 * N + i];
+  const double etaS = pTh[4 * N + i];
+  const double zetaS = pTh[5 * N + i];
+  const double taupi = pTh[6 * N + i], tauPi = pTh[7 * N + i];
+  const double eta = etaS * s;
+  // (the clock and the cell sizes are the grid's: uniform)
+  bool ok = gamma <= 0x1p100 && dt >= 0x1p-60 && tau - dt >= 0x1p-60 && tau <= 0x1p60 &&
+            crm::mk_den_ok(g.dx) && crm::mk_den_ok(g.dy) && taupi >= 0. && taupi <= 0x1p60 &&
+            (eta == 0. || crm::mk_den_ok(eta)) && exp_ok<140>(etaS) &&
+            exp_ok<140>(s) && exp_ok<140>(u[1]) && exp_ok<140>(u[2]) && exp_ok<140>(u[3]) &&
+            exp_ok<140>(vz);
+  // no relaxation time (below 1 GeV/fm^3 or 100 MeV, most cells): the
+  // second-order terms are +-0, and a warp of such cells leaves them out
+  const bool still = taupi < 0.5 * dt;
+#pragma unroll
+  for (int k = 0; k < 10; k++) ok = ok && (still ? exp_ok<300>(cpi[k]) : exp_ok<140>(cpi[k]));
+
+  // ------------------------------------------------------ NSquant
+  double piNS[10], PiNS, du;
+  double dmu[4][4];
+  if (vac) {
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+      for (int b = 0; b < 4; b++) dmu[a][b] = 0.;
+#pragma unroll
+    for (int k = 0; k < 10; k++) piNS[k] = 0.;
+    PiNS = du = 0.;
+  } else {
+    const double VMIN = 1e-2;
+    // quotients by u^k are used where |u^k| >= VMIN only
+    double ud[4], ru[4];
+    bool slowu[4];
+    ud[0] = gamma;
+    ru[0] = rg;
+    slowu[0] = false;
+#pragma unroll
+    for (int k = 1; k < 4; k++) {
+      slowu[k] = fabs(u[k]) < VMIN;
+      ud[k] = slowu[k] ? 1.0 : u[k];
+      ru[k] = 1.0 / ud[k];
+    }
+    auto over3 = [](double a, double b) {  // |a / b| > UDIFF = 3
+      return fma(-3., fabs(b), fabs(a)) > 0x1p-52 * fabs(b);
+    };
+    {  // the time row: u at tau - dt (B) and at tau (C)
+      const double e0 = pBC[4 * N + i];
+      const double rdt = 1.0 / dt;
+      const bool zero = e <= 0. || e0 <= 0.;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const double u0 = pBC[k * N + i], u1 = pBC[(5 + k) * N + i];
+        const bool diff = slowu[k] || over3(0.5 * (u1 + u0), u1);
+        const double z = diff ? u1 - u0 : (u1 * u1 - u0 * u0) / 2.;
+        ok = ok && exp_ok<500>(z);
+        const double x = mk_raw(diff ? z : mk_raw(z, ud[k], ru[k]), dt, rdt);
+        dmu[0][k] = zero ? 0. : x;
+      }
+    }
+    int ix, iy, iz;
+    coords(g, i, ix, iy, iz);
+#pragma unroll
+    for (int d = 1; d <= 3; d++) {
+      long long ip, im;
+      double h;
+      if (d == 1) {
+        ip = cidx(g, ix + 1, iy, iz);
+        im = cidx(g, ix - 1, iy, iz);
+        h = g.dx;
+      } else if (d == 2) {
+        ip = cidx(g, ix, iy + 1, iz);
+        im = cidx(g, ix, iy - 1, iz);
+        h = g.dy;
+      } else {
+        ip = cidx(g, ix, iy, iz + 1);
+        im = cidx(g, ix, iy, iz - 1);
+        h = g.dz;
+      }
+      const double ep = pD[ip], em = pD[im];
+      if (ep > 0. && em > 0.) {
+        const double rh = 1.0 / h;
+        const double th = tau + 0.5 * dt, rth = d == 3 ? 1.0 / th : 0.;
+        // (an infinite dz, one cell in eta, divides the ordinary way)
+        const bool fin = d < 3 || crm::mk_den_ok(h);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const double u0 = pD[(1 + k) * N + im], u1 = pD[(1 + k) * N + ip];
+          const bool diff = slowu[k] || over3(0.5 * (u1 + u0), u[k]);
+          const double z = diff ? 0.5 * (u1 - u0) : 0.25 * (u1 * u1 - u0 * u0);
+          ok = ok && exp_ok<500>(z);
+          const double y = diff ? z : mk_raw(z, ud[k], ru[k]);
+          double x = fin ? mk_raw(y, h, rh) : y / h;
+          if (d == 3) x = mk_raw(x, th, rth);
+          dmu[d][k] = x;
+        }
+      } else {
+        dmu[d][0] = dmu[d][1] = dmu[d][2] = dmu[d][3] = 0.;
+      }
+    }
+    dmu[3][0] += ddivp(u[3], tau - 0.5 * dt);
+    dmu[3][3] += ddivp(u[0], tau - 0.5 * dt);
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+      for (int b = 0; b < 4; b++) ok = ok && exp_ok<140>(dmu[a][b]);
+    const double gdiag[4] = {1., -1., -1., -1.};
+    const double r5068 = 1.0 / 5.068, r3 = 1.0 / 3.0;
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+      for (int b = 0; b <= a; b++) {
+        const double gab = (a == b) ? gdiag[a] : 0.;
+        const double trace = 2.0 * mk_raw(gab - u[a] * u[b], 3.0, r3);
+        double acc = 0.0;
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+#pragma unroll
+          for (int l = 0; l < 4; l++) {
+            if (b != l && a != l && k != l) continue;  // Z = 0
+            double Z = 0.0;  // 2 Z
+            const double gak = (a == k) ? gdiag[a] : 0.;
+            const double gbk = (b == k) ? gdiag[b] : 0.;
+            if (b == l) Z += gak - u[a] * u[k];
+            if (a == l) Z += gbk - u[b] * u[k];
+            if (k == l) Z -= trace;
+            acc += mk_raw(Z * dmu[k][l] * etaS * s, 5.068, r5068);
+          }
+        piNS[index44(a, b)] = acc;
+      }
+    PiNS = ddivp(-zetaS * s * (dmu[0][0] + dmu[1][1] + dmu[2][2] + dmu[3][3]), 5.068);
+    du = dmu[0][0] + dmu[1][1] + dmu[2][2] + dmu[3][3];
+#pragma unroll
+    for (int k = 0; k < 10; k++) ok = ok && exp_ok<140>(piNS[k]);
+    ok = ok && exp_ok<140>(du);
+  }
+  double phi7 = pTh[8 * N + i];
+  if (isinf(phi7)) phi7 = 0.0;
+  phi7 = ddiv(phi7, taupi);
+  if (taupi < 0.5 * dt) phi7 = 0.0;
+
+  // ------------------------------------------------ ISformal loop 1 body
+  double sig[10];
+  const double reta = 1.0 / (eta == 0. ? 1.0 : eta);
+#pragma unroll
+  for (int k = 0; k < 10; k++) {
+    sig[k] = eta == 0. ? 0. : mk_raw(0.5 * piNS[k], eta, reta) * 5.068;
+    ok = ok && exp_ok<140>(sig[k]);
+  }
+  if (!ok || !exp_ok<140>(phi7)) return false;
+  const double deltapipi = still ? 0. : 4. / 3., taupipi = still ? 0. : 10. / 7.;
+  const double lambdapiPi = still ? 0. : 6. / 5.;
+  const double delPiPi = tauPi < 0.5 * dt ? 0. : 2. / 3.;
+  const double hdt = 0.5 * dt;
+  const double rtaupi = taupi > 0.5 * dt ? 1.0 / taupi : 0.;
+  double h0[10];
+#pragma unroll
+  for (int k = 0; k < 10; k++)
+    h0[k] = taupi > 0.5 * dt
+                ? cpi[k] - mk_raw(mk_raw((cpi[k] - piNS[k]) * dt / 2.0, gamma, rg), taupi, rtaupi)
+                : piNS[k];
+  double H0;
+  if (tauPi > 0.5 * dt)
+    H0 = cPi - ddivp(ddivp((cPi - PiNS) * dt / 2.0, gamma), tauPi);
+  else
+    H0 = PiNS;
+  double tau1 = tau - dt * 0.75;
+  double vt = ddivp(vz, tau1);
+  h0[index44(0, 0)] += ddivp(-2. * vz * PI(0, 3), tau1) * dt / 2.;
+  h0[index44(3, 3)] += -(2. * vt * PI(0, 3)) * dt / 2.;
+  h0[index44(3, 0)] += -(vt * PI(0, 0) + vt * PI(3, 3)) * dt / 2.;
+  h0[index44(1, 0)] += -vt * PI(1, 3) * dt / 2.;
+  h0[index44(2, 0)] += -vt * PI(2, 3) * dt / 2.;
+  h0[index44(3, 1)] += -(vt * PI(0, 1)) * dt / 2.;
+  h0[index44(3, 2)] += -(vt * PI(0, 2)) * dt / 2.;
+  // The relaxation sums over (a, b) run as a loop with (a, b) known only at
+  // run time, so that its body is fetched once per warp instead of ten times
+  // unrolled: the unrolled kernel's instruction stream outgrew the
+  // instruction caches.  Operands indexed by a or b come from shared memory
+  // ([component][thread]); the arithmetic of every term is the reference's,
+  // in its order.
+  extern __shared__ double relax_smem[];
+  double(*sm)[kRelaxBlock] = reinterpret_cast<double(*)[kRelaxBlock]>(relax_smem);
+  const int t = threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < 10; k++) {
+    sm[kSmPI + k][t] = cpi[k];
+    sm[kSmSIG + k][t] = sig[k];
+    sm[kSmH + k][t] = h0[k];
+    sm[kSmY + k][t] = phi7 * cpi[k] - taupipi * sig[k];
+  }
+#pragma unroll
+  for (int k = 0; k < 4; k++) sm[kSmU + k][t] = u[k];
+  const double htp = taupipi * 0.5;
+#pragma unroll 1
+  for (int ab = 0; ab < 10; ab++) {
+    const int a = ab >= 6 ? 3 : ab >= 3 ? 2 : ab >= 1 ? 1 : 0;
+    const int b = ab - a * (a + 1) / 2;
+    const double ua = sm[kSmU + a][t], ub = sm[kSmU + b][t];
+    double dab = -ua * ub;  // Delta[index44(a, b)]
+    if (a == b) dab += a == 0 ? 1. : -1.;
+    const double d3 = 1. / 3. * dab;
+    double w[10];  // the pi^{kl} Y^{kl} terms
+#pragma unroll
+    for (int k = 0; k < 10; k++) w[k] = 0.;
+    double acc = sm[kSmH + ab][t];
+    if (!still) {
+#pragma unroll
+      for (int k = 0; k < 10; k++)
+        w[k] = mk_raw(d3 * sm[kSmPI + k][t] * sm[kSmY + k][t], gamma, rg) * hdt;
+      acc += ddivp(-deltapipi * sm[kSmPI + ab][t] * du + lambdapiPi * cPi * sm[kSmSIG + ab][t],
+                   gamma) *
+             0.5 * dt;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const double gk = k == 0 ? 1. : -1.;
+      const double pak = sm[kSmPI + index44(a, k)][t], pbk = sm[kSmPI + index44(b, k)][t];
+      if (!still) {
+        const double sak = sm[kSmSIG + index44(a, k)][t], sbk = sm[kSmSIG + index44(b, k)][t];
+        const double n0 = phi7 * pak * pbk * gk - htp * (pak * sbk * gk + pbk * sak * gk);
+        acc += mk_raw(n0, gamma, rg) * hdt;
+      }
+      const double c = -pak * ub - pbk * ua;
+#pragma unroll
+      for (int l = 0; l < 4; l++) {
+        const double n1 = c * u[l] * dmu[l][k] * gk;
+        const double gl = l == 0 ? 1. : -1.;
+        acc += mk_raw(n1, gamma, rg) * hdt - w[index44(k, l)] * (gk * gl);
+      }
+    }
+    sm[kSmH + ab][t] = acc;
+  }
+#pragma unroll
+  for (int k = 0; k < 10; k++) {
+    h0[k] = sm[kSmH + k][t];
+    ok = ok && (still ? exp_ok<300>(h0[k]) : exp_ok<140>(h0[k]));
+  }
+  H0 += 0.;  // lamPipi = 0
+  H0 += ddivp(-delPiPi * cPi * du, gamma) * 0.5 * dt;
+  if (!ok || isinf(H0) || isnan(H0)) return false;
+#define H(a, b) h0[index44(a, b)]
+  double f0[10];
+#pragma unroll
+  for (int k = 0; k < 10; k++)
+    f0[k] = taupi > 0.5 * dt
+                ? sm[kSmPI + k][t] - mk_raw(mk_raw((h0[k] - piNS[k]) * dt, gamma, rg), taupi, rtaupi)
+                : piNS[k];
+  double F0;
+  if (tauPi > 0.5 * dt)
+    F0 = cPi - ddivp(ddivp((H0 - PiNS) * dt, gamma), tauPi);
+  else
+    F0 = PiNS;
+  tau1 = tau - dt * 0.5;
+  vt = ddivp(vz, tau1);
+  f0[index44(0, 0)] += -2. * vt * H(0, 3) * dt;
+  f0[index44(3, 3)] += -(2. * vt * H(0, 3)) * dt;
+  f0[index44(3, 0)] += -(vt * H(0, 0) + vt * H(3, 3)) * dt;
+  f0[index44(1, 0)] += -vt * H(1, 3) * dt;
+  f0[index44(2, 0)] += -vt * H(2, 3) * dt;
+  f0[index44(3, 1)] += -(vt * H(0, 1)) * dt;
+  f0[index44(3, 2)] += -(vt * H(0, 2)) * dt;
+#pragma unroll
+  for (int k = 0; k < 10; k++) {
+    sm[kSmF + k][t] = f0[k];
+    sm[kSmY + k][t] = phi7 * h0[k] - taupipi * sm[kSmSIG + k][t];
+  }
+#pragma unroll 1
+  for (int ab = 0; ab < 10; ab++) {
+    const int a = ab >= 6 ? 3 : ab >= 3 ? 2 : ab >= 1 ? 1 : 0;
+    const int b = ab - a * (a + 1) / 2;
+    const double ua = sm[kSmU + a][t], ub = sm[kSmU + b][t];
+    double dab = -ua * ub;  // Delta[index44(a, b)]
+    if (a == b) dab += a == 0 ? 1. : -1.;
+    const double d3 = 1. / 3. * dab;
+    double w[10];
+#pragma unroll
+    for (int k = 0; k < 10; k++) w[k] = 0.;
+    double acc = sm[kSmF + ab][t];
+    if (!still) {
+#pragma unroll
+      for (int k = 0; k < 10; k++) w[k] = d3 * sm[kSmH + k][t] * sm[kSmY + k][t];
+      acc += ddivp(-deltapipi * sm[kSmH + ab][t] * du + lambdapiPi * H0 * sm[kSmSIG + ab][t],
+                   gamma) *
+             dt;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const double gk = k == 0 ? 1. : -1.;
+      const double hak = sm[kSmH + index44(a, k)][t], hbk = sm[kSmH + index44(b, k)][t];
+      if (!still) {
+        const double pak = sm[kSmPI + index44(a, k)][t];
+        const double sak = sm[kSmSIG + index44(a, k)][t], sbk = sm[kSmSIG + index44(b, k)][t];
+        const double n0 = phi7 * pak * hbk * gk - htp * (hak * sbk * gk + hbk * sak * gk);
+        acc += mk_raw(n0, gamma, rg) * dt;
+      }
+      const double c = -hak * ub - hbk * ua;
+#pragma unroll
+      for (int l = 0; l < 4; l++) {
+        const double gl = l == 0 ? 1. : -1.;
+        const double n = c * u[l] * dmu[l][k] * gk - w[index44(k, l)] * (gk * gl);
+        acc += mk_raw(n, gamma, rg) * dt;
+      }
+    }
+    sm[kSmF + ab][t] = acc;
+  }
+  F0 += 0.;  // lamPipi = 0
+  F0 += ddivp(-delPiPi * H0 * du, gamma) * dt;
+#pragma unroll
+  for (int k = 0; k < 10; k++) {
+    piH0[k * N + i] = sm[kSmH + k][t];
+    pi0[k * N + i] = sm[kSmF + k][t];
+  }
+  PiH0[i] = H0;
+  Pi0[i] = F0;
+#undef PI
+#undef H
+  return true;
+}
+
+
+__device__ __forceinline__ void d_is_relax(
+    const Geo& g, const double* __restrict__ pA, const double* __restrict__ pD,
+    const double* __restrict__ pTh, const double* __restrict__ pBC, const double* __restrict__ pi,
+    const double* __restrict__ Pi, double* __restrict__ pi0, double* __restrict__ piH0,
+    double* __restrict__ Pi0, double* __restrict__ PiH0, double* __restrict__ flux,
+    const double* __restrict__ clk, unsigned* err, const int* __restrict__ active,
+    const int* __restrict__ nactive, long long blk) {
+  const int idx = (int)(blk * blockDim.x + threadIdx.x);
+  if (idx >= *nactive) return;
+  const int entry = active[idx];  // a cell with matter (k_visc_prims)
+  const bool vac = entry < 0;     // next to vacuum
+  const long long i = vac ? ~entry : entry;
+  if (!relax_fast(g, pA, pD, pTh, pBC, pi, Pi, pi0, piH0, Pi0, PiH0, flux, clk, i, vac))
+    relax_general(g, pA, pD, pTh, pBC, pi, Pi, pi0, piH0, Pi0, PiH0, flux, clk, err, i, vac);
+}
 __global__ void __launch_bounds__(kRelaxBlock, kRelaxMinBlocks) k_is_relax(
-    Geo g, EosDev E, TrDev tr, const double* __restrict__ Q, const double* __restrict__ Qprev,
-    const double* __restrict__ m, const double* __restrict__ pA, const double* __restrict__ pD,
-    const double* __restrict__ pTh, const double* __restrict__ pBC,
-    const double* __restrict__ pi, const double* __restrict__ Pi, double* __restrict__ pi0,
-    double* __restrict__ piH0, double* __restrict__ Pi0, double* __restrict__ PiH0,
-    double* __restrict__ flux, const double* __restrict__ clk, unsigned* err,
-    const int* __restrict__ active, const int* __restrict__ nactive) {
-  d_is_relax(g, E, tr, Q, Qprev, m, pA, pD, pTh, pBC, pi, Pi, pi0, piH0, Pi0, PiH0, flux, clk,
-             err, active, nactive, blockIdx.x);
+    Geo g, const double* __restrict__ pA, const double* __restrict__ pD,
+    const double* __restrict__ pTh, const double* __restrict__ pBC, const double* __restrict__ pi,
+    const double* __restrict__ Pi, double* __restrict__ pi0, double* __restrict__ piH0,
+    double* __restrict__ Pi0, double* __restrict__ PiH0, double* __restrict__ flux,
+    const double* __restrict__ clk, unsigned* err, const int* __restrict__ active,
+    const int* __restrict__ nactive) {
+  d_is_relax(g, pA, pD, pTh, pBC, pi, Pi, pi0, piH0, Pi0, PiH0, flux, clk, err, active, nactive,
+             blockIdx.x);
 }
 
 
@@ -1091,7 +1473,8 @@ __device__ __forceinline__ void d_is_advect(const Geo& g, const double* __restri
   // they are, as the reference's loop 2 leaves them (e <= 0)
   const int idx = (int)(blk * blockDim.x + threadIdx.x);
   if (idx >= *nactive) return;
-  const long long i = active[idx];
+  const int entry = active[idx];
+  const long long i = entry < 0 ? ~entry : entry;
   int ix, iy, iz;
   coords(g, i, ix, iy, iz);
   const long long N = g.N;
@@ -1415,9 +1798,9 @@ static int launch_step_ek(const StepArgs& a, cudaStream_t s, LaunchMarker* mk) {
       done(KK_VORT);
     }
     // the relaxation on full warps of cells with matter
-    k_is_relax<<<nb128, kRelaxBlock, kRelaxSmem, s>>>(g, a.eos, a.tr, F.Q, F.Qprev, m, F.pA, F.pD, F.pTh,
-                                             F.pBC, F.pi, F.Pi, F.pi0, F.piH0, F.Pi0, F.PiH0,
-                                             F.flux, a.clk, F.err, F.active, F.nactive);
+    k_is_relax<<<nb128, kRelaxBlock, kRelaxSmem, s>>>(g, F.pA, F.pD, F.pTh, F.pBC, F.pi, F.Pi,
+                                                      F.pi0, F.piH0, F.Pi0, F.PiH0, F.flux, a.clk,
+                                                      F.err, F.active, F.nactive);
     done(KK_IS_RELAX);
     k_is_advect<<<nb, bs, 0, s>>>(g, F.pA, F.pi0, F.piH0, F.Pi0, F.PiH0, F.pi, F.piH, F.Pi, F.PiH,
                                   F.vcc, F.flux, a.clk, F.active, F.nactive);
@@ -1578,11 +1961,8 @@ __global__ void __launch_bounds__(128, kPrimsMinBlocks) kb_visc_prims(const Step
 __global__ void __launch_bounds__(kRelaxBlock, kRelaxMinBlocks) kb_is_relax(
     const StepDev* __restrict__ evs, const BItem* __restrict__ items) {
   VH_ITEM
-  const EosDev E = A.eos;
-  const TrDev tr = A.tr;
-  d_is_relax(g, E, tr, A.f.Q, A.f.Qprev, A.f.m2, A.f.pA, A.f.pD, A.f.pTh, A.f.pBC, A.f.pi,
-             A.f.Pi, A.f.pi0, A.f.piH0, A.f.Pi0, A.f.PiH0, A.f.flux, A.clk, A.f.err, A.f.active,
-             A.f.nactive, blk);
+  d_is_relax(g, A.f.pA, A.f.pD, A.f.pTh, A.f.pBC, A.f.pi, A.f.Pi, A.f.pi0, A.f.piH0, A.f.Pi0,
+             A.f.PiH0, A.f.flux, A.clk, A.f.err, A.f.active, A.f.nactive, blk);
 }
 
 __global__ void __launch_bounds__(128) kb_is_advect(const StepDev* __restrict__ evs,

@@ -94,13 +94,14 @@ struct Fields {
   int *fcount;                   // [6] their numbers: predictor, corrector
   double *flux;                  // [4][N] viscous flux accumulator
   double *pA;                    // [8][N] prims of Qh at tau_{n+1} - dt/2
-  double *pD;                    // [4][N] e, v of Qh at tau_{n+1}
+  double *pD;                    // [5][N] e, u^mu of Qh at tau_{n+1}
   double *pTh;                   // [9][N] thermodynamics and transport at pA
   double *pBC;                   // [9][N] four-velocities for NSquant's d/dtau
   double *pi0, *piH0;            // [10][N] IS relaxation results
   double *Pi0, *PiH0;            // [N]
   int *active, *nactive;         // [N] cells with matter (e > 0) for the
-                                 // relaxation, and their count ([1])
+                                 // relaxation, those next to vacuum
+                                 // complemented, and their count ([1])
   int *gsrc;                     // [nx+ny+nz] ghost-cell source map
   unsigned char *gdst;           // [nx+ny+nz] ghost-cell destination flags
   unsigned *err;                 // device error word

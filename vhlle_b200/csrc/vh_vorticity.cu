@@ -172,8 +172,11 @@ __global__ void __launch_bounds__(kVortBlock) k_vort_ops(
     if (e1 > 0. && e0 > 0.) {
       f |= VF_SET1 << (d - 1);
       double u0[4], u1[4];
-      four_velocity(pD[N + im], pD[2 * N + im], pD[3 * N + im], u0);
-      four_velocity(pD[N + ip], pD[2 * N + ip], pD[3 * N + ip], u1);
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        u0[k] = pD[(1 + k) * N + im];
+        u1[k] = pD[(1 + k) * N + ip];
+      }
       const double T1 = v.TD[ip], T0 = v.TD[im];
       const double h = d == 1 ? g.dx : d == 2 ? g.dy : g.dz * (tau + 0.5 * dt);
       const bool zero = e1 <= 0. || e0 <= 0. || T1 <= 0. || T0 <= 0.;
