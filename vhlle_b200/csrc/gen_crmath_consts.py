@@ -5,9 +5,14 @@ Exact rational arithmetic (fractions) and a 60-digit decimal ln 2
 (decimal.Decimal.ln); run it to check the literals in the header:
 
     python vhlle_b200/csrc/gen_crmath_consts.py
+
+It also writes vh_crmath_tab.cuh: for exp's and log's short forms ln 2 and
+ln 2 / 64 in two doubles, 2^(j/64) and, per 1/128 of [1, 2), the reciprocal
+of the middle and minus its logarithm as double-double pairs.
 """
 import decimal
 import math
+import os
 from fractions import Fraction
 
 decimal.getcontext().prec = 80
@@ -44,5 +49,33 @@ def main():
         print("INV_FACT[%d] = {%s, %s}" % (n, hi.hex(), lo.hex()))
 
 
+def pair(q: Fraction):
+    hi = rn(q)
+    return hi, rn(q - Fraction(hi))
+
+
+def tables():
+    dec = lambda q: decimal.Decimal(q.numerator) / decimal.Decimal(q.denominator)  # noqa: E731
+    out = ["// Written by gen_crmath_consts.py: the tables of vh_crmath.cuh's short forms.",
+           "#pragma once", ""]
+    for name, q, bits in (("LN2", LN2, 42), ("LN2_64", LN2 / 64, 36)):
+        h = trunc_bits(q, bits)
+        out.append("#define VH_CRM_%sH %s" % (name, h.hex()))
+        out.append("#define VH_CRM_%sL %s" % (name, rn(q - Fraction(h)).hex()))
+    out.append("#define VH_CRM_64_LN2 %s" % rn(64 / LN2).hex())
+    exp2 = [pair(Fraction((decimal.Decimal(j) / 64 * decimal.Decimal(2).ln()).exp())) for j in range(64)]
+    logs = []
+    for i in range(128):
+        c = rn(1 / (1 + Fraction(2 * i + 1, 256)))
+        logs.append((c,) + pair(-Fraction(dec(Fraction(c)).ln())))
+    for name, rows in (("EXP_TAB", exp2), ("LOG_TAB", logs)):
+        out.append("#define VH_CRM_%s \\" % name)
+        out += ["  " + ", ".join(float(v).hex() for v in r) + (", \\" if r is not rows[-1] else "") for r in rows]
+    path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "vh_crmath_tab.cuh")
+    with open(path, "w") as f:
+        f.write("\n".join(out) + "\n")
+
+
 if __name__ == "__main__":
     main()
+    tables()

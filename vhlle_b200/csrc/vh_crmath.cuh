@@ -22,6 +22,12 @@
 //        double-double.  Relative error before the final rounding < 2^-98.
 //   log: a Newton step on the exp above from a faithful seed (log_cr).
 //   x^y: exp of y log(x), both in double-double (pow_cr).
+//   exp and x^y first take a short form (exp_try, log_short; Ziv's strategy,
+//        ACM TOMS 17 (1991)): tables of 2^(j/64) and of log at 1/128 steps
+//        (Tang's table method, ACM TOMS 15 (1989) and 16 (1990), the first
+//        two orders of each series in double-double), whose result is taken
+//        when its error bound cannot move the rounding; the forms above
+//        decide the rest, about one argument in eight thousand.
 //   x^(1/4): sqrt(x) as a double-double (the correctly rounded square root
 //        and its exact residual by fma), its square root the same way, and
 //        one rounding of the sum.
@@ -32,10 +38,15 @@
 
 #include <math.h>
 
+#include "vh_crmath_tab.cuh"
+
 #ifdef __CUDACC__
 #define VH_CRM __host__ __device__ __forceinline__
+// the long forms stay out of line: they run for one argument in thousands
+#define VH_CRM_COLD static __host__ __device__ __noinline__
 #else
 #define VH_CRM static inline
+#define VH_CRM_COLD static inline
 #endif
 
 namespace vh {
@@ -44,6 +55,27 @@ namespace crm {
 struct dd {
   double hi, lo;
 };
+
+#ifdef __CUDACC__
+static __device__ const double kExpTabDev[128] = {VH_CRM_EXP_TAB};
+static __device__ const double kLogTabDev[384] = {VH_CRM_LOG_TAB};
+#endif
+static const double kExpTabHost[128] = {VH_CRM_EXP_TAB};
+static const double kLogTabHost[384] = {VH_CRM_LOG_TAB};
+VH_CRM double exp_tab(int k) {
+#ifdef __CUDA_ARCH__
+  return __ldg(kExpTabDev + k);
+#else
+  return kExpTabHost[k];
+#endif
+}
+VH_CRM double log_tab(int k) {
+#ifdef __CUDA_ARCH__
+  return __ldg(kLogTabDev + k);
+#else
+  return kLogTabHost[k];
+#endif
+}
 
 VH_CRM dd two_sum(double a, double b) {
   const double s = a + b;
@@ -146,7 +178,7 @@ VH_CRM dd expm1_dd(dd r) {
   return e;
 }
 
-VH_CRM double exp_cr(double x) {
+VH_CRM_COLD double exp_long(double x) {
   if (!(x == x)) return x;  // NaN
   if (x > 709.8) return (double)INFINITY;
   if (x < -746.0) return 0.0;
@@ -245,7 +277,7 @@ VH_CRM double exp_dd_cr(dd t) {
 // special values: x^0 = 1 and 1^y = 1 (NaN included), NaN otherwise
 // propagates; 0^y = +0 (y > 0) or +inf (y < 0), with -0 kept for odd
 // integers y; inf^y = inf or 0; negative x for integer y only (NaN else).
-VH_CRM double pow_cr(double x, double y) {
+VH_CRM_COLD double pow_long(double x, double y) {
   if (y == 0. || x == 1.) return 1.;
   if (!(x == x) || !(y == y)) return x + y;
   if (y == 2.) return x * x;
@@ -267,6 +299,81 @@ VH_CRM double pow_cr(double x, double y) {
   if (t.hi > 709.8) return sgn * (double)INFINITY;
   if (t.hi < -746.0) return sgn * 0.;
   return sgn * exp_dd_cr(t);
+}
+
+// exp(t.hi + t.lo) for |t.hi| <= 700, |t.lo| <= 2^-30, in the short form:
+// t = k ln2/64 + r, |r| < 2^-7.5, 2^(j/64) (1 + r + r^2/2 + r^3 P(r)); true
+// and the result in *out if the result's relative error, below 2^-72 plus
+// t's own absolute error (at most 2^-70), leaves one double to round to.
+VH_CRM bool exp_try(dd t, double* out) {
+  const double k = rint(t.hi * VH_CRM_64_LN2);
+  const double rh = fma(-k, VH_CRM_LN2_64H, t.hi);  // exact: k H has 53 bits
+  const dd r = fast_two_sum(rh, fma(-k, VH_CRM_LN2_64L, t.lo));
+  const dd r2 = two_prod(r.hi, r.hi);
+  double P = 0x1.a01a01a01a01ap-16;  // 1/8!
+  P = fma(P, r.hi, 0x1.a01a01a01a01ap-13);
+  P = fma(P, r.hi, 0x1.6c16c16c16c17p-10);
+  P = fma(P, r.hi, 0x1.1111111111111p-7);
+  P = fma(P, r.hi, 0x1.5555555555555p-5);
+  P = fma(P, r.hi, 0x1.5555555555555p-3);
+  // q = exp(r) - 1
+  const dd s = fast_two_sum(r.hi, 0.5 * r2.hi);
+  const double ql = (r.hi * r2.hi) * P + (s.lo + (r.lo + (0.5 * r2.lo + r.hi * r.lo)));
+  const dd q = fast_two_sum(s.hi, ql);
+  const int n = (int)k, j = n & 63;
+  const double th = exp_tab(2 * j), tl = exp_tab(2 * j + 1);
+  const dd p = two_prod(th, q.hi);
+  const dd a = fast_two_sum(th, p.hi);
+  const dd y = fast_two_sum(a.hi, a.lo + (p.lo + (tl + (th * q.lo + tl * q.hi))));
+  const double err = 0x1p-67 * y.hi;
+  const double up = y.hi + (y.lo + err), down = y.hi + (y.lo - err);
+  *out = up * pow2i((n - j) >> 6);  // exact: |t.hi| <= 700
+  return up == down;
+}
+
+// log(x) for a normal x > 0 as a double-double, absolute error below 2^-73:
+// x = 2^k m, m c = 1 + r with c the table's reciprocal near 1/m, |r| < 2^-7.9,
+// k ln2 - log c + r - r^2/2 + r^3 P(r)
+VH_CRM dd log_short(double x) {
+  const unsigned long long u = to_bits(x);
+  const double k = (double)((int)(u >> 52) - 1023);
+  const double m = from_bits((u & 0x000fffffffffffffull) | 0x3ff0000000000000ull);
+  const int i = 3 * (int)((u >> 45) & 127);
+  const double c = log_tab(i);
+  const dd mc = two_prod(m, c);
+  const dd r = fast_two_sum(mc.hi - 1., mc.lo);
+  const dd r2 = two_prod(r.hi, r.hi);
+  double P = 0x1.c71c71c71c71cp-4;  // 1/9
+  P = fma(P, r.hi, -0x1p-3);
+  P = fma(P, r.hi, 0x1.2492492492492p-3);
+  P = fma(P, r.hi, -0x1.5555555555555p-3);
+  P = fma(P, r.hi, 0x1.999999999999ap-3);
+  P = fma(P, r.hi, -0x1p-2);
+  P = fma(P, r.hi, 0x1.5555555555555p-2);
+  const dd s1 = two_sum(k * VH_CRM_LN2H, log_tab(i + 1));  // k H exact
+  const dd s2 = two_sum(s1.hi, r.hi);
+  const dd s3 = two_sum(s2.hi, -0.5 * r2.hi);
+  const double lo = (r.hi * r2.hi) * P + (s3.lo + (s2.lo + (s1.lo + (r.lo - (0.5 * r2.lo + r.hi * r.lo) +
+                    fma(k, VH_CRM_LN2L, log_tab(i + 2))))));
+  return two_sum(s3.hi, lo);
+}
+
+VH_CRM double exp_cr(double x) {
+  double r;
+  if (fabs(x) <= 700. && exp_try({x, 0.}, &r)) return r;
+  return exp_long(x);
+}
+
+VH_CRM double pow_cr(double x, double y) {
+  if (x >= 0x1p-1022 && x <= 0x1.fffffffffffffp1023 && x != 1. && fabs(y) <= 8. && y != 2. &&
+      y != 0.) {
+    const dd L = log_short(x);
+    const dd p = two_prod(y, L.hi);
+    const dd t = fast_two_sum(p.hi, fma(y, L.lo, p.lo));
+    double r;
+    if (fabs(t.hi) <= 700. && exp_try(t, &r)) return r;
+  }
+  return pow_long(x, y);
 }
 
 // x^(1/4) for x >= 0 (x = +0 gives +0, x = inf gives inf)
@@ -329,6 +436,7 @@ VH_CRM double mk_div(double y, double b, double r) {
 }  // namespace vh
 
 #undef VH_CRM
+#undef VH_CRM_COLD
 #undef VH_CRM_LN2_1
 #undef VH_CRM_LN2_2
 #undef VH_CRM_LN2_3

@@ -20,9 +20,8 @@
 //   k_ic_terms    a normalisation pass's per-cell terms (s95p_e and the
 //                 cell's energy, or its baryon number), written in the
 //                 reference's loop order (ix, iy, iz)
-//   k_seq_sum     their sum in that order, one thread adding tiles that
-//                 the block's other warps stage in shared memory: the same
-//                 rounded sum as the host loop
+//   k_seq_sum     their sum in that order, rounded after every addition as
+//                 the host loop, by whole-number sums within a binade
 //   k_ic_set      e = s95p_e(..), nb, setPrimVar, setAllM for every cell
 //   k_ic_gubser, k_table_prep, k_ic_table   the other two modules
 //
@@ -59,8 +58,8 @@ constexpr int kS95pMaxIt = 200;    // the reference iterates without a bound
 constexpr int kNormMaxIt = 10000;  // likewise its normalisation loops
 
 // x^y and e^x kept out of line: s95p_s holds up to six powers and two
-// exponentials, each ~800 FP64 operations inlined, and the Newton loop
-// around it would otherwise be tens of KB of straight-line code per kernel
+// exponentials, and the Newton loop around it would otherwise be tens of KB
+// of straight-line code per kernel
 __device__ __noinline__ double pw(double x, double y) { return crm::pow_cr(x, y); }
 __device__ __noinline__ double ex(double x) { return crm::exp_cr(x); }
 
@@ -334,56 +333,101 @@ __global__ void __launch_bounds__(kTpb) k_ic_terms(TermArgs a) {
 }
 
 // sum of t[0..n) from 0.0 in index order, rounded after every addition as
-// the host loop: thread 0 adds a tile of terms from shared memory while the
-// block's loader warps stage the next tile, so the running sum waits only on
-// its own additions.  Each loader warp keeps its 256 terms of the tile with
-// the zeros squeezed out, in order (ballot and prefix count), and thread 0
-// adds the warps' runs in warp order: the same sequence of non-zero
-// additions as the host loop, whose zero terms change nothing (the running
-// sum starts at +0 and is never -0, and s + (+-0) = s for every other s; the
-// vacuum cells' terms are exactly zero).
-constexpr int kSumLoaders = 8;                     // loader warps
-constexpr int kSumThreads = 32 * (1 + kSumLoaders);
-constexpr int kSumRun = 256;                       // terms per loader warp and tile
-constexpr int kSumTile = kSumLoaders * kSumRun;    // 2 x 16 KB of shared memory
+// the host loop, without its chain of additions.
+//
+// While the running sum s stays in one binade [2^k, 2^(k+1)) it is a whole
+// number of u = 2^(k-52), and RN(s + t) = s + RN_u(t), t rounded to a
+// multiple of u: the same for every s there, unless t lies halfway between
+// two multiples (the tie goes by the last bit of s).  So the additions of a
+// run of non-negative terms without ties, as long as their sum stays below
+// 2^(k+1), are a sum of whole numbers below 2^53, in any order.  A sub-tile
+// (the 256 terms of a warp) with a tie, a negative or non-finite term, or
+// the step into the next binade is added term by term; over n terms of one
+// size that happens about ln n times for ties and log2 n times for binades.
+// One block, since each tile needs the sum before it; 520,251 terms took
+// 977 us as a chain of additions.
+constexpr int kSumThreads = 1024;
+constexpr int kSumPer = 8;                       // terms per thread and tile
+constexpr int kSumRun = 32 * kSumPer;            // a sub-tile
+constexpr int kSumTile = kSumThreads * kSumPer;  // 32 sub-tiles
 
 __global__ void __launch_bounds__(kSumThreads) k_seq_sum(const double* __restrict__ t, long long n,
                                                          double* __restrict__ out) {
-  __shared__ double buf[2][kSumTile];
-  __shared__ int cnt[2][kSumLoaders];
-  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const long long ntile = (n + kSumTile - 1) / kSumTile;
-  // loader warp w stages terms [w * kSumRun, (w + 1) * kSumRun) of a tile
-  auto stage = [&](long long tile, int b) {
-    const int w = warp - 1;
-    const long long base = tile * kSumTile + (long long)w * kSumRun;
-    double* dst = buf[b] + w * kSumRun;
-    int c = 0;
-    for (int r = 0; r < kSumRun; r += 32) {
-      const long long k = base + r + lane;
-      const double v = k < n ? t[k] : 0.0;
-      const unsigned live = __ballot_sync(0xffffffffu, v != 0.0);  // NaN counts
-      if (v != 0.0) dst[c + __popc(live & ((1u << lane) - 1u))] = v;
-      c += __popc(live);
+  __shared__ double wsum[32];
+  __shared__ int wbad[32];
+  __shared__ double s_sh;
+  __shared__ int pos_sh;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double s = 0.0, v[kSumPer];
+  auto load = [&](long long tile, double* x) {
+    const long long base = tile * kSumTile + warp * kSumRun + lane;
+#pragma unroll
+    for (int r = 0; r < kSumPer; r++) {
+      const long long k = base + 32 * r;
+      x[r] = k < n ? t[k] : 0.0;
     }
-    if (lane == 0) cnt[b][w] = c;
   };
-  if (warp > 0 && ntile > 0) stage(0, 0);
-  __syncthreads();
-  double s = 0.0;
+  const long long ntile = (n + kSumTile - 1) / kSumTile;
+  load(0, v);
   for (long long tile = 0; tile < ntile; tile++) {
-    const int b = (int)(tile & 1);
-    if (warp > 0 && tile + 1 < ntile) stage(tile + 1, b ^ 1);
-    if (tid == 0)
-      for (int w = 0; w < kSumLoaders; w++) {
-        const double* p = buf[b] + w * kSumRun;
-        const int m = cnt[b][w];
-#pragma unroll 4
-        for (int j = 0; j < m; j++) s += p[j];
+    double next[kSumPer];
+    load(tile + 1, next);  // (zeros past the end)
+    int pos = 0;           // the first sub-tile not added yet
+    while (pos < 32) {
+      // s in whole numbers of its last bit; s = 0 takes zero terms only
+      const int ex = (int)((unsigned long long)__double_as_longlong(s) >> 52);  // sign included
+      const bool fit = ex >= 60 && ex <= 1980;
+      const double scale = fit ? crm::pow2i(52 + 1023 - ex) : 0.0;
+      const double u = fit ? crm::pow2i(ex - 1023 - 52) : 0.0;
+      double sum = 0.0;
+      bool bad = !fit && s != 0.0;
+#pragma unroll
+      for (int r = 0; r < kSumPer; r++) {
+        const double x = v[r] * scale, w = rint(x);
+        sum += w;
+        bad |= fit ? !(v[r] >= 0.0 && x < 0x1p51) || fabs(x - w) == 0.5 : v[r] != 0.0;
       }
-    __syncthreads();
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      const unsigned any = __ballot_sync(0xffffffffu, bad);
+      if (lane == 0) {
+        wsum[warp] = sum;
+        wbad[warp] = any != 0;
+      }
+      __syncthreads();
+      if (warp == 0) {
+        double run = lane >= pos ? wsum[lane] : 0.0;  // inclusive prefix sums
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const double x = __shfl_up_sync(0xffffffffu, run, o);
+          if (lane >= o) run += x;
+        }
+        const double S = s * scale;
+        const bool stop = lane >= pos && (wbad[lane] || !(S + run < 0x1p53));
+        const unsigned st = __ballot_sync(0xffffffffu, stop);
+        const int f = st ? __ffs((int)st) - 1 : 32;  // the first sub-tile to add term by term
+        const double before = __shfl_sync(0xffffffffu, run, f > 0 ? f - 1 : 0);
+        if (f > pos) s = fit ? (S + before) * u : s;
+        if (lane == 0) {
+          if (f < 32) {
+            const long long b = tile * kSumTile + (long long)f * kSumRun;
+            const int m = (int)(n - b < kSumRun ? (n - b > 0 ? n - b : 0) : kSumRun);
+#pragma unroll 8
+            for (int j = 0; j < m; j++) s += t[b + j];
+          }
+          s_sh = s;
+          pos_sh = f < 32 ? f + 1 : 32;
+        }
+      }
+      __syncthreads();
+      s = s_sh;
+      pos = pos_sh;
+      __syncthreads();
+    }
+#pragma unroll
+    for (int r = 0; r < kSumPer; r++) v[r] = next[r];
   }
-  if (tid == 0) out[0] = s;
+  if (threadIdx.x == 0) out[0] = s;
 }
 
 struct SetArgs {
