@@ -1320,10 +1320,10 @@ vh_status vh_sync(vh_ctx* ctx) {
 vh_status vh_launches_per_step(vh_ctx* ctx, int* n) {
   if (!ctx || !n) return VH_ERR_ARG;
   // update_m, 2 x (face list, faces, update), 2 ghost, the viscous four
-  // (prims, relaxation, advection, update) and the six of the
+  // (prims, relaxation, advection, update) and the five of the
   // vorticity, the MLP guess, the clock
   int k = 1 + 2 * (vh::face_lists(ctx->g, 128) ? 3 : 2) + 1 + (ctx->viscous ? 4 : 0) + 1 +
-          (ctx->viscous && ctx->vort_on ? 6 : 0) + (ctx->mlp ? 1 : 0) + 1;
+          (ctx->viscous && ctx->vort_on ? 5 : 0) + (ctx->mlp ? 1 : 0) + 1;
   *n = k;
   return VH_OK;
 }
@@ -1734,6 +1734,7 @@ vh_status vh_enable_vorticity(vh_ctx* ctx, int on) {
   if (on && !v.dbeta) {
     vh_status st;
     if ((st = dalloc(ctx, &v.dbeta, (size_t)16 * N)) || (st = dalloc(ctx, &v.TD, (size_t)N)) ||
+        (st = dalloc(ctx, &v.TB, (size_t)N)) || (st = dalloc(ctx, &v.TC, (size_t)N)) ||
         (st = dalloc(ctx, &v.val, (size_t)18 * N)) || (st = dalloc(ctx, &v.R, (size_t)2 * N)) ||
         (st = dalloc(ctx, &v.flag, (size_t)N)) || (st = dalloc(ctx, &v.last, (size_t)5 * N)) ||
         (st = dalloc(ctx, &v.agg, (size_t)5 * vh::vort_scan_blocks(N))))

@@ -286,7 +286,7 @@ __device__ __forceinline__ void d_update(const Geo& g, const EosDev& E, double* 
                                          const unsigned char* __restrict__ fact,
                                          const double* __restrict__ clk, unsigned* err,
                                          double* __restrict__ pB, double* __restrict__ pA,
-                                         long long blk) {
+                                         double* __restrict__ nbB, long long blk) {
   const double tau = clk[0], dt = clk[1];  // the step's clock (device)
   const long long i = blk * blockDim.x + threadIdx.x;
   if (i >= g.N) return;
@@ -338,6 +338,7 @@ __device__ __forceinline__ void d_update(const Geo& g, const EosDev& E, double* 
       pB[i] = 1.;
 #pragma unroll
       for (int k = 1; k < 5; k++) pB[k * N + i] = 0.;
+      if (nbB) nbB[i] = 0.;
     }
     return;
   }
@@ -379,6 +380,7 @@ __device__ __forceinline__ void d_update(const Geo& g, const EosDev& E, double* 
     pB[2 * N + i] = ut * pp.vy;
     pB[3 * N + i] = ut * pp.vz;
     pB[4 * N + i] = pp.e;
+    if (nbB) nbB[i] = pp.nb;  // with the vorticity on: B's T needs it
   }
   double kk[7];
   kk[T_] = -q[T_] * pp.vz * pp.vz - pp.p * (1. + pp.vz * pp.vz);
@@ -418,8 +420,9 @@ __global__ void __launch_bounds__(128, kUpdateMinBlocks) k_update(Geo g, EosDev 
                                                 const double* __restrict__ Fz,
                                                 const unsigned char* __restrict__ fact,
                                                 const double* __restrict__ clk, unsigned* err,
-                                                double* __restrict__ pB, double* __restrict__ pA) {
-  d_update<PRED, EK>(g, E, Q, Qh, Qprev, Fx, Fy, Fz, fact, clk, err, pB, pA, blockIdx.x);
+                                                double* __restrict__ pB, double* __restrict__ pA,
+                                                double* __restrict__ nbB) {
+  d_update<PRED, EK>(g, E, Q, Qh, Qprev, Fx, Fy, Fz, fact, clk, err, pB, pA, nbB, blockIdx.x);
 }
 
 
@@ -505,7 +508,9 @@ __device__ __forceinline__ Prim loadA(const double* __restrict__ pA, long long N
   return a;
 }
 
-template <int EK>
+// VORT: also T of the states that the vorticity's rows divide by (TD at D,
+// TB at B, TC at C), so that it solves nothing again.
+template <int EK, bool VORT>
 __device__ __forceinline__ void d_visc_prims(const Geo& g, const EosDev& E, const TrDev& tr,
                                              const double* __restrict__ Q,
                                              const double* __restrict__ Qprev,
@@ -516,7 +521,9 @@ __device__ __forceinline__ void d_visc_prims(const Geo& g, const EosDev& E, cons
                                              const double* __restrict__ clk,
                                              const unsigned char* __restrict__ isdst,
                                              int* __restrict__ active,
-                                             int* __restrict__ nactive, long long blk) {
+                                             int* __restrict__ nactive, double* __restrict__ TD,
+                                             double* __restrict__ TB, double* __restrict__ TC,
+                                             long long blk) {
   const double dt = clk[1], tau = clk[0] + dt;  // tau_{n+1} (src/hdo.cpp:1095)
   const long long i = blk * blockDim.x + threadIdx.x;
   const long long N = g.N;
@@ -582,6 +589,11 @@ __device__ __forceinline__ void d_visc_prims(const Geo& g, const EosDev& E, cons
     pD[2 * N + i] = ut * d.vx;
     pD[3 * N + i] = ut * d.vy;
     pD[4 * N + i] = ut * d.vz;
+    if (VORT) {
+      double T, mub, p;
+      eos_eval<EK>(E, d.e, d.nb, T, mub, p);
+      TD[i] = T;
+    }
   }
   if (a.e <= 0.) return;
   {
@@ -607,6 +619,11 @@ __device__ __forceinline__ void d_visc_prims(const Geo& g, const EosDev& E, cons
   // B is the predictor's con2prim when the divisors agree bit for bit
   // (k_update<true> stored it in pBC); otherwise computed here
   const bool haveB = (clk[0] + dt) - dt == clk[0];
+  if (VORT && haveB) {
+    double T, mub, p;
+    eos_eval<EK>(E, pBC[4 * N + i], TB[i], T, mub, p);
+    TB[i] = T;  // (held B's nb until here)
+  }
 #pragma unroll 1
   for (int w = haveB ? 1 : 0; w < 2; w++) {
     const double* src = w == 0 ? Qprev : Q;
@@ -624,9 +641,14 @@ __device__ __forceinline__ void d_visc_prims(const Geo& g, const EosDev& E, cons
     pBC[(o + 2) * N + i] = ut * P.vy;
     pBC[(o + 3) * N + i] = ut * P.vz;
     if (w == 0) pBC[4 * N + i] = P.e;
+    if (VORT) {
+      double T, mub, p;
+      eos_eval<EK>(E, P.e, P.nb, T, mub, p);
+      (w == 0 ? TB : TC)[i] = T;
+    }
   }
 }
-template <int EK>
+template <int EK, bool VORT>
 __global__ void __launch_bounds__(128, kPrimsMinBlocks) k_visc_prims(Geo g, EosDev E, TrDev tr,
                                                     const double* __restrict__ Q,
                                                     const double* __restrict__ Qprev,
@@ -638,9 +660,12 @@ __global__ void __launch_bounds__(128, kPrimsMinBlocks) k_visc_prims(Geo g, EosD
                                                     double* __restrict__ pBC, const double* __restrict__ clk,
                                                     const unsigned char* __restrict__ isdst,
                                                     int* __restrict__ active,
-                                                    int* __restrict__ nactive) {
-  d_visc_prims<EK>(g, E, tr, Q, Qprev, Qh, m, pA, pD, pTh, pBC, clk, isdst, active, nactive,
-                   blockIdx.x);
+                                                    int* __restrict__ nactive,
+                                                    double* __restrict__ TD,
+                                                    double* __restrict__ TB,
+                                                    double* __restrict__ TC) {
+  d_visc_prims<EK, VORT>(g, E, tr, Q, Qprev, Qh, m, pA, pD, pTh, pBC, clk, isdst, active, nactive,
+                         TD, TB, TC, blockIdx.x);
 }
 
 
@@ -1744,7 +1769,7 @@ bool face_lists(const Geo& g, int bs) { return face_blocks(g, bs) > face_residen
 const char* const kKernelNames[KK_COUNT] = {
     "k_update_m", "k_face", "k_update", "k_ghost",
     "k_visc_prims", "k_is_relax", "k_is_advect", "k_visc_update",
-    "vorticity (k_vort_*, 6 kernels)"};
+    "vorticity (k_vort_*, 5 kernels)"};
 
 
 template <int EK>
@@ -1758,6 +1783,7 @@ static int launch_step_ek(const StepArgs& a, cudaStream_t s, LaunchMarker* mk) {
   const bool lists = face_lists(g, bs);
   const unsigned nface = (unsigned)std::min(fblocks, resident);
   const unsigned char* fact = lists ? a.f.fact : nullptr;
+  const bool vort = a.vort && a.viscous;
   int launches = 0;
   const Fields& F = a.f;
   auto done = [&](int kind) {
@@ -1781,19 +1807,26 @@ static int launch_step_ek(const StepArgs& a, cudaStream_t s, LaunchMarker* mk) {
     done(KK_FACE);
     if (pred)
       k_update<true, EK><<<nb, bs, 0, s>>>(g, a.eos, F.Q, F.Qh, F.Qprev, F.Fx, F.Fy, F.Fz, fact, a.clk,
-                                           F.err, a.viscous ? F.pBC : nullptr, nullptr);
+                                           F.err, a.viscous ? F.pBC : nullptr, nullptr,
+                                           vort ? a.vort->TB : nullptr);
     else
       k_update<false, EK><<<nb, bs, 0, s>>>(g, a.eos, F.Q, F.Qh, F.Qprev, F.Fx, F.Fy, F.Fz, fact, a.clk,
-                                            F.err, nullptr, a.viscous ? F.pA : nullptr);
+                                            F.err, nullptr, a.viscous ? F.pA : nullptr, nullptr);
     done(KK_UPDATE);
   }
   k_ghost<false><<<nb, bs, 0, s>>>(g, F.gsrc, F.gdst, F.Q, F.Qh, F.pi, F.Pi);
   done(KK_GHOST);
   if (a.viscous) {
-    k_visc_prims<EK><<<nb, bs, 0, s>>>(g, a.eos, a.tr, F.Q, F.Qprev, F.Qh, m, F.pA, F.pD, F.pTh,
-                                   F.pBC, a.clk, F.gdst, F.active, F.nactive);
+    if (vort)
+      k_visc_prims<EK, true><<<nb, bs, 0, s>>>(g, a.eos, a.tr, F.Q, F.Qprev, F.Qh, m, F.pA, F.pD,
+                                               F.pTh, F.pBC, a.clk, F.gdst, F.active, F.nactive,
+                                               a.vort->TD, a.vort->TB, a.vort->TC);
+    else
+      k_visc_prims<EK, false><<<nb, bs, 0, s>>>(g, a.eos, a.tr, F.Q, F.Qprev, F.Qh, m, F.pA, F.pD,
+                                                F.pTh, F.pBC, a.clk, F.gdst, F.active, F.nactive,
+                                                nullptr, nullptr, nullptr);
     done(KK_VISC_PRIMS);
-    if (a.vort) {
+    if (vort) {
       launches += launch_vorticity(a, s) - 1;
       done(KK_VORT);
     }
@@ -1939,7 +1972,7 @@ __global__ void __launch_bounds__(128, kUpdateMinBlocks) kb_update(const StepDev
   double* pB = PRED && A.viscous ? A.f.pBC : nullptr;
   double* pA = !PRED && A.viscous ? A.f.pA : nullptr;
   d_update<PRED, EK>(g, E, A.f.Q, A.f.Qh, A.f.Qprev, A.f.Fx, A.f.Fy, A.f.Fz, A.f.fact, A.clk,
-                     A.f.err, pB, pA, blk);
+                     A.f.err, pB, pA, nullptr, blk);
 }
 
 template <bool FULL>
@@ -1954,8 +1987,9 @@ __global__ void __launch_bounds__(128, kPrimsMinBlocks) kb_visc_prims(const Step
   VH_ITEM
   const EosDev E = A.eos;
   const TrDev tr = A.tr;
-  d_visc_prims<EK>(g, E, tr, A.f.Q, A.f.Qprev, A.f.Qh, A.f.m2, A.f.pA, A.f.pD, A.f.pTh,
-                   A.f.pBC, A.clk, A.f.gdst, A.f.active, A.f.nactive, blk);
+  d_visc_prims<EK, false>(g, E, tr, A.f.Q, A.f.Qprev, A.f.Qh, A.f.m2, A.f.pA, A.f.pD, A.f.pTh,
+                   A.f.pBC, A.clk, A.f.gdst, A.f.active, A.f.nactive, nullptr,
+                   nullptr, nullptr, blk);
 }
 
 __global__ void __launch_bounds__(kRelaxBlock, kRelaxMinBlocks) kb_is_relax(

@@ -110,7 +110,7 @@ struct Fields {
 // Device buffers of the vorticity output (Hydro::enableVorticity).
 struct VortDev {
   double* dbeta;        // [16][N] d_mu beta_nu per cell (4 mu + nu), clamped
-  double* TD;           // [N] T at the prims of Qh at tau_{n+1}
+  double *TD, *TB, *TC; // [N] T at k_visc_prims' D, B and C
   double* val;          // [18][N] the 16 values NSquant writes, the 2 increments
   double* R;            // [2][N] running M[3][0], M[3][3] at lone increments
   unsigned char* flag;  // [N] VF_* bits

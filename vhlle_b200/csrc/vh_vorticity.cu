@@ -17,9 +17,11 @@
 // and M[3][0], M[3][3] add, in loop order, the increments of the
 // participating cells after that writer.
 //
-// Device form, per step (six launches, off the hot step unless enabled):
-//   k_vort_T            T of every cell's Qh state at tau_{n+1} (what the
-//                       neighbour rows read)
+// Device form, per step (five launches, off the hot step unless enabled),
+// from the states k_visc_prims has solved (four-velocities, and T with the
+// vorticity on; solving the three states again and looking up their T took
+// 137 of the vorticity's 174 us a step at 101x101x51, keeping T takes 15 and
+// the whole 110):
 //   k_vort_ops          per cell: the values NSquant writes, which rows, the
 //                       two increments
 //   k_vort_scan_blocks  inclusive max-scans over loop positions of the last
@@ -82,35 +84,12 @@ __device__ __forceinline__ void four_velocity(double vx, double vy, double vz, d
   u[3] = u[0] * vz;
 }
 
-// T at the prims of Qh at tau_{n+1} (Cell::getPrimVarHCenter(tau) then
-// EoS::eos, src/hdo.cpp:471-480): the same con2prim as k_visc_prims' pD
-template <int EK>
-__global__ void __launch_bounds__(kVortBlock) k_vort_T(Geo g, EosDev E,
-                                                       const double* __restrict__ Qh,
-                                                       const double* __restrict__ clk,
-                                                       double* __restrict__ TD) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= g.N) return;
-  const long long N = g.N;
-  const double tau = clk[0] + clk[1];
-  double qs[7], q[7];
-#pragma unroll
-  for (int k = 0; k < 7; k++) qs[k] = Qh[k * N + i];
-  q_over(qs, tau, q);
-  Prim d;
-  transform_pv<EK>(E, q, d, c2p_guess(E, i));
-  double T, mub, p;
-  eos_eval<EK>(E, d.e, d.nb, T, mub, p);
-  TD[i] = T;
-}
-
 // What NSquant does to M at cell i (src/hdo.cpp:397-414, 418-459, 466-500,
 // 512-546, 558-592, 606-611)
-template <int EK>
 __global__ void __launch_bounds__(kVortBlock) k_vort_ops(
-    Geo g, EosDev E, const double* __restrict__ Q, const double* __restrict__ Qprev,
-    const double* __restrict__ m, const double* __restrict__ pA, const double* __restrict__ pD,
-    const double* __restrict__ pTh, const double* __restrict__ clk, VortDev v) {
+    Geo g, const double* __restrict__ m, const double* __restrict__ pA,
+    const double* __restrict__ pD, const double* __restrict__ pTh, const double* __restrict__ pBC,
+    const double* __restrict__ clk, VortDev v) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= g.N) return;
   const long long N = g.N;
@@ -134,24 +113,16 @@ __global__ void __launch_bounds__(kVortBlock) k_vort_ops(
   unsigned f = VF_NONEMPTY | VF_PART;
   double out[18];
   {
-    // row 0: Qprev at tau - dt and Q at tau (getPrimVarPrev, getPrimVar)
-    double qs[7], q[7];
-    Prim P0, P1;
-#pragma unroll
-    for (int k = 0; k < 7; k++) qs[k] = Qprev[k * N + i];
-    q_over(qs, tau - dt, q);
-    transform_pv<EK>(E, q, P0, c2p_guess(E, i));
-#pragma unroll
-    for (int k = 0; k < 7; k++) qs[k] = Q[k * N + i];
-    q_over(qs, tau, q);
-    transform_pv<EK>(E, q, P1, c2p_guess(E, i));
-    double T0, T1, mub, p;
-    eos_eval<EK>(E, P0.e, P0.nb, T0, mub, p);
-    eos_eval<EK>(E, P1.e, P1.nb, T1, mub, p);
+    // row 0: Qprev at tau - dt and Q at tau (getPrimVarPrev, getPrimVar),
+    // k_visc_prims' B and C
     double u0[4], u1[4];
-    four_velocity(P0.vx, P0.vy, P0.vz, u0);
-    four_velocity(P1.vx, P1.vy, P1.vz, u1);
-    const bool zero = eH <= 0. || P0.e <= 0. || T1 <= 0. || T0 <= 0.;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      u0[k] = pBC[k * N + i];
+      u1[k] = pBC[(5 + k) * N + i];
+    }
+    const double e0 = pBC[4 * N + i], T0 = v.TB[i], T1 = v.TC[i];
+    const bool zero = eH <= 0. || e0 <= 0. || T1 <= 0. || T0 <= 0.;
 #pragma unroll
     for (int k = 0; k < 4; k++) out[k] = zero ? 0. : (u1[k] / T1 - u0[k] / T0) / dt;
   }
@@ -379,32 +350,12 @@ int launch_vorticity(const StepArgs& a, cudaStream_t s) {
   const VortDev& v = *a.vort;
   const unsigned nb = vblk(g.N, kVortBlock);
   const int nsb = vort_scan_blocks(g.N);
-  if (a.eos.kind == 3) {  // per EoS class, as the step's con2prim kernels
-    k_vort_T<EK_TABLE3><<<nb, kVortBlock, 0, s>>>(g, a.eos, F.Qh, a.clk, v.TD);
-    k_vort_ops<EK_TABLE3><<<nb, kVortBlock, 0, s>>>(g, a.eos, F.Q, F.Qprev, F.m2, F.pA, F.pD,
-                                                    F.pTh, a.clk, v);
-  } else if (a.eos.kind == 7) {
-    k_vort_T<EK_CMFE><<<nb, kVortBlock, 0, s>>>(g, a.eos, F.Qh, a.clk, v.TD);
-    k_vort_ops<EK_CMFE><<<nb, kVortBlock, 0, s>>>(g, a.eos, F.Q, F.Qprev, F.m2, F.pA, F.pD,
-                                                  F.pTh, a.clk, v);
-  } else if (a.eos.kind == 6) {
-    k_vort_T<EK_AZH><<<nb, kVortBlock, 0, s>>>(g, a.eos, F.Qh, a.clk, v.TD);
-    k_vort_ops<EK_AZH><<<nb, kVortBlock, 0, s>>>(g, a.eos, F.Q, F.Qprev, F.m2, F.pA, F.pD,
-                                                 F.pTh, a.clk, v);
-  } else if (a.eos.kind == 2) {
-    k_vort_T<EK_CHIRAL><<<nb, kVortBlock, 0, s>>>(g, a.eos, F.Qh, a.clk, v.TD);
-    k_vort_ops<EK_CHIRAL><<<nb, kVortBlock, 0, s>>>(g, a.eos, F.Q, F.Qprev, F.m2, F.pA, F.pD,
-                                                    F.pTh, a.clk, v);
-  } else {
-    k_vort_T<EK_TABLE><<<nb, kVortBlock, 0, s>>>(g, a.eos, F.Qh, a.clk, v.TD);
-    k_vort_ops<EK_TABLE><<<nb, kVortBlock, 0, s>>>(g, a.eos, F.Q, F.Qprev, F.m2, F.pA, F.pD,
-                                                   F.pTh, a.clk, v);
-  }
+  k_vort_ops<<<nb, kVortBlock, 0, s>>>(g, F.m2, F.pA, F.pD, F.pTh, F.pBC, a.clk, v);
   k_vort_scan_blocks<<<nsb, kVortScan, 0, s>>>(g, v, nsb);
   k_vort_scan_aggs<<<1, 1024, 0, s>>>(v.agg, nsb);
   k_vort_orphan<<<nb, kVortBlock, 0, s>>>(g, v, nsb);
   k_vort_store<<<nb, kVortBlock, 0, s>>>(g, v, nsb);
-  return 6;
+  return 5;
 }
 
 // ------------------------------------------------------------ beta.dat
