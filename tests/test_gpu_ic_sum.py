@@ -14,7 +14,7 @@ from vhlle_b200 import workloads as W
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nx,ny,nz,xmax", [(9, 9, 3, 8.), (15, 17, 2, 8.), (32, 32, 8, 9.), (33, 31, 9, 9.),
+@pytest.mark.parametrize("nx,ny,nz,xmax", [(9, 9, 3, 8.), (15, 17, 4, 8.), (32, 32, 8, 9.), (33, 31, 9, 9.),
                                            (41, 40, 16, 24.)])
 @pytest.mark.parametrize("name", ["RHIC62", "LHC276"])
 def test_norms_equal_the_sequential_sums(nx, ny, nz, xmax, name, tmp_path):

@@ -159,8 +159,8 @@ vh_status capture(vh_batch* b, const std::vector<int>& nsub, const Config& cfg,
     if (n > 1) vh::launch_clock_op(c->clk, 1, n, s);  // dt / n
     for (int j = 0; j < n; j++) {
       if (c->mlp) vh::launch_mlp_guess(c->mlp->packed, a.f.Q, c->g.N, c->clk, c->vguess, s);
+      a.tick = c->clk;  // tau += dt
       vh::launch_step(a, s);
-      vh::launch_clock_op(c->clk, 0, 0, s);  // tau += dt
       std::swap(a.f.m, a.f.m2);
     }
     if (n > 1) vh::launch_clock_op(c->clk, 2, n, s);  // dt * n
@@ -258,7 +258,6 @@ vh_status capture_stages(vh_batch* b, const std::vector<int>& nsub, cudaGraphExe
     }
     vh::launch_step_batched(b->stage_ek, b->stage_viscous, ddev + pt.dev0, pt.nev,
                             idev + pt.item0, pt.nitems, b->origin);
-    vh::launch_clock_op_batched(ddev + pt.dev0, pt.nev, 0, nullptr, b->origin);  // tau += dt
   }
   vh::launch_clock_op_batched(ddev, parts[0].nev, 2, ndev, b->origin);  // dt * n
   cudaGraph_t graph = nullptr;

@@ -610,7 +610,7 @@ vh_status vh_create(const vh_grid* grid, const vh_eos* eos, const vh_trcoeff* tr
   ALLOC(f.Fz, 7 * N);
   ALLOC(f.fact, N);
   ALLOC(f.flist, 3 * N);
-  ALLOC(f.fcount, 6);
+  ALLOC(f.fcount, 7);
   if (c->viscous) {
     ALLOC(f.flux, 4 * N);
     ALLOC(f.pA, 8 * N);
@@ -622,6 +622,7 @@ vh_status vh_create(const vh_grid* grid, const vh_eos* eos, const vh_trcoeff* tr
     ALLOC(f.Pi0, N);
     ALLOC(f.PiH0, N);
     ALLOC(f.active, N);
+    ALLOC(f.wet, N);
     ALLOC(f.nactive, 1);
   }
   ALLOC(c->clk, 2);
@@ -795,6 +796,7 @@ static vh::StepArgs step_args(vh_ctx* ctx) {
   a.eos.vguess = ctx->mlp ? ctx->vguess : nullptr;
   a.tr = ctx->tr;
   a.f = ctx->f;
+  a.tick = ctx->clk;
   a.clk = ctx->clk;  // holds (tau, dt): set when the host changes them, advanced per step
   a.viscous = ctx->viscous;
   a.vort = ctx->vort_on && ctx->viscous ? &ctx->vort : nullptr;
@@ -841,8 +843,7 @@ static bool capture_step(vh_ctx* ctx, int par) {
     return false;
   }
   if (ctx->mlp) vh::launch_mlp_guess(ctx->mlp->packed, ctx->f.Q, ctx->g.N, ctx->clk, ctx->vguess, s);
-  const int n = vh::launch_step(a, s);
-  vh::launch_clock_op(ctx->clk, 0, 0, s);
+  const int n = vh::launch_step(a, s);  // and tau += dt on the device
   cudaGraph_t graph = nullptr;
   cudaError_t e = cudaStreamEndCapture(s, &graph);
   unsigned long long flags = cudaGraphInstantiateFlagUseNodePriority;
@@ -891,7 +892,6 @@ vh_status vh_step(vh_ctx* ctx) {
   } else {
     ctx->launches = vh::launch_step(a, ctx->stream);
   }
-  vh::launch_clock_op(ctx->clk, 0, 0, ctx->stream);  // tau += dt on the device
   VH_CUDA(ctx, cudaGetLastError());
   std::swap(ctx->f.m, ctx->f.m2);
   ctx->tau += ctx->dt;  // src/hdo.cpp:1095
@@ -1001,7 +1001,6 @@ static bool capture_host_step(vh_ctx* ctx, int par, const vh_state_view* in,
   if (e == cudaSuccess) {
     if (ctx->mlp) vh::launch_mlp_guess(ctx->mlp->packed, F.Q, N, ctx->clk, ctx->vguess, s);
     n = vh::launch_step(a, s, &mk);
-    vh::launch_clock_op(ctx->clk, 0, 0, s);
     e = mk.err;
   }
   // the rest comes back at the end

@@ -31,10 +31,10 @@ namespace {
 
 constexpr long long kMaxCells = VH_NOALLOC_MAX_CELLS;
 constexpr int kMaxDim = VH_NOALLOC_MAX_DIM;
-constexpr long long kDoublesPerCell = 84;  // m2 3, Fx/Fy/Fz 21, flux 4, pA 8, pD 5,
+constexpr long long kDoublesPerCell = 85;  // m2 3, Fx/Fy/Fz 21, flux 4, pA 8, pD 5,
                                            // pTh 9, pBC 9, pi0/piH0 20, Pi0/PiH0 2,
-                                           // the active-cell list (ints) 1, the
-                                           // face lists and flags 2
+                                           // the cell lists (ints) 2, the face
+                                           // lists and flags 2
 constexpr size_t kHeaderBytes = 256 + 3 * kMaxDim * sizeof(int) + 3 * kMaxDim;  // err, maps
 constexpr size_t kHeaderAligned = (kHeaderBytes + 255) / 256 * 256;
 constexpr size_t kScratchBytes = kHeaderAligned + (size_t)kDoublesPerCell * kMaxCells * sizeof(double);
@@ -242,6 +242,7 @@ extern "C" vh_status vh_step_noalloc(const vh_grid* grid, const vh_eos* eos_dev,
   f.flist = reinterpret_cast<int*>(d);
   f.fact = reinterpret_cast<unsigned char*>(f.flist + 3 * N);
   f.fcount = reinterpret_cast<int*>(base + 64);
+  f.wet = reinterpret_cast<int*>(d + 2 * N);
   f.Q = s->Q;
   f.Qh = s->Qh;
   f.Qprev = s->Qprev;

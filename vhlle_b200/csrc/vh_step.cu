@@ -22,10 +22,11 @@
 namespace vh {
 
 // resident blocks of 128 threads per SM, from sweeps on the 101x101x51 event
-// (us per step at the stated counts): the face kernel 6 / 7 / 8 / 10 blocks
-// 369 / 341 / 330 / 364; the update 6 / 8 / 10 / 12: 112 / 113 / 124 / 129;
-// the viscous primitives 6 / 7 / 8 / 10: 57.3 / 55.5 / 57.3 / 60.9
-constexpr int kFaceMinBlocks = 8, kUpdateMinBlocks = 6, kPrimsMinBlocks = 7;
+// (us per step at the stated counts): the face kernel 5 / 6 / 8 blocks 161 /
+// 160 / 153; the update 4 / 5 / 6 / 8: 100 / 94 / 97 / 93, where the 2+1D
+// grid of 101x101 takes 36 / 37 / 39 / 40 us a step and 201x201x101 462 / 401 /
+// 391 / 363; the viscous primitives 6 / 7 / 8: 30.8 / 31.5 / 33.1
+constexpr int kFaceMinBlocks = 8, kUpdateMinBlocks = 5, kPrimsMinBlocks = 6;
 
 // -------------------------------------------------------------- updateM
 // Fluid::updateM, src/fld.cpp:384-423 (both passes; out of place).
@@ -36,7 +37,7 @@ __device__ __forceinline__ void d_update_m(const Geo& g, const double* __restric
   const double tau = clk[0], dt = clk[1];  // the step's clock (device)
   const long long i = blk * blockDim.x + threadIdx.x;
   // the step's list counters, filled by later kernels
-  if (i < 6) fcount[i] = 0;
+  if (i < 7) fcount[i] = 0;
   if (i == 0 && nactive) *nactive = 0;
   if (i >= g.N) return;
   int ix, iy, iz;
@@ -108,11 +109,15 @@ __device__ __forceinline__ void d_face_list(const Geo& g, const double* __restri
     const int cc[3] = {ix, iy, iz}, nn[3] = {g.nx, g.ny, g.nz};
     const long long ss[3] = {1, g.nx, (long long)g.nx * g.ny};
     const double x1 = QT[i], huge = 0.9e10 * clk[0];
+    double up[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) up[d] = cc[d] < nn[d] - 1 ? QT[i + ss[d]] : 0.;
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-      if (cc[d] >= nn[d] - 1) continue;
+      const double x2 = up[d];
+      // two empty cells have two empty edges (a slope takes the smaller side)
+      if (cc[d] >= nn[d] - 1 || (x1 == 0. && x2 == 0.)) continue;
       const long long st = ss[d];
-      const double x2 = QT[i + st];
       const double x0 = cc[d] > 0 ? QT[i - st] : x1, x3 = cc[d] < nn[d] - 2 ? QT[i + 2 * st] : x2;
       const double el = x1 + minmod((x2 - x1) / 2., (x1 - x0) / 2.);
       const double er = x2 - minmod((x3 - x2) / 2., (x2 - x1) / 2.);
@@ -273,6 +278,54 @@ __global__ void __launch_bounds__(128, kFaceMinBlocks) k_face(
 }
 
 
+// ------------------------------------------------------- cells with matter
+// i joins the list: one atomic for the lanes that arrive together
+__device__ __forceinline__ void append(int* __restrict__ list, int* __restrict__ n, int i) {
+  const unsigned with = __activemask();
+  const int lane = threadIdx.x & 31, first = __ffs((int)with) - 1;
+  int base = 0;
+  if (lane == first) base = atomicAdd(n, __popc(with));
+  base = __shfl_sync(with, base, first);
+  list[base + __popc(with & ((1u << lane) - 1u))] = i;
+}
+// The same for the whole block (every thread calls it): one atomic, and the
+// block's entries in thread order, so that a list keeps the grid's runs (with
+// one atomic per warp the relaxation over the list took 112 instead of 101 us
+// at 101x101x51).
+__device__ __forceinline__ void append_block(int* __restrict__ list, int* __restrict__ n, int i,
+                                             bool with) {
+  __shared__ int cnt[4], first;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const unsigned bal = __ballot_sync(0xffffffffu, with);
+  __syncthreads();  // an earlier call's reads
+  if (lane == 0) cnt[warp] = __popc(bal);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int c = 0;
+    for (int w = 0; w < nw; w++) c += cnt[w];
+    first = c ? atomicAdd(n, c) : 0;
+  }
+  __syncthreads();
+  if (!with) return;
+  int at = first + __popc(bal & ((1u << lane) - 1u));
+  for (int w = 0; w < warp; w++) at += cnt[w];
+  list[at] = i;
+}
+// the cells the ghost copy writes (Fluid::correctImagCells: the two outermost
+// of every side)
+__device__ __forceinline__ bool is_ghost(const Geo& g, int ix, int iy, int iz) {
+  return ix < 2 || ix >= g.nx - 2 || iy < 2 || iy >= g.ny - 2 || iz < 2 || iz >= g.nz - 2;
+}
+// what the viscous stages read of an empty cell: e and v at the half step, e
+// at the full one
+__device__ __forceinline__ void empty_prims(double* __restrict__ pA, double* __restrict__ pD,
+                                            long long N, long long i) {
+  pA[i] = 0.;
+#pragma unroll
+  for (int k = 5; k < 8; k++) pA[k * N + i] = 0.;
+  pD[i] = 0.;
+}
+
 // --------------------------------------------------- ideal cell update
 // Gathers the six face fluxes and the Milne source (Hydro::source_step,
 // src/hdo.cpp:307-353), then Cell::updateQtoQhByFlux (predictor) or
@@ -286,13 +339,20 @@ __device__ __forceinline__ void d_update(const Geo& g, const EosDev& E, double* 
                                          const unsigned char* __restrict__ fact,
                                          const double* __restrict__ clk, unsigned* err,
                                          double* __restrict__ pB, double* __restrict__ pA,
-                                         double* __restrict__ nbB, long long blk) {
+                                         double* __restrict__ nbB, double* __restrict__ pD,
+                                         int* __restrict__ wet, int* __restrict__ nwet,
+                                         long long blk) {
   const double tau = clk[0], dt = clk[1];  // the step's clock (device)
   const long long i = blk * blockDim.x + threadIdx.x;
-  if (i >= g.N) return;
-  int ix, iy, iz;
-  coords(g, i, ix, iy, iz);
   const long long N = g.N;
+  const bool in = i < N;
+  int ix = 0, iy = 0, iz = 0;
+  if (in) coords(g, i, ix, iy, iz);
+  const bool ghost = is_ghost(g, ix, iy, iz);
+  // the viscous stages' cells; the ghost copy settles its own
+  const bool prims = !PRED && pA && in && !ghost;
+  if (!PRED && pA) append_block(wet, nwet, (int)i, prims && !(Qh[i] <= 0.));
+  if (!in) return;
   const long long sy = g.nx, sz = (long long)g.nx * g.ny;
   const double* field = PRED ? Q : Qh;
   const double tau1 = PRED ? tau : tau + 0.5 * dt;
@@ -316,11 +376,7 @@ __device__ __forceinline__ void d_update(const Geo& g, const EosDev& E, double* 
   // vacuum that nothing flows into: no flux, no source, the row stays
   const bool still = !faces && qin[T_] <= 0. && qin[Z_] == 0.;
   if (!PRED && still) {
-    if (pA) {
-      pA[i] = 0.;  // e and v are read of empty cells too, the rest of none
-#pragma unroll
-      for (int k = 5; k < 8; k++) pA[k * N + i] = 0.;
-    }
+    if (prims) empty_prims(pA, pD, N, i);
     return;
   }
 #pragma unroll
@@ -334,7 +390,7 @@ __device__ __forceinline__ void d_update(const Geo& g, const EosDev& E, double* 
     }
     // pB is read of cells with matter at the half step: not of this one,
     // unless the ghost copy puts matter there
-    if (pB && (ix < 2 || ix >= g.nx - 2 || iy < 2 || iy >= g.ny - 2 || iz < 2 || iz >= g.nz - 2)) {
+    if (pB && ghost) {
       pB[i] = 1.;
 #pragma unroll
       for (int k = 1; k < 5; k++) pB[k * N + i] = 0.;
@@ -357,7 +413,8 @@ __device__ __forceinline__ void d_update(const Geo& g, const EosDev& E, double* 
   q_over(qin, tau1, q);
   Prim pp;
   transform_pv<EK>(E, q, pp, c2p_guess(E, i));
-  if (!PRED && pA) {
+  if (prims && qin[T_] <= 0.) empty_prims(pA, pD, N, i);
+  if (prims && !(qin[T_] <= 0.)) {
     // con2prim(Qh / (tau_n + dt/2)) is the viscous stage's A =
     // con2prim(Qh / (tau_{n+1} - dt/2)) for every cell that the ghost copy
     // does not overwrite, whenever the divisors agree bit for bit
@@ -421,67 +478,115 @@ __global__ void __launch_bounds__(128, kUpdateMinBlocks) k_update(Geo g, EosDev 
                                                 const unsigned char* __restrict__ fact,
                                                 const double* __restrict__ clk, unsigned* err,
                                                 double* __restrict__ pB, double* __restrict__ pA,
-                                                double* __restrict__ nbB) {
-  d_update<PRED, EK>(g, E, Q, Qh, Qprev, Fx, Fy, Fz, fact, clk, err, pB, pA, nbB, blockIdx.x);
+                                                double* __restrict__ nbB, double* __restrict__ pD,
+                                                int* __restrict__ wet, int* __restrict__ nwet) {
+  d_update<PRED, EK>(g, E, Q, Qh, Qprev, Fx, Fy, Fz, fact, clk, err, pB, pA, nbB, pD, wet, nwet,
+                     blockIdx.x);
 }
 
 
 // ------------------------------------------------------------- ghosts
-// Fluid::correctImagCells (FULL = false: Q and Qh) and correctImagCellsFull
-// (FULL = true: Q, pi, Pi), src/fld.cpp:211-382, as a gather from the
-// per-dimension source maps; copies into a ghost zero the row when Q_t < 0
-// (Cell::setQ / setQh).
-template <bool FULL>
+// Fluid::correctImagCells (HALF: Q and Qh) and correctImagCellsFull (FULL:
+// Q, pi, Pi), src/fld.cpp:211-382, as a gather from the per-dimension source
+// maps, over the cells that are copied into only (78 of 520 thousand at
+// 101x101x51); copies into a ghost zero the row when Q_t < 0 (Cell::setQ /
+// setQh).  An ideal step, where nothing lies between the two, does both at
+// once.  HALF in a viscous step (wet not null) also settles the copied
+// cells for the viscous stages; FULL, the step's last kernel, advances the
+// clock (which it does not read).
+struct Shell {  // the copied-into cells: the z planes, then rows, then ends
+  int gx, gy, gz, iy, iz;
+  long long a, b, n;
+};
+__host__ __device__ inline Shell ghost_shell(const Geo& g) {
+  Shell s;
+  s.gx = g.nx < 4 ? g.nx : 4;
+  s.gy = g.ny < 4 ? g.ny : 4;
+  s.gz = g.nz < 4 ? g.nz : 4;
+  s.iy = g.ny - s.gy;
+  s.iz = g.nz - s.gz;
+  s.a = (long long)s.gz * g.nx * g.ny;
+  s.b = s.a + (long long)s.iz * s.gy * g.nx;
+  s.n = s.b + (long long)s.iz * s.iy * s.gx;
+  return s;
+}
+__device__ __forceinline__ int ghost_index(int k, int n) { return k < 2 || n <= 4 ? k : n - 4 + k; }
+
+template <bool HALF, bool FULL>
 __device__ __forceinline__ void d_ghost(const Geo& g, const int* __restrict__ src,
-                                        const unsigned char* __restrict__ isdst,
-                                        double* __restrict__ Q, double* __restrict__ Qh,
-                                        double* __restrict__ pi, double* __restrict__ Pi,
-                                        long long blk) {
-  const long long i = blk * blockDim.x + threadIdx.x;
-  if (i >= g.N) return;
+                                        const Fields& f, int* wet, double* tick, long long blk) {
+  const long long t = blk * blockDim.x + threadIdx.x;
+  if (FULL && tick && t == 0) tick[0] += tick[1];  // tau += dt (src/hdo.cpp:1095)
+  const Shell sh = ghost_shell(g);
+  if (t >= sh.n) return;
   int ix, iy, iz;
-  coords(g, i, ix, iy, iz);
+  if (t < sh.a) {
+    const unsigned r = (unsigned)t, p = (unsigned)(g.nx * g.ny), k = r / p, q = r - k * p;
+    iy = (int)(q / (unsigned)g.nx);
+    ix = (int)(q - iy * (unsigned)g.nx);
+    iz = ghost_index((int)k, g.nz);
+  } else if (t < sh.b) {
+    const unsigned r = (unsigned)(t - sh.a), p = (unsigned)(sh.gy * g.nx), k = r / p, q = r - k * p;
+    const unsigned w = q / (unsigned)g.nx;
+    ix = (int)(q - w * (unsigned)g.nx);
+    iy = ghost_index((int)w, g.ny);
+    iz = 2 + (int)k;
+  } else {
+    const unsigned r = (unsigned)(t - sh.b), p = (unsigned)(sh.iy * sh.gx), k = r / p, q = r - k * p;
+    const unsigned w = q / (unsigned)sh.gx;
+    ix = ghost_index((int)(q - w * (unsigned)sh.gx), g.nx);
+    iy = 2 + (int)w;
+    iz = 2 + (int)k;
+  }
   const int* sx = src;
   const int* sy = src + g.nx;
   const int* sz = src + g.nx + g.ny;
-  if (!(isdst[ix] | isdst[g.nx + iy] | isdst[g.nx + g.ny + iz])) return;
   const long long N = g.N;
+  const long long i = (long long)ix + (long long)g.nx * (iy + (long long)g.ny * iz);
   const long long s = (long long)sx[ix] + (long long)g.nx * (sy[iy] + (long long)g.ny * sz[iz]);
   {
     double q[7];
 #pragma unroll
-    for (int k = 0; k < 7; k++) q[k] = Q[k * N + s];
+    for (int k = 0; k < 7; k++) q[k] = f.Q[k * N + s];
     const bool neg = q[0] < 0.;
 #pragma unroll
-    for (int k = 0; k < 7; k++) Q[k * N + i] = neg ? 0. : q[k];
+    for (int k = 0; k < 7; k++) f.Q[k * N + i] = neg ? 0. : q[k];
   }
-  if (!FULL) {
+  if (HALF) {
     double q[7];
 #pragma unroll
-    for (int k = 0; k < 7; k++) q[k] = Qh[k * N + s];
+    for (int k = 0; k < 7; k++) q[k] = f.Qh[k * N + s];
     const bool neg = q[0] < 0.;
 #pragma unroll
-    for (int k = 0; k < 7; k++) Qh[k * N + i] = neg ? 0. : q[k];
-  } else {
+    for (int k = 0; k < 7; k++) f.Qh[k * N + i] = neg ? 0. : q[k];
+    if (wet) {
+      if (!(q[0] <= 0.))
+        append(wet, f.fcount + 6, (int)i);
+      else
+        empty_prims(f.pA, f.pD, N, i);
+    }
+  }
+  if (FULL) {
     double p[10];
 #pragma unroll
-    for (int k = 0; k < 10; k++) p[k] = pi[k * N + s];
-    const double P = Pi[s];
+    for (int k = 0; k < 10; k++) p[k] = f.pi[k * N + s];
+    const double P = f.Pi[s];
 #pragma unroll
-    for (int k = 0; k < 10; k++) pi[k * N + i] = p[k];
-    Pi[i] = P;
+    for (int k = 0; k < 10; k++) f.pi[k * N + i] = p[k];
+    f.Pi[i] = P;
   }
 }
-template <bool FULL>
-__global__ void k_ghost(Geo g, const int* __restrict__ src, const unsigned char* __restrict__ isdst,
-                        double* __restrict__ Q, double* __restrict__ Qh,
-                        double* __restrict__ pi, double* __restrict__ Pi) {
-  d_ghost<FULL>(g, src, isdst, Q, Qh, pi, Pi, blockIdx.x);
+template <bool HALF, bool FULL>
+__global__ void k_ghost(Geo g, Fields f, int* wet, double* tick) {
+  d_ghost<HALF, FULL>(g, f.gsrc, f, wet, tick, blockIdx.x);
 }
 
 
 // ------------------------------------------------ viscous cell prims
-// Per-cell inputs of the viscous stages, one thread per cell:
+// Per-cell inputs of the viscous stages, one thread per cell of the list that
+// the corrector and the ghost copy made of the cells with Qh_t > 0 (in grid
+// order the root finds ran on 17 of a warp's 32 lanes at 101x101x51 with
+// 80 % vacuum):
 //  A  = con2prim(Qh / (tau - dt/2))  (getPrimVarHCenter in ISformal, NSquant,
 //                                     visc_flux, visc_source_step),
 //  D  = con2prim(Qh / tau), e and u  (the six NSquant neighbour velocities),
@@ -519,30 +624,27 @@ __device__ __forceinline__ void d_visc_prims(const Geo& g, const EosDev& E, cons
                                              double* __restrict__ pD, double* __restrict__ pTh,
                                              double* __restrict__ pBC,
                                              const double* __restrict__ clk,
-                                             const unsigned char* __restrict__ isdst,
                                              int* __restrict__ active,
                                              int* __restrict__ nactive, double* __restrict__ TD,
                                              double* __restrict__ TB, double* __restrict__ TC,
-                                             long long blk) {
+                                             long long i, bool in) {
   const double dt = clk[1], tau = clk[0] + dt;  // tau_{n+1} (src/hdo.cpp:1095)
-  const long long i = blk * blockDim.x + threadIdx.x;
   const long long N = g.N;
   double q[7], qh[7];
   const double tA = tau - dt / 2.;
   Prim a{0., 0., 0., 0., 0., 0., 0., 0.};
   int gx = 0, gy = 0, gz = 0;
   bool vac = false;
-  if (i < N) {
+  if (in) {
     coords(g, i, gx, gy, gz);
-    qh[0] = Qh[i];
+#pragma unroll
+    for (int k = 0; k < 7; k++) qh[k] = Qh[k * N + i];
     // A is the corrector's con2prim (k_update<false> stored it in pA) when
     // its divisor tau_n + dt/2 equals tA bit for bit and the ghost copy has
     // not changed this cell's Qh since
-    if (tA == clk[0] + 0.5 * dt && !(isdst[gx] | isdst[g.nx + gy] | isdst[g.nx + g.ny + gz])) {
+    if (tA == clk[0] + 0.5 * dt && !is_ghost(g, gx, gy, gz)) {
       a = loadA(pA, N, i);
     } else {
-#pragma unroll
-      for (int k = 1; k < 7; k++) qh[k] = Qh[k * N + i];
       q_over(qh, tA, q);
       transform_pv<EK>(E, q, a, c2p_guess(E, i));
       pA[0 * N + i] = a.e;
@@ -554,32 +656,21 @@ __device__ __forceinline__ void d_visc_prims(const Geo& g, const EosDev& E, cons
       pA[6 * N + i] = a.vy;
       pA[7 * N + i] = a.vz;
     }
-  }
-  {
-    // the list of cells with matter, for the relaxation and the advection
-    // (the complement of a cell next to vacuum, which NSquant leaves alone):
-    // packed in warp order (one atomic per warp; the order between warps
-    // varies, and every cell's result depends on that cell alone)
-    const bool act = i < N && !(a.e <= 0.);
-    if (act)
+    if (!(a.e <= 0.))
       vac = maxM_at(g, m, gx + 1, gy, gz) <= 0.9 || maxM_at(g, m, gx, gy + 1, gz) <= 0.9 ||
             maxM_at(g, m, gx - 1, gy, gz) <= 0.9 || maxM_at(g, m, gx, gy - 1, gz) <= 0.9 ||
             maxM_at(g, m, gx + 1, gy + 1, gz) <= 0.9 ||
             maxM_at(g, m, gx + 1, gy - 1, gz) <= 0.9 ||
             maxM_at(g, m, gx - 1, gy + 1, gz) <= 0.9 || maxM_at(g, m, gx - 1, gy - 1, gz) <= 0.9;
-    const int lane = threadIdx.x & 31;
-    const unsigned bal = __ballot_sync(0xffffffffu, act);
-    int base = 0;
-    if (lane == 0 && bal) base = atomicAdd(nactive, __popc(bal));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (act) active[base + __popc(bal & ((1u << lane) - 1u))] = vac ? ~(int)i : (int)i;
   }
-  if (i >= N) return;
-  if (qh[0] <= 0.) {  // vacuum: the neighbours read e first, and stop there
-    pD[i] = 0.;
-  } else {
-#pragma unroll
-    for (int k = 1; k < 7; k++) qh[k] = Qh[k * N + i];
+  {
+    // the list of cells with matter, for the relaxation and the advection
+    // (the complement of a cell next to vacuum, which NSquant leaves alone);
+    // every cell's result depends on that cell alone, not on the order
+    append_block(active, nactive, vac ? ~(int)i : (int)i, in && !(a.e <= 0.));
+  }
+  if (!in) return;
+  {
     q_over(qh, tau, q);
     Prim d;
     transform_pv<EK>(E, q, d, c2p_guess(E, i));
@@ -658,14 +749,19 @@ __global__ void __launch_bounds__(128, kPrimsMinBlocks) k_visc_prims(Geo g, EosD
                                                     double* __restrict__ pD,
                                                     double* __restrict__ pTh,
                                                     double* __restrict__ pBC, const double* __restrict__ clk,
-                                                    const unsigned char* __restrict__ isdst,
+                                                    const int* __restrict__ wet,
+                                                    const int* __restrict__ nwet,
                                                     int* __restrict__ active,
                                                     int* __restrict__ nactive,
                                                     double* __restrict__ TD,
                                                     double* __restrict__ TB,
                                                     double* __restrict__ TC) {
-  d_visc_prims<EK, VORT>(g, E, tr, Q, Qprev, Qh, m, pA, pD, pTh, pBC, clk, isdst, active, nactive,
-                         TD, TB, TC, blockIdx.x);
+  const int n = *nwet;
+  for (int b = blockIdx.x * blockDim.x; b < n; b += gridDim.x * blockDim.x) {
+    const int idx = b + threadIdx.x;
+    d_visc_prims<EK, VORT>(g, E, tr, Q, Qprev, Qh, m, pA, pD, pTh, pBC, clk, active, nactive, TD, TB,
+                           TC, idx < n ? wet[idx] : 0, idx < n);
+  }
 }
 
 
@@ -684,15 +780,16 @@ __device__ __forceinline__ double maxM_at(const Geo& g, const double* __restrict
 // (writing them, 208 bytes a cell, took 25 us of a 988 us step at 101x101x51
 // with 80 % vacuum).  One thread per cell, every index a compile-time
 // constant; the con2prims and the thermodynamics come precomputed from
-// k_visc_prims.  Four 128-thread blocks per SM (128 registers) hide the FP64
-// latency better than fewer, spill-free ones (measured: 3 and 2 blocks per SM
-// are 7 % and 35 % slower, 5 and 6 are 9 % and 3 % slower).
-constexpr int kRelaxMinBlocks = 4;
+// k_visc_prims.  Three 128-thread blocks per SM (168
+// registers): with four (128 registers, 450 bytes of spills) 112 instead of
+// 89 us a step at 101x101x51 and 298 instead of 259 at 201x201x101, with two
+// (no spills) 97 and 301.
+constexpr int kRelaxMinBlocks = 3;
 
 constexpr int kRelaxBlock = 128;
 // shared-memory rows of k_is_relax's relaxation loops: pi, sigma, u, h0, f0,
 // and phi7 h0^{kl} - tau_pipi sigma^{kl} of the second loop (dynamic shared
-// memory: 55 KB per block, four blocks per SM)
+// memory: 55 KB per block)
 constexpr int kSmPI = 0, kSmSIG = 10, kSmU = 20, kSmH = 24, kSmF = 34, kSmY = 44, kSmRows = 54;
 constexpr size_t kRelaxSmem = sizeof(double) * kSmRows * kRelaxBlock;
 
@@ -1452,7 +1549,7 @@ __device__ __forceinline__ void d_is_relax(
     double* __restrict__ Pi0, double* __restrict__ PiH0, double* __restrict__ flux,
     const double* __restrict__ clk, unsigned* err, const int* __restrict__ active,
     const int* __restrict__ nactive, long long blk) {
-  const int idx = (int)(blk * blockDim.x + threadIdx.x);
+  const long long idx = blk * blockDim.x + threadIdx.x;
   if (idx >= *nactive) return;
   const int entry = active[idx];  // a cell with matter (k_visc_prims)
   const bool vac = entry < 0;     // next to vacuum
@@ -1475,7 +1572,10 @@ __global__ void __launch_bounds__(kRelaxBlock, kRelaxMinBlocks) k_is_relax(
 // ------------------------------------------------ ISformal, loop #2
 // Semi-Lagrangian advection of pi0/piH0 from the 2x2x2 upwind cells, the
 // viscous-correction limiter and the -(tau) * delta Q_{n+1} flux
-// (src/hdo.cpp:866-962).
+// (src/hdo.cpp:866-962).  Bound by the latency of its 176 scattered loads a
+// cell.  Two threads per cell (pi and piH apart, 64 registers, 8 blocks per
+// SM) were slower: 49 against 42 us at 101x101x51, 206 against 118 at
+// 201x201x101.
 __device__ __forceinline__ double sgn(double x) {
   if (x > 0) return 1.;
   if (x < 0.) return -1.;
@@ -1784,6 +1884,9 @@ static int launch_step_ek(const StepArgs& a, cudaStream_t s, LaunchMarker* mk) {
   const unsigned nface = (unsigned)std::min(fblocks, resident);
   const unsigned char* fact = lists ? a.f.fact : nullptr;
   const bool vort = a.vort && a.viscous;
+  const unsigned wide = 128 / bs;
+  const unsigned nprims = std::min(nb, 148 * kPrimsMinBlocks * wide);
+  const unsigned ngh = nblk(ghost_shell(g).n, bs);
   int launches = 0;
   const Fields& F = a.f;
   auto done = [&](int kind) {
@@ -1808,22 +1911,26 @@ static int launch_step_ek(const StepArgs& a, cudaStream_t s, LaunchMarker* mk) {
     if (pred)
       k_update<true, EK><<<nb, bs, 0, s>>>(g, a.eos, F.Q, F.Qh, F.Qprev, F.Fx, F.Fy, F.Fz, fact, a.clk,
                                            F.err, a.viscous ? F.pBC : nullptr, nullptr,
-                                           vort ? a.vort->TB : nullptr);
+                                           vort ? a.vort->TB : nullptr, nullptr, nullptr, nullptr);
     else
       k_update<false, EK><<<nb, bs, 0, s>>>(g, a.eos, F.Q, F.Qh, F.Qprev, F.Fx, F.Fy, F.Fz, fact, a.clk,
-                                            F.err, nullptr, a.viscous ? F.pA : nullptr, nullptr);
+                                            F.err, nullptr, a.viscous ? F.pA : nullptr, nullptr, F.pD,
+                                            F.wet, F.fcount + 6);
     done(KK_UPDATE);
   }
-  k_ghost<false><<<nb, bs, 0, s>>>(g, F.gsrc, F.gdst, F.Q, F.Qh, F.pi, F.Pi);
-  done(KK_GHOST);
-  if (a.viscous) {
+  if (!a.viscous) {
+    k_ghost<true, true><<<ngh, bs, 0, s>>>(g, F, nullptr, a.tick);
+    done(KK_GHOST);
+  } else {
+    k_ghost<true, false><<<ngh, bs, 0, s>>>(g, F, F.wet, nullptr);
+    done(KK_GHOST);
     if (vort)
-      k_visc_prims<EK, true><<<nb, bs, 0, s>>>(g, a.eos, a.tr, F.Q, F.Qprev, F.Qh, m, F.pA, F.pD,
-                                               F.pTh, F.pBC, a.clk, F.gdst, F.active, F.nactive,
+      k_visc_prims<EK, true><<<nprims, bs, 0, s>>>(g, a.eos, a.tr, F.Q, F.Qprev, F.Qh, m, F.pA, F.pD,
+                                               F.pTh, F.pBC, a.clk, F.wet, F.fcount + 6, F.active, F.nactive,
                                                a.vort->TD, a.vort->TB, a.vort->TC);
     else
-      k_visc_prims<EK, false><<<nb, bs, 0, s>>>(g, a.eos, a.tr, F.Q, F.Qprev, F.Qh, m, F.pA, F.pD,
-                                                F.pTh, F.pBC, a.clk, F.gdst, F.active, F.nactive,
+      k_visc_prims<EK, false><<<nprims, bs, 0, s>>>(g, a.eos, a.tr, F.Q, F.Qprev, F.Qh, m, F.pA, F.pD,
+                                                F.pTh, F.pBC, a.clk, F.wet, F.fcount + 6, F.active, F.nactive,
                                                 nullptr, nullptr, nullptr);
     done(KK_VISC_PRIMS);
     if (vort) {
@@ -1840,9 +1947,9 @@ static int launch_step_ek(const StepArgs& a, cudaStream_t s, LaunchMarker* mk) {
     done(KK_IS_ADVECT);
     k_visc_update<<<nb, bs, 0, s>>>(g, F.pA, F.piH, F.PiH, m, F.flux, F.Q, a.clk);
     done(KK_VISC_UPDATE);
+    k_ghost<false, true><<<ngh, bs, 0, s>>>(g, F, nullptr, a.tick);
+    done(KK_GHOST);
   }
-  k_ghost<true><<<nb, bs, 0, s>>>(g, F.gsrc, F.gdst, F.Q, F.Qh, F.pi, F.Pi);
-  done(KK_GHOST);
   return launches;
 }
 
@@ -1972,24 +2079,28 @@ __global__ void __launch_bounds__(128, kUpdateMinBlocks) kb_update(const StepDev
   double* pB = PRED && A.viscous ? A.f.pBC : nullptr;
   double* pA = !PRED && A.viscous ? A.f.pA : nullptr;
   d_update<PRED, EK>(g, E, A.f.Q, A.f.Qh, A.f.Qprev, A.f.Fx, A.f.Fy, A.f.Fz, A.f.fact, A.clk,
-                     A.f.err, pB, pA, nullptr, blk);
+                     A.f.err, pB, pA, nullptr, A.f.pD, A.f.wet, A.f.fcount + 6, blk);
 }
 
-template <bool FULL>
+template <bool HALF, bool FULL>
 __global__ void kb_ghost(const StepDev* __restrict__ evs, const BItem* __restrict__ items) {
   VH_ITEM
-  d_ghost<FULL>(g, A.f.gsrc, A.f.gdst, A.f.Q, A.f.Qh, A.f.pi, A.f.Pi, blk);
+  d_ghost<HALF, FULL>(g, A.f.gsrc, A.f, HALF && A.viscous ? A.f.wet : nullptr, FULL ? A.clk : nullptr,
+                      blk);
 }
 
 template <int EK>
 __global__ void __launch_bounds__(128, kPrimsMinBlocks) kb_visc_prims(const StepDev* __restrict__ evs,
                                                      const BItem* __restrict__ items) {
   VH_ITEM
+  const int n = A.f.fcount[6];
+  const long long first = blk * blockDim.x, idx = first + threadIdx.x;
+  if (first >= n) return;
   const EosDev E = A.eos;
   const TrDev tr = A.tr;
   d_visc_prims<EK, false>(g, E, tr, A.f.Q, A.f.Qprev, A.f.Qh, A.f.m2, A.f.pA, A.f.pD, A.f.pTh,
-                   A.f.pBC, A.clk, A.f.gdst, A.f.active, A.f.nactive, nullptr,
-                   nullptr, nullptr, blk);
+                   A.f.pBC, A.clk, A.f.active, A.f.nactive, nullptr,
+                          nullptr, nullptr, idx < n ? A.f.wet[idx] : 0, idx < n);
 }
 
 __global__ void __launch_bounds__(kRelaxBlock, kRelaxMinBlocks) kb_is_relax(
@@ -2042,17 +2153,20 @@ static int launch_step_batched_ek(bool viscous, const StepDev* evs, int nev, con
   kb_face_list<<<nb, kBatchBlock, 0, s>>>(evs, items, false);
   kb_face<EK><<<fgrid, kBatchBlock, 0, s>>>(evs, items, false);
   kb_update<false, EK><<<nb, kBatchBlock, 0, s>>>(evs, items);
-  kb_ghost<false><<<nb, kBatchBlock, 0, s>>>(evs, items);
-  launches += 7;
-  if (viscous) {
+  launches += 6;
+  if (!viscous) {
+    kb_ghost<true, true><<<nb, kBatchBlock, 0, s>>>(evs, items);
+    launches++;
+  } else {
+    kb_ghost<true, false><<<nb, kBatchBlock, 0, s>>>(evs, items);
     kb_visc_prims<EK><<<nb, kBatchBlock, 0, s>>>(evs, items);
     kb_is_relax<<<nb, kRelaxBlock, kRelaxSmem, s>>>(evs, items);
     kb_is_advect<<<nb, kBatchBlock, 0, s>>>(evs, items);
     kb_visc_update<<<nb, kBatchBlock, 0, s>>>(evs, items);
-    launches += 4;
+    kb_ghost<false, true><<<nb, kBatchBlock, 0, s>>>(evs, items);
+    launches += 6;
   }
-  kb_ghost<true><<<nb, kBatchBlock, 0, s>>>(evs, items);
-  return launches + 1;
+  return launches;
 }
 
 int step_ek(const EosDev& E) {

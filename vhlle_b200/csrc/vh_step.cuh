@@ -91,7 +91,9 @@ struct Fields {
                                  // fact has the direction's bit
   unsigned char *fact;           // [N] bit d: the +d face may carry a flux
   int *flist;                    // [3][N] the cells whose +d face may
-  int *fcount;                   // [6] their numbers: predictor, corrector
+  int *fcount;                   // [7] their numbers: predictor, corrector;
+                                 // the number of wet cells
+  int *wet;                      // [N] cells with Qh_t > 0 (viscous steps)
   double *flux;                  // [4][N] viscous flux accumulator
   double *pA;                    // [8][N] prims of Qh at tau_{n+1} - dt/2
   double *pD;                    // [5][N] e, u^mu of Qh at tau_{n+1}
@@ -126,6 +128,7 @@ struct StepArgs {
   TrDev tr;
   Fields f;
   const double* clk;  // device [tau, dt] of the step (launch_clock_set)
+  double* tick = nullptr;  // the clock the step's last kernel advances, if any
   bool viscous;
   int block = 128;    // threads per block of the step kernels (64 or 128; the
                       // relaxation kernel always uses 128)
@@ -186,7 +189,8 @@ cudaError_t step_kernels_setup();
 // Whether launch_step lists the faces that can carry a flux (two launches
 // more) on this grid, with bs threads per block.
 bool face_lists(const Geo& g, int bs);
-// Enqueues one performStep on stream s; returns the number of launches.
+// Enqueues one performStep on stream s, and tau += dt on a.tick; returns the
+// number of launches.
 // Leaves the updated fill fractions in f.m2 (the caller swaps m and m2).
 int launch_step(const StepArgs& a, cudaStream_t s, LaunchMarker* mk = nullptr);
 void launch_clock_set(double* clk, double tau, double dt, cudaStream_t s);
