@@ -205,9 +205,9 @@ __device__ bool lines_equal(const Line& l1, const Line& l2) {
 
 // ---------------------------------------------------------------------
 // The warp's part: 48 square instances (8 3-cubes x 6 squares) across the
-// lanes, each 3-cube's polygons in one of 8 lanes, the joining into
-// polyhedra in lane 0, the tetrahedra of the centroid and normal sums across
-// the lanes.
+// lanes, each 3-cube's polygons in one of 8 lanes, the comparisons of the
+// polygons across the lanes and their joining into polyhedra in lane 0, the
+// tetrahedra of the centroid and normal sums across the lanes.
 namespace cnw {
 
 using cn::kEps;
@@ -233,6 +233,11 @@ struct WarpWork {
   // reference's sums: element e owns tetrahedra es[e] .. es[e+1]-1
   unsigned char tp[96], tl[96];  // polygon code (8 * 3-cube + polygon), line id
   int es[kMaxElem + 1], nel;
+  // the polygons in the reference's order, and for an ambiguous hypercube
+  // bit q of adj[i]: polygon i has a line equal to one of polygon q
+  unsigned char fl[64];
+  int nf, amb;
+  unsigned long long adj[64];
   double term[96][5];  // per-tetrahedron terms of the current sum
 };
 
@@ -380,17 +385,14 @@ __device__ void cube_polygons(WarpWork& w, int c) {
   for (int q = 0; q < np; q++) poly_centroid(w, w.P[c][q], c >> 1);
 }
 
-// Hypercube::check_ambiguous + construct_polyhedrons (src/cornelius.cpp:
-// 1776-1878), one lane: fills the tetrahedron list and w.nel (-1 where the
-// reference stops).
-__device__ void assemble(WarpWork& w, double E0) {
-  int namb = 0, nlines = 0;
-  unsigned char fl[64];  // polygons in the reference's order: 3-cube, then polygon
-  int nf = 0;
+// Hypercube::check_ambiguous (src/cornelius.cpp:1776-1800), one lane: the
+// polygon list and whether the polyhedra have to be told apart.
+__device__ void list_polygons(WarpWork& w, double E0) {
+  int namb = 0, nlines = 0, nf = 0;
   for (int c = 0; c < 8; c++) {
     if (w.camb[c]) namb++;
     nlines += w.nl[c];
-    for (int q = 0; q < w.np[c]; q++) fl[nf++] = (unsigned char)(8 * c + q);
+    for (int q = 0; q < w.np[c]; q++) w.fl[nf++] = (unsigned char)(8 * c + q);
   }
   int amb = namb;
   if (amb == 0) {
@@ -401,31 +403,58 @@ __device__ void assemble(WarpWork& w, double E0) {
     if (pts > 8) pts = 16 - pts;
     if (nlines == 24 && pts == 2) amb++;
   }
-  unsigned char ph[kMaxElem][64];
-  int nph[kMaxElem], nel = 0;
-  if (amb > 0) {
-    unsigned long long unused = nf >= 64 ? ~0ull : ((1ull << nf) - 1);
-    int used = 0;
+  w.nf = nf;
+  w.amb = amb;
+}
+
+// Which polygons share a line (Polyhedron::lines_equal over their lines), all
+// lanes, a pair each.  In one lane, inside the joining loop, these
+// comparisons took most of the kernel's time: an ambiguous hypercube has
+// over a thousand, and a warp waited for them (a surface of 10 thousand
+// elements: 372 us then, 212 so).
+__device__ void polygon_pairs(WarpWork& w) {
+  const int lane = threadIdx.x & 31, nf = w.nf;
+  for (int i = lane; i < nf; i += 32) w.adj[i] = 0;
+  __syncwarp();
+  for (int t = lane; t < nf * nf; t += 32) {
+    const int i = t / nf, q = t - i * nf;
+    if (i == q) continue;
+    const Poly& p = w.P[w.fl[i] >> 3][w.fl[i] & 7];
+    const Poly& pq = w.P[w.fl[q] >> 3][w.fl[q] & 7];
+    bool eq = false;
+    for (int j = 0; j < p.n && !eq; j++)
+      for (int k = 0; k < pq.n && !eq; k++) eq = cn::lines_equal(w.L[p.li[j]], w.L[pq.li[k]]);
+    if (eq) atomicOr(&w.adj[i], 1ull << q);
+  }
+}
+
+// Hypercube::construct_polyhedrons (src/cornelius.cpp:1802-1878), one lane:
+// fills the tetrahedron list and w.nel (-1 where the reference stops).
+__device__ void assemble(WarpWork& w) {
+  const int nf = w.nf;
+  unsigned long long unused = nf >= 64 ? ~0ull : ((1ull << nf) - 1);
+  int used = 0, nel = 0, nt = 0;
+  auto take = [&](int f) {  // polygon f's lines as the current element's next tetrahedra
+    const Poly& pg = w.P[w.fl[f] >> 3][w.fl[f] & 7];
+    for (int j = 0; j < pg.n; j++) {
+      w.tp[nt] = w.fl[f];
+      w.tl[nt] = pg.li[j];
+      nt++;
+    }
+  };
+  if (w.amb > 0) {
     do {
       if (nel >= kMaxElem) {
         w.nel = -1;
         return;
       }
-      nph[nel] = 0;
+      w.es[nel] = nt;
+      unsigned long long group = 0;
       for (int i = 0; i < nf; i++) {
         if (!((unused >> i) & 1)) continue;
-        bool add = nph[nel] == 0;
-        if (!add) {
-          const Poly& p = w.P[fl[i] >> 3][fl[i] & 7];
-          for (int q = 0; q < nph[nel] && !add; q++) {
-            const Poly& pq = w.P[ph[nel][q] >> 3][ph[nel][q] & 7];
-            for (int j = 0; j < p.n && !add; j++)
-              for (int k = 0; k < pq.n && !add; k++)
-                if (cn::lines_equal(w.L[p.li[j]], w.L[pq.li[k]])) add = true;
-          }
-        }
-        if (add) {
-          ph[nel][nph[nel]++] = fl[i];
+        if (group == 0 || (w.adj[i] & group)) {
+          group |= 1ull << i;
+          take(i);
           unused &= ~(1ull << i);
           used++;
           i = 0;
@@ -434,21 +463,9 @@ __device__ void assemble(WarpWork& w, double E0) {
       nel++;
     } while (used < nf);
   } else {
-    nph[0] = 0;
-    for (int i = 0; i < nf; i++) ph[0][nph[0]++] = fl[i];
+    w.es[0] = 0;
+    for (int i = 0; i < nf; i++) take(i);
     nel = 1;
-  }
-  int nt = 0;
-  for (int e = 0; e < nel; e++) {
-    w.es[e] = nt;
-    for (int q = 0; q < nph[e]; q++) {
-      const Poly& pg = w.P[ph[e][q] >> 3][ph[e][q] & 7];
-      for (int j = 0; j < pg.n; j++) {
-        w.tp[nt] = ph[e][q];
-        w.tl[nt] = pg.li[j];
-        nt++;
-      }
-    }
   }
   w.es[nel] = nt;
   w.nel = nel;
@@ -556,12 +573,14 @@ __device__ int find_surface_warp(WarpWork& w, const double* dx, double E0, doubl
   __syncwarp();
   if (lane < 8) cube_polygons(w, lane);
   __syncwarp();
-  if (lane == 0) {
-    if (w.err)
-      w.nel = -1;
-    else
-      assemble(w, E0);
+  if (w.err) return -1;  // uniform across the warp
+  if (lane == 0) list_polygons(w, E0);
+  __syncwarp();
+  if (w.amb > 0) {
+    polygon_pairs(w);
+    __syncwarp();
   }
+  if (lane == 0) assemble(w);
   __syncwarp();
   const int nel = w.nel;
   for (int e = 0; e < nel; e++) element(w, e, geo);

@@ -20,6 +20,7 @@
 namespace vh {
 
 // Fluid::getCMFvariables, src/fld.cpp:50-60
+template <int EK>
 __device__ __forceinline__ void cmf_variables(const EosDev& E, const double* __restrict__ Q,
                                               long long N, long long i, double eta, double tau,
                                               Prim& P, double& Y) {
@@ -27,7 +28,7 @@ __device__ __forceinline__ void cmf_variables(const EosDev& E, const double* __r
 #pragma unroll
   for (int k = 0; k < 7; k++) qs[k] = Q[k * N + i];
   q_over(qs, tau, q);
-  transform_pv(E, q, P);
+  transform_pv<EK>(E, q, P);
   Y = eta + 1. / 2. * log((1. + P.vz) / (1. - P.vz));
   P.vx = P.vx * cosh(Y - eta) / cosh(Y);
   P.vy = P.vy * cosh(Y - eta) / cosh(Y);
@@ -41,6 +42,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 
 constexpr int kTotBlock = 256;
 
+template <int EK>
 __global__ void __launch_bounds__(kTotBlock) k_totals(Geo g, EosDev E, const double* __restrict__ Q,
                                                       const double* __restrict__ pi,
                                                       const double* __restrict__ vcc, double tau,
@@ -54,21 +56,25 @@ __global__ void __launch_bounds__(kTotBlock) k_totals(Geo g, EosDev E, const dou
 #pragma unroll
   for (int k = 0; k < kTotals; k++) c[k] = 0.;
   if (t < nint) {
-    // interior cell, z fastest like the reference loop (ix, iy outer)
-    const int iz = g.zt0 + (int)(t % niz);
-    const int iy = 2 + (int)((t / niz) % niy);
-    const int ix = 2 + (int)(t / ((long long)niz * niy));
+    // interior cell, x fastest (a warp reads consecutive cells; with z
+    // fastest, as the reference loops, every lane's 18 loads were in lines
+    // of their own)
+    const unsigned r = (unsigned)(t / nix);
+    const int ix = 2 + (int)(t - (long long)r * nix);
+    const int iy = 2 + (int)(r % (unsigned)niy);
+    const int iz = g.zt0 + (int)(r / (unsigned)niy);
     const long long N = g.N;
     const long long i = ix + (long long)g.nx * iy + (long long)g.nx * g.ny * iz;
     const double dz = g.dz;
     const double eta = etamin + iz * dz;
     Prim P;
     double vz;
-    cmf_variables(E, Q, N, i, eta, tau, P, vz);
+    cmf_variables<EK>(E, Q, N, i, eta, tau, P, vz);
     const double e = P.e, vx = P.vx, vy = P.vy;
-    double T, mub, p;
-    eos_eval(E, e, P.nb, T, mub, p);
-    double s = eos_s(E, e, P.nb, P.nq, P.ns);
+    // EoS::eos and EoS::s at the same point (eos_s) from one lookup
+    double T, mub, muq, mus, p;
+    eos_eval_q<EK>(E, e, P.nb, T, mub, muq, mus, p);
+    double s = T > 0.0 ? ddivp(e + p - mub * P.nb - muq * P.nq - mus * P.ns, T) : 0.;
     const double cosh_int = (sinh(eta + 0.5 * dz) - sinh(eta - 0.5 * dz)) / dz;
     const double sinh_int = (cosh(eta + 0.5 * dz) - cosh(eta - 0.5 * dz)) / dz;
     const double th = tanh(vz);
@@ -166,7 +172,14 @@ int totals_blocks(const Geo& g) {
 void launch_totals(const Geo& g, const EosDev& E, const Fields& f, double tau, double ecrit,
                    double etamin, bool viscous, double* partial, double* out, cudaStream_t s) {
   const int nb = totals_blocks(g);
-  k_totals<<<nb, kTotBlock, 0, s>>>(g, E, f.Q, f.pi, f.vcc, tau, ecrit, etamin, viscous, partial);
+  // the common table kinds alone, the others by kind at run time: with every
+  // kind's lookup compiled in, the kernel held 2 blocks per SM
+  if (E.kind <= 1)
+    k_totals<EK_TABLE><<<nb, kTotBlock, 0, s>>>(g, E, f.Q, f.pi, f.vcc, tau, ecrit, etamin, viscous,
+                                                partial);
+  else
+    k_totals<EK_ANY><<<nb, kTotBlock, 0, s>>>(g, E, f.Q, f.pi, f.vcc, tau, ecrit, etamin, viscous,
+                                              partial);
   k_totals_final<<<1, kTotBlock, 0, s>>>(partial, nb, out);
 }
 
