@@ -77,6 +77,29 @@ def test_pressure_at_zero_charge(kind, nbaxis):
     h.close()
 
 
+@pytest.mark.parametrize("kind", ["log", "linear", "from_zero", "irregular"])
+@pytest.mark.parametrize("nbaxis", ["two", "many", "symmetric", "above_zero", "off_zero"])
+def test_lookup_with_charge(kind, nbaxis):
+    """The table at nb != 0 (its packed axis, its last cells, outside it)
+    equals the oracle's in every output."""
+    eg = _axis(kind, 301)
+    ng = {"two": np.array([0., 1.]), "many": np.linspace(0., 1., 40), "symmetric": np.linspace(-1., 1., 41),
+          "above_zero": np.linspace(0.1, 1., 7), "off_zero": np.linspace(-0.95, 1., 40)}[nbaxis]
+    E, B = np.meshgrid(eg, ng)
+    s = W.small_glauber3d(5, 5)
+    s.eos = W.EosTable(kind=1, egrid=eg, ngrid=ng, p=(0.3 * E - 0.01 + 0.02 * B * B).reshape(-1),
+                       T=(0.1 + 0.05 * E ** 0.25 + 0.01 * B).reshape(-1), mub=(B * (1. + 0.01 * E)).reshape(-1))
+    rng = np.random.default_rng(3)
+    axis = np.concatenate([ng, np.nextafter(ng, -9), np.nextafter(ng, 9), [-3., 3., -0., 1e-300, -1e-300, 1e9]])
+    ends = np.concatenate([eg[:3], eg[-3:], np.nextafter(eg[:3], 1e9), np.nextafter(eg[-3:], 0), [0., 5e-324, 1e9]])
+    e, nb = (a.reshape(-1) for a in np.meshgrid(ends, axis))
+    e = np.concatenate([e, rng.uniform(0., 100., 3000), 10. ** rng.uniform(-9, 4, 3000), rng.choice(eg, 500)])
+    nb = np.concatenate([nb, rng.uniform(-1.5, 1.5, 6000), rng.choice(axis, 500)])
+    h, o = capi.GpuHydro(s), P.OracleRun(s)
+    assert np.array_equal(h.eos6(e, nb), o.eos6(e, nb), equal_nan=True)
+    h.close()
+
+
 @pytest.mark.parametrize("eos", ["table", "nb_table", "conformal", "chiral"])
 def test_root_find_equals_oracle(eos):
     """transformPV from vacuum and rest to |M| > Q_t, over 24 decades, with and

@@ -333,6 +333,29 @@ static vh_status upload_eos(vh_ctx* c, const vh_eos* eos, vh::EosDev& E) {
       }
       rdev += r.size();
     }
+    // the axes packed per interval (eos1f_packed)
+    E.eax = E.nax = nullptr;
+    if (E.erinv && E.nrinv && E.emode != vh::GRID_BSEARCH && (nn <= 2 || E.nmode != vh::GRID_BSEARCH) &&
+        eos->egrid[0] >= 0x1p-800) {
+      std::vector<double> ax((size_t)4 * (ne - 1 + nn - 1));
+      double* v = ax.data();
+      for (int a = 0; a < 2; a++)
+        for (int k = 0; k + 1 < lens[a]; k++, v += 4) {
+          const double den = axes[a][k + 1] - axes[a][k];
+          v[0] = axes[a][k];
+          v[1] = axes[a][k + 1];
+          v[2] = 1.0 / den;
+          v[3] = den;
+        }
+      double* dev = nullptr;
+      if ((st = dalloc(c, &dev, ax.size())) != VH_OK) return st;
+      if ((e = cudaMemcpy(dev, ax.data(), ax.size() * sizeof(double), cudaMemcpyHostToDevice))) {
+        cuda_fail(c, e, "vh_create: EoS upload");
+        return VH_ERR_CUDA;
+      }
+      E.eax = reinterpret_cast<const double2*>(dev);
+      E.nax = E.eax + 2 * (ne - 1);
+    }
     // the row of nb = 0 (eos1f_row0): its bracket as the binary search finds
     // it, where the bracket starts at 0 exactly and no term of the next row
     // can be anything but +-0

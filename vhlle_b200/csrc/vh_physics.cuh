@@ -79,6 +79,11 @@ struct EosDev {
   // interpolation weights then take crm::mk_div instead of a divide
   const double* __restrict__ erinv;
   const double* __restrict__ nrinv;
+  // kind 1, axes with an index guess and interval reciprocals: per interval
+  // {g[k], g[k+1]}, {RN(1/(g[k+1]-g[k])), g[k+1]-g[k]}; both or neither
+  // (eos1f_packed; every egrid point at least 2^-800)
+  const double2* __restrict__ eax;
+  const double2* __restrict__ nax;
   // kind 1: the lookup at nb = 0 where that is one row of the table (its nb
   // bracket starts at 0 and the row's and the next row's p are finite), per
   // e interval {g[k], g[k+1]}, {RN(1/(g[k+1]-g[k])), g[k+1]-g[k]},
@@ -245,6 +250,69 @@ __device__ __forceinline__ bool is_bracket(int k, int n, double x, double gk, do
   return (k == 0 || !(x < gk)) && (k == n - 2 || x < gk1);
 }
 
+// eos1f with the axes packed per interval: four 16-byte loads for the two
+// brackets instead of six 8-byte ones from three arrays, fixed steps of one
+// on a wrong guess, and the e weight's division without a range test (e - g
+// is +0 or at least 2^-853; where the quotient overflows the sums are NaN
+// either way).  The same operations on the same values, so the same bits.
+template <bool WANT_T, bool WANT_D>
+__device__ __forceinline__ void eos1f_packed(const EosDev& E, double e, double nb, double& T,
+                                             double& mub, double& p, double* dpde, double* dpdn) {
+  const int ne = E.ne, nn = E.nn;
+  const float fe = (float)e, fn = (float)nb;
+  const float te = (E.emode == GRID_LOG ? __log2f(fe) - E.e0 : fe - E.e0) * E.einv;
+  const float tn = (E.nmode == GRID_LOG ? __log2f(fn) - E.n0 : fn - E.n0) * E.ninv;
+  // (a NaN guesses 0: its sums are NaN in any bracket)
+  int ke = (int)fminf(fmaxf(te, 0.f), (float)(ne - 2));
+  int kn = nn <= 2 ? 0 : (int)fminf(fmaxf(tn, 0.f), (float)(nn - 2));
+  double2 ge = __ldg(E.eax + 2 * ke), de = __ldg(E.eax + 2 * ke + 1);
+  double2 gn = __ldg(E.nax + 2 * kn), dn = __ldg(E.nax + 2 * kn + 1);
+  while ((ke > 0 && e < ge.x) || (ke < ne - 2 && e >= ge.y)) {
+    ke += e < ge.x ? -1 : 1;
+    ge = __ldg(E.eax + 2 * ke);
+    de = __ldg(E.eax + 2 * ke + 1);
+  }
+  while ((kn > 0 && nb < gn.x) || (kn < nn - 2 && nb >= gn.y)) {
+    kn += nb < gn.x ? -1 : 1;
+    gn = __ldg(E.nax + 2 * kn);
+    dn = __ldg(E.nax + 2 * kn + 1);
+  }
+  const double num = e - ge.x, q0 = num * de.x;
+  const double ue = fma(fma(-q0, de.y, num), de.x, q0);
+  const double un = interp_weight(nb, gn.x, gn.y, true, dn.x);
+  const int b00 = ke + ne * kn, b01 = b00 + ne;
+  const double we0 = 1. - ue, we1 = ue;
+  const double wn0 = 1. - un, wn1 = un;
+  const double p00 = __ldg(E.p + b00), p01 = __ldg(E.p + b01);
+  const double p10 = __ldg(E.p + b00 + 1), p11 = __ldg(E.p + b01 + 1);
+  double sp = 0.;
+  sp += we0 * wn0 * p00;
+  sp += we0 * wn1 * p01;
+  sp += we1 * wn0 * p10;
+  sp += we1 * wn1 * p11;
+  if (WANT_D) {
+    const double se = wn0 * (p10 - p00) + wn1 * (p11 - p01);
+    const double sn = we0 * (p01 - p00) + we1 * (p11 - p10);
+    *dpde = sp < 0. ? 0. : se * de.x;
+    *dpdn = sp < 0. ? 0. : sn * dn.x;
+  }
+  if (sp < 0.) sp = 0.;
+  p = sp;
+  if (WANT_T) {
+    double sT = 0., sm = 0.;
+    sT += we0 * wn0 * __ldg(E.T + b00);
+    sT += we0 * wn1 * __ldg(E.T + b01);
+    sT += we1 * wn0 * __ldg(E.T + b00 + 1);
+    sT += we1 * wn1 * __ldg(E.T + b01 + 1);
+    sm += we0 * wn0 * __ldg(E.mub + b00);
+    sm += we0 * wn1 * __ldg(E.mub + b01);
+    sm += we1 * wn0 * __ldg(E.mub + b00 + 1);
+    sm += we1 * wn1 * __ldg(E.mub + b01 + 1);
+    T = sT;
+    mub = sm;
+  }
+}
+
 // EoS1f::eos, src/eo1.cpp:100-123.  Both axes' brackets are guessed
 // without loads (or searched, for an axis without a guess), and the bracket
 // ends, the interval reciprocals and the four table corners are loaded
@@ -257,6 +325,10 @@ template <bool WANT_T, bool WANT_D = false>
 __device__ __forceinline__ void eos1f(const EosDev& E, double e, double nb,
                                       double& T, double& mub, double& p, double* dpde = nullptr,
                                       double* dpdn = nullptr) {
+  if (E.eax) {
+    eos1f_packed<WANT_T, WANT_D>(E, e, nb, T, mub, p, dpde, dpdn);
+    return;
+  }
   const int ne = E.ne, nn = E.nn;
   int ke, kn, k2;
   if (E.emode == GRID_BSEARCH || ne <= 2)
