@@ -583,10 +583,14 @@ __global__ void k_ghost(Geo g, Fields f, int* wet, double* tick) {
 
 
 // ------------------------------------------------ viscous cell prims
-// Per-cell inputs of the viscous stages, one thread per cell of the list that
-// the corrector and the ghost copy made of the cells with Qh_t > 0 (in grid
-// order the root finds ran on 17 of a warp's 32 lanes at 101x101x51 with
-// 80 % vacuum):
+// Per-cell inputs of the viscous stages over the list that the corrector and
+// the ghost copy made of the cells with Qh_t > 0 (in grid order the root finds
+// ran on 17 of a warp's 32 lanes at 101x101x51 with 80 % vacuum).  Two threads
+// per cell, in the two halves of a block: the first takes A, D and the
+// thermodynamics, the second B and C.  A cell is a chain of root finds, which
+// the few cells of a coarse grid do not hide (us per step with one thread and
+// with two: 47x61x23 24.9 and 20.0, 101x101x51 32.6 and 33.5, 201x201x101 90.7
+// and 90.6; 101x101x51 with charge 35.4 and 37.8):
 //  A  = con2prim(Qh / (tau - dt/2))  (getPrimVarHCenter in ISformal, NSquant,
 //                                     visc_flux, visc_source_step),
 //  D  = con2prim(Qh / tau), e and u  (the six NSquant neighbour velocities),
@@ -627,7 +631,7 @@ __device__ __forceinline__ void d_visc_prims(const Geo& g, const EosDev& E, cons
                                              int* __restrict__ active,
                                              int* __restrict__ nactive, double* __restrict__ TD,
                                              double* __restrict__ TB, double* __restrict__ TC,
-                                             long long i, bool in) {
+                                             long long i, bool in, bool second) {
   const double dt = clk[1], tau = clk[0] + dt;  // tau_{n+1} (src/hdo.cpp:1095)
   const long long N = g.N;
   double q[7], qh[7];
@@ -637,24 +641,26 @@ __device__ __forceinline__ void d_visc_prims(const Geo& g, const EosDev& E, cons
   bool vac = false;
   if (in) {
     coords(g, i, gx, gy, gz);
-#pragma unroll
-    for (int k = 0; k < 7; k++) qh[k] = Qh[k * N + i];
     // A is the corrector's con2prim (k_update<false> stored it in pA) when
     // its divisor tau_n + dt/2 equals tA bit for bit and the ghost copy has
     // not changed this cell's Qh since
     if (tA == clk[0] + 0.5 * dt && !is_ghost(g, gx, gy, gz)) {
       a = loadA(pA, N, i);
     } else {
+#pragma unroll
+      for (int k = 0; k < 7; k++) qh[k] = Qh[k * N + i];
       q_over(qh, tA, q);
       transform_pv<EK>(E, q, a, c2p_guess(E, i));
-      pA[0 * N + i] = a.e;
-      pA[1 * N + i] = a.p;
-      pA[2 * N + i] = a.nb;
-      pA[3 * N + i] = a.nq;
-      pA[4 * N + i] = a.ns;
-      pA[5 * N + i] = a.vx;
-      pA[6 * N + i] = a.vy;
-      pA[7 * N + i] = a.vz;
+      if (!second) {
+        pA[0 * N + i] = a.e;
+        pA[1 * N + i] = a.p;
+        pA[2 * N + i] = a.nb;
+        pA[3 * N + i] = a.nq;
+        pA[4 * N + i] = a.ns;
+        pA[5 * N + i] = a.vx;
+        pA[6 * N + i] = a.vy;
+        pA[7 * N + i] = a.vz;
+      }
     }
     if (!(a.e <= 0.))
       vac = maxM_at(g, m, gx + 1, gy, gz) <= 0.9 || maxM_at(g, m, gx, gy + 1, gz) <= 0.9 ||
@@ -667,27 +673,33 @@ __device__ __forceinline__ void d_visc_prims(const Geo& g, const EosDev& E, cons
     // the list of cells with matter, for the relaxation and the advection
     // (the complement of a cell next to vacuum, which NSquant leaves alone);
     // every cell's result depends on that cell alone, not on the order
-    append_block(active, nactive, vac ? ~(int)i : (int)i, in && !(a.e <= 0.));
+    append_block(active, nactive, vac ? ~(int)i : (int)i, in && !second && !(a.e <= 0.));
   }
-  if (!in) return;
+  if (!in || (second && (a.e <= 0. || vac))) return;
+  // D from Qh, or C from Q (only where NSquant reaches it), both at tau
   {
-    q_over(qh, tau, q);
-    Prim d;
-    transform_pv<EK>(E, q, d, c2p_guess(E, i));
-    const double ut = 1.0 / sqrt(1.0 - d.vx * d.vx - d.vy * d.vy - d.vz * d.vz);
-    pD[0 * N + i] = d.e;
-    pD[1 * N + i] = ut;
-    pD[2 * N + i] = ut * d.vx;
-    pD[3 * N + i] = ut * d.vy;
-    pD[4 * N + i] = ut * d.vz;
+    const double* src = second ? Q : Qh;
+    double qs[7];
+#pragma unroll
+    for (int k = 0; k < 7; k++) qs[k] = src[k * N + i];
+    q_over(qs, tau, q);
+    Prim P;
+    transform_pv<EK>(E, q, P, c2p_guess(E, i));
+    const double ut = 1.0 / sqrt(1.0 - P.vx * P.vx - P.vy * P.vy - P.vz * P.vz);
+    double* o = second ? pBC + 5 * N + i : pD + N + i;
+    o[0] = ut;
+    o[N] = ut * P.vx;
+    o[2 * N] = ut * P.vy;
+    o[3 * N] = ut * P.vz;
+    if (!second) pD[i] = P.e;
     if (VORT) {
       double T, mub, p;
-      eos_eval<EK>(E, d.e, d.nb, T, mub, p);
-      TD[i] = T;
+      eos_eval<EK>(E, P.e, P.nb, T, mub, p);
+      (second ? TC : TD)[i] = T;
     }
   }
-  if (a.e <= 0.) return;
-  {
+  if (!second) {
+    if (a.e <= 0.) return;
     double T, mub, mus, p;
     eos_eval<EK>(E, a.e, a.nb, T, mub, mus, p);
     // EoS::s at the same point (eos_s, muq = 0) from this lookup
@@ -705,38 +717,35 @@ __device__ __forceinline__ void d_visc_prims(const Geo& g, const EosDev& E, cons
     pTh[6 * N + i] = taupi;
     pTh[7 * N + i] = tauPi;
     pTh[8 * N + i] = 9. / 70. / p;  // eos_p at the same point is this p
+    return;
   }
-  if (vac) return;
   // B is the predictor's con2prim when the divisors agree bit for bit
   // (k_update<true> stored it in pBC); otherwise computed here
-  const bool haveB = (clk[0] + dt) - dt == clk[0];
-  if (VORT && haveB) {
-    double T, mub, p;
-    eos_eval<EK>(E, pBC[4 * N + i], TB[i], T, mub, p);
-    TB[i] = T;  // (held B's nb until here)
-  }
-#pragma unroll 1
-  for (int w = haveB ? 1 : 0; w < 2; w++) {
-    const double* src = w == 0 ? Qprev : Q;
-    const double tt = w == 0 ? tau - dt : tau;
+  double eB, nbB;
+  if ((clk[0] + dt) - dt == clk[0]) {
+    if (!VORT) return;
+    eB = pBC[4 * N + i];
+    nbB = TB[i];  // held until here for this
+  } else {
     double qs[7];
 #pragma unroll
-    for (int k = 0; k < 7; k++) qs[k] = src[k * N + i];
-    q_over(qs, tt, q);
+    for (int k = 0; k < 7; k++) qs[k] = Qprev[k * N + i];
+    q_over(qs, tau - dt, q);
     Prim P;
     transform_pv<EK>(E, q, P, c2p_guess(E, i));
     const double ut = 1.0 / sqrt(1.0 - P.vx * P.vx - P.vy * P.vy - P.vz * P.vz);
-    const int o = w == 0 ? 0 : 5;
-    pBC[(o + 0) * N + i] = ut;
-    pBC[(o + 1) * N + i] = ut * P.vx;
-    pBC[(o + 2) * N + i] = ut * P.vy;
-    pBC[(o + 3) * N + i] = ut * P.vz;
-    if (w == 0) pBC[4 * N + i] = P.e;
-    if (VORT) {
-      double T, mub, p;
-      eos_eval<EK>(E, P.e, P.nb, T, mub, p);
-      (w == 0 ? TB : TC)[i] = T;
-    }
+    pBC[0 * N + i] = ut;
+    pBC[1 * N + i] = ut * P.vx;
+    pBC[2 * N + i] = ut * P.vy;
+    pBC[3 * N + i] = ut * P.vz;
+    pBC[4 * N + i] = P.e;
+    eB = P.e;
+    nbB = P.nb;
+  }
+  if (VORT) {
+    double T, mub, p;
+    eos_eval<EK>(E, eB, nbB, T, mub, p);
+    TB[i] = T;
   }
 }
 template <int EK, bool VORT>
@@ -756,11 +765,12 @@ __global__ void __launch_bounds__(128, kPrimsMinBlocks) k_visc_prims(Geo g, EosD
                                                     double* __restrict__ TD,
                                                     double* __restrict__ TB,
                                                     double* __restrict__ TC) {
-  const int n = *nwet;
-  for (int b = blockIdx.x * blockDim.x; b < n; b += gridDim.x * blockDim.x) {
-    const int idx = b + threadIdx.x;
+  const int n = *nwet, half = blockDim.x >> 1;
+  const bool second = (int)threadIdx.x >= half;
+  for (int b = blockIdx.x * half; b < n; b += gridDim.x * half) {
+    const int idx = b + (second ? threadIdx.x - half : threadIdx.x);
     d_visc_prims<EK, VORT>(g, E, tr, Q, Qprev, Qh, m, pA, pD, pTh, pBC, clk, active, nactive, TD, TB,
-                           TC, idx < n ? wet[idx] : 0, idx < n);
+                           TC, idx < n ? wet[idx] : 0, idx < n, second);
   }
 }
 
@@ -1885,7 +1895,7 @@ static int launch_step_ek(const StepArgs& a, cudaStream_t s, LaunchMarker* mk) {
   const unsigned char* fact = lists ? a.f.fact : nullptr;
   const bool vort = a.vort && a.viscous;
   const unsigned wide = 128 / bs;
-  const unsigned nprims = std::min(nb, 148 * kPrimsMinBlocks * wide);
+  const unsigned nprims = std::min(2 * nb, 148 * kPrimsMinBlocks * wide);
   const unsigned ngh = nblk(ghost_shell(g).n, bs);
   int launches = 0;
   const Fields& F = a.f;
@@ -2093,14 +2103,17 @@ template <int EK>
 __global__ void __launch_bounds__(128, kPrimsMinBlocks) kb_visc_prims(const StepDev* __restrict__ evs,
                                                      const BItem* __restrict__ items) {
   VH_ITEM
-  const int n = A.f.fcount[6];
-  const long long first = blk * blockDim.x, idx = first + threadIdx.x;
+  // a work item's 128 cells: two blocks (grid.y) of two threads a cell
+  const int n = A.f.fcount[6], half = blockDim.x >> 1;
+  const bool second = (int)threadIdx.x >= half;
+  const long long first = (2 * blk + blockIdx.y) * half;
+  const long long idx = first + (second ? threadIdx.x - half : threadIdx.x);
   if (first >= n) return;
   const EosDev E = A.eos;
   const TrDev tr = A.tr;
   d_visc_prims<EK, false>(g, E, tr, A.f.Q, A.f.Qprev, A.f.Qh, A.f.m2, A.f.pA, A.f.pD, A.f.pTh,
                    A.f.pBC, A.clk, A.f.active, A.f.nactive, nullptr,
-                          nullptr, nullptr, idx < n ? A.f.wet[idx] : 0, idx < n);
+                          nullptr, nullptr, idx < n ? A.f.wet[idx] : 0, idx < n, second);
 }
 
 __global__ void __launch_bounds__(kRelaxBlock, kRelaxMinBlocks) kb_is_relax(
@@ -2159,7 +2172,7 @@ static int launch_step_batched_ek(bool viscous, const StepDev* evs, int nev, con
     launches++;
   } else {
     kb_ghost<true, false><<<nb, kBatchBlock, 0, s>>>(evs, items);
-    kb_visc_prims<EK><<<nb, kBatchBlock, 0, s>>>(evs, items);
+    kb_visc_prims<EK><<<dim3(nb, 2), kBatchBlock, 0, s>>>(evs, items);
     kb_is_relax<<<nb, kRelaxBlock, kRelaxSmem, s>>>(evs, items);
     kb_is_advect<<<nb, kBatchBlock, 0, s>>>(evs, items);
     kb_visc_update<<<nb, kBatchBlock, 0, s>>>(evs, items);
