@@ -713,7 +713,7 @@ vh_status vh_transport_eval(vh_ctx *ctx, const double *in_dev, long n,
  * time at the start of the step; the caller advances it by dt.
  * All scratch lives in one static device array sized for at most
  * VH_NOALLOC_MAX_CELLS cells and VH_NOALLOC_MAX_DIM cells per dimension
- * (about 21 MB held on every GPU that loads the library until exit); larger
+ * (about 23 MB held on every GPU that loads the library until exit); larger
  * grids are rejected with VH_ERR_ARG.  Nothing is allocated: no cudaMalloc,
  * cudaFree, host malloc or library allocator is called.  The array is a
  * module variable: the CUDA runtime maps it (and loads the step kernels)

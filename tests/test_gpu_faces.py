@@ -163,6 +163,27 @@ def test_listed_faces_equal_oracle(nx, ny, nz, nb):
     h.close()
 
 
+# the ideal update runs on a list above 888 blocks of 128 cells: sizes on both
+# sides of the line, the list's blocks of 512 with and without a remainder,
+# and the temperatures that the vorticity takes from it
+@pytest.mark.parametrize("nx,ny,nz", [(48, 48, 49), (49, 49, 48), (64, 64, 28), (337, 339, 1)])
+def test_listed_updates_equal_oracle(nx, ny, nz):
+    test_listed_faces_equal_oracle(nx, ny, nz, 0.0)
+
+
+def test_listed_update_with_vorticity_equals_oracle():
+    s = W.glauber3d_setup(nx=49, ny=49, nz=48, xmax=14.0, etamax=7.0, b=9.0, nb_peak=0.3)
+    h, o = capi.GpuHydro(s), P.OracleRun(s, vorticity=True)
+    h.enable_vorticity()
+    for _ in range(2):
+        h.step(1)
+        assert o.step(1) == 0
+        assert np.array_equal(h.get_dbeta(), o.dbeta, equal_nan=True)
+    bad = compare_states(gpu_state_as_oracle(h.get_state()), o.get_state())
+    assert not bad, bad
+    h.close()
+
+
 @pytest.mark.parametrize("form", ["ordinary", "tiny", "mixed", "zero", "no_shear", "bump", "large_dt"])
 def test_relaxation_ranges_equal_oracle(form):
     """Shear and bulk stresses inside and outside the ranges in which the

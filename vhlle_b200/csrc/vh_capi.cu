@@ -117,22 +117,13 @@ static vh_status dgrow(vh_ctx* c, T** p, size_t* cap, size_t need) {
 // cell 2 into 1 and 0, then cell n-3 into n-2 and n-1, each index clamped
 // into [0, n-1] (src/fld.cpp:211-273).  Simulating that sequence gives, for
 // every index, the original cell its final value comes from.
-static void ghost_map(int n, int* src, unsigned char* dst) {
-  for (int i = 0; i < n; i++) {
-    src[i] = i;
-    dst[i] = 0;
-  }
+static void ghost_map(int n, int* src) {
+  for (int i = 0; i < n; i++) src[i] = i;
   auto cl = [n](int i) { return std::min(std::max(i, 0), n - 1); };
   int s = cl(2);
-  for (int d : {cl(1), cl(0)}) {
-    src[d] = src[s];
-    dst[d] = 1;
-  }
+  for (int d : {cl(1), cl(0)}) src[d] = src[s];
   s = cl(n - 3);
-  for (int d : {cl(n - 2), cl(n - 1)}) {
-    src[d] = src[s];
-    dst[d] = 1;
-  }
+  for (int d : {cl(n - 2), cl(n - 1)}) src[d] = src[s];
 }
 
 // Chooses how the device searches a table axis: the index guess of a log
@@ -633,7 +624,8 @@ vh_status vh_create(const vh_grid* grid, const vh_eos* eos, const vh_trcoeff* tr
   ALLOC(f.Fz, 7 * N);
   ALLOC(f.fact, N);
   ALLOC(f.flist, 3 * N);
-  ALLOC(f.fcount, 7);
+  ALLOC(f.fcount, 9);
+  ALLOC(f.ulist, N);
   if (c->viscous) {
     ALLOC(f.flux, 4 * N);
     ALLOC(f.pA, 8 * N);
@@ -653,15 +645,12 @@ vh_status vh_create(const vh_grid* grid, const vh_eos* eos, const vh_trcoeff* tr
   ALLOC(c->tot_out, vh::kTotals);
   const int ng = g.nx + g.ny + g.nz;
   ALLOC(f.gsrc, ng);
-  ALLOC(f.gdst, ng);
   ALLOC(f.err, 1);
   std::vector<int> hsrc(ng);
-  std::vector<unsigned char> hdst(ng);
-  ghost_map(g.nx, hsrc.data(), hdst.data());
-  ghost_map(g.ny, hsrc.data() + g.nx, hdst.data() + g.nx);
-  ghost_map(g.nz, hsrc.data() + g.nx + g.ny, hdst.data() + g.nx + g.ny);
+  ghost_map(g.nx, hsrc.data());
+  ghost_map(g.ny, hsrc.data() + g.nx);
+  ghost_map(g.nz, hsrc.data() + g.nx + g.ny);
   if ((e = cudaMemcpy(f.gsrc, hsrc.data(), ng * sizeof(int), cudaMemcpyHostToDevice)) ||
-      (e = cudaMemcpy(f.gdst, hdst.data(), ng, cudaMemcpyHostToDevice)) ||
       (e = cudaMemset(f.err, 0, sizeof(unsigned))) ||
       (e = cudaMemcpy(c->clk, std::vector<double>{tau0, dt}.data(), 2 * sizeof(double),
                       cudaMemcpyHostToDevice))) {
@@ -1341,11 +1330,11 @@ vh_status vh_sync(vh_ctx* ctx) {
 
 vh_status vh_launches_per_step(vh_ctx* ctx, int* n) {
   if (!ctx || !n) return VH_ERR_ARG;
-  // update_m, 2 x (face list, faces, update), 2 ghost, the viscous four
-  // (prims, relaxation, advection, update) and the five of the
-  // vorticity, the MLP guess, the clock
-  int k = 1 + 2 * (vh::face_lists(ctx->g, 128) ? 3 : 2) + 1 + (ctx->viscous ? 4 : 0) + 1 +
-          (ctx->viscous && ctx->vort_on ? 5 : 0) + (ctx->mlp ? 1 : 0) + 1;
+  // update_m, 2 x (face list, faces, update), a ghost copy; the viscous four
+  // (prims, relaxation, advection, update) and their ghost copy, the five of
+  // the vorticity; the MLP guess
+  int k = 1 + 2 * (vh::face_lists(ctx->g, 128) ? 3 : 2) + 1 + (ctx->viscous ? 5 : 0) +
+          (ctx->viscous && ctx->vort_on ? 5 : 0) + (ctx->mlp ? 1 : 0);
   *n = k;
   return VH_OK;
 }

@@ -12,7 +12,7 @@
 // or host allocation.
 //
 // Limits and sharing: the scratch array is sized for VH_NOALLOC_MAX_CELLS
-// cells (about 21 MB, held on every GPU that loads this library until the
+// cells (about 23 MB, held on every GPU that loads this library until the
 // process exits), and every call on a device uses the same array.  Calls
 // whose work overlaps on one GPU (concurrent streams or threads) race on it
 // and must be serialised by the caller.  The array keeps the previous call's
@@ -31,11 +31,11 @@ namespace {
 
 constexpr long long kMaxCells = VH_NOALLOC_MAX_CELLS;
 constexpr int kMaxDim = VH_NOALLOC_MAX_DIM;
-constexpr long long kDoublesPerCell = 85;  // m2 3, Fx/Fy/Fz 21, flux 4, pA 8, pD 5,
+constexpr long long kDoublesPerCell = 86;  // m2 3, Fx/Fy/Fz 21, flux 4, pA 8, pD 5,
                                            // pTh 9, pBC 9, pi0/piH0 20, Pi0/PiH0 2,
-                                           // the cell lists (ints) 2, the face
+                                           // the cell lists (ints) 3, the face
                                            // lists and flags 2
-constexpr size_t kHeaderBytes = 256 + 3 * kMaxDim * sizeof(int) + 3 * kMaxDim;  // err, maps
+constexpr size_t kHeaderBytes = 256 + 3 * kMaxDim * sizeof(int);  // err, map
 constexpr size_t kHeaderAligned = (kHeaderBytes + 255) / 256 * 256;
 constexpr size_t kScratchBytes = kHeaderAligned + (size_t)kDoublesPerCell * kMaxCells * sizeof(double);
 
@@ -85,24 +85,15 @@ vh_status cfail(cudaError_t e, const char* where) {
 }
 
 // Same copy sequence as the context path (src/fld.cpp:211-273).
-void ghost_map_fixed(int n, int* src, unsigned char* dst) {
-  for (int i = 0; i < n; i++) {
-    src[i] = i;
-    dst[i] = 0;
-  }
+void ghost_map_fixed(int n, int* src) {
+  for (int i = 0; i < n; i++) src[i] = i;
   auto cl = [n](int i) { return i < 0 ? 0 : (i > n - 1 ? n - 1 : i); };
   int s = cl(2);
   const int l[2] = {cl(1), cl(0)};
-  for (int d : l) {
-    src[d] = src[s];
-    dst[d] = 1;
-  }
+  for (int d : l) src[d] = src[s];
   s = cl(n - 3);
   const int r[2] = {cl(n - 2), cl(n - 1)};
-  for (int d : r) {
-    src[d] = src[s];
-    dst[d] = 1;
-  }
+  for (int d : r) src[d] = src[s];
 }
 
 }  // namespace
@@ -201,15 +192,13 @@ extern "C" vh_status vh_step_noalloc(const vh_grid* grid, const vh_eos* eos_dev,
                    tr->zetaSWidthT};
   a.viscous = tr->etaS0 > 0. || tr->zetaS0 > 0. || tr->etaSparam > 0 || tr->zetaSparam > 0;
 
-  // scratch layout: [err, clock, active and face counts | ghost src maps | ghost dst
-  // flags | pad][doubles...]
+  // scratch layout: [err, clock, counts | ghost map | pad][doubles...]
   vh::Fields& f = a.f;
   f.err = reinterpret_cast<unsigned*>(base);
   f.nactive = reinterpret_cast<int*>(base + 32);
   double* clk = reinterpret_cast<double*>(base + 16);
   a.clk = clk;
   f.gsrc = reinterpret_cast<int*>(base + 256);
-  f.gdst = base + 256 + 3 * kMaxDim * sizeof(int);
   double* d = reinterpret_cast<double*>(base + kHeaderAligned);
   f.m2 = d;
   d += 3 * N;
@@ -243,6 +232,7 @@ extern "C" vh_status vh_step_noalloc(const vh_grid* grid, const vh_eos* eos_dev,
   f.fact = reinterpret_cast<unsigned char*>(f.flist + 3 * N);
   f.fcount = reinterpret_cast<int*>(base + 64);
   f.wet = reinterpret_cast<int*>(d + 2 * N);
+  f.ulist = reinterpret_cast<int*>(d + 3 * N);
   f.Q = s->Q;
   f.Qh = s->Qh;
   f.Qprev = s->Qprev;
@@ -255,13 +245,11 @@ extern "C" vh_status vh_step_noalloc(const vh_grid* grid, const vh_eos* eos_dev,
 
   // ghost-cell maps from fixed-size host buffers (no host allocation)
   int hsrc[3 * kMaxDim];
-  unsigned char hdst[3 * kMaxDim];
-  ghost_map_fixed(grid->nx, hsrc, hdst);
-  ghost_map_fixed(grid->ny, hsrc + grid->nx, hdst + grid->nx);
-  ghost_map_fixed(grid->nz, hsrc + grid->nx + grid->ny, hdst + grid->nx + grid->ny);
+  ghost_map_fixed(grid->nx, hsrc);
+  ghost_map_fixed(grid->ny, hsrc + grid->nx);
+  ghost_map_fixed(grid->nz, hsrc + grid->nx + grid->ny);
   const int ng = grid->nx + grid->ny + grid->nz;
   if ((e = cudaMemcpyAsync(f.gsrc, hsrc, ng * sizeof(int), cudaMemcpyHostToDevice, st)) ||
-      (e = cudaMemcpyAsync(f.gdst, hdst, ng, cudaMemcpyHostToDevice, st)) ||
       (e = cudaMemsetAsync(f.err, 0, sizeof(unsigned), st)))
     return cfail(e, "scratch initialisation");
 

@@ -21,12 +21,13 @@
 
 namespace vh {
 
-// resident blocks of 128 threads per SM, from sweeps on the 101x101x51 event
-// (us per step at the stated counts): the face kernel 5 / 6 / 8 blocks 161 /
-// 160 / 153; the update 4 / 5 / 6 / 8: 100 / 94 / 97 / 93, where the 2+1D
-// grid of 101x101 takes 36 / 37 / 39 / 40 us a step and 201x201x101 462 / 401 /
-// 391 / 363; the viscous primitives 6 / 7 / 8: 30.8 / 31.5 / 33.1
-constexpr int kFaceMinBlocks = 8, kUpdateMinBlocks = 5, kPrimsMinBlocks = 6;
+// resident blocks of 128 threads per SM, from sweeps (us per step at the
+// stated counts): the face kernel 5 / 6 / 8 blocks 161 / 160 / 153 on the
+// 101x101x51 event; the update on a list 5 / 6 / 7 / 8: 64 / 54 / 56 / 58
+// there, 149 / 145 / 148 / 156 on 201x201x101, and on every cell of the 2+1D
+// grid of 101x101 4 / 5 / 6: 36 / 37 / 40; the viscous primitives 6 / 7 / 8:
+// 30.8 / 31.5 / 33.1
+constexpr int kFaceMinBlocks = 8, kUpdateMinBlocks = 6, kUpdateFewMinBlocks = 4, kPrimsMinBlocks = 6;
 
 // -------------------------------------------------------------- updateM
 // Fluid::updateM, src/fld.cpp:384-423 (both passes; out of place).
@@ -37,7 +38,7 @@ __device__ __forceinline__ void d_update_m(const Geo& g, const double* __restric
   const double tau = clk[0], dt = clk[1];  // the step's clock (device)
   const long long i = blk * blockDim.x + threadIdx.x;
   // the step's list counters, filled by later kernels
-  if (i < 7) fcount[i] = 0;
+  if (i < 9) fcount[i] = 0;
   if (i == 0 && nactive) *nactive = 0;
   if (i >= g.N) return;
   int ix, iy, iz;
@@ -79,6 +80,54 @@ __global__ void k_update_m(Geo g, const double* __restrict__ m, double* __restri
 }
 
 
+// ------------------------------------------------------- cells with matter
+// i joins the list: one atomic for the lanes that arrive together
+__device__ __forceinline__ void append(int* __restrict__ list, int* __restrict__ n, int i) {
+  const unsigned with = __activemask();
+  const int lane = threadIdx.x & 31, first = __ffs((int)with) - 1;
+  int base = 0;
+  if (lane == first) base = atomicAdd(n, __popc(with));
+  base = __shfl_sync(with, base, first);
+  list[base + __popc(with & ((1u << lane) - 1u))] = i;
+}
+// The same for the whole block (every thread calls it): one atomic, and the
+// block's entries in thread order, so that a list keeps the grid's runs (with
+// one atomic per warp the relaxation over the list took 112 instead of 101 us
+// at 101x101x51).
+__device__ __forceinline__ void append_block(int* __restrict__ list, int* __restrict__ n, int i,
+                                             bool with) {
+  __shared__ int cnt[4], first;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const unsigned bal = __ballot_sync(0xffffffffu, with);
+  __syncthreads();  // an earlier call's reads
+  if (lane == 0) cnt[warp] = __popc(bal);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int c = 0;
+    for (int w = 0; w < nw; w++) c += cnt[w];
+    first = c ? atomicAdd(n, c) : 0;
+  }
+  __syncthreads();
+  if (!with) return;
+  int at = first + __popc(bal & ((1u << lane) - 1u));
+  for (int w = 0; w < warp; w++) at += cnt[w];
+  list[at] = i;
+}
+// the cells the ghost copy writes (Fluid::correctImagCells: the two outermost
+// of every side)
+__device__ __forceinline__ bool is_ghost(const Geo& g, int ix, int iy, int iz) {
+  return ix < 2 || ix >= g.nx - 2 || iy < 2 || iy >= g.ny - 2 || iz < 2 || iz >= g.nz - 2;
+}
+// what the viscous stages read of an empty cell: e and v at the half step, e
+// at the full one
+__device__ __forceinline__ void empty_prims(double* __restrict__ pA, double* __restrict__ pD,
+                                            long long N, long long i) {
+  pA[i] = 0.;
+#pragma unroll
+  for (int k = 5; k < 8; k++) pA[k * N + i] = 0.;
+  pD[i] = 0.;
+}
+
 // ------------------------------------------------------------ face lists
 // The faces that can carry a flux, one list per direction (cell i for its
 // face on the + side).  Most of a grid is vacuum (80 to 92 % of the cells of
@@ -93,68 +142,107 @@ __global__ void k_update_m(Geo g, const double* __restrict__ m, double* __restri
 // for two vacuum edges, and for two unfilled cells unless it stops the run
 // for e > 1e10, which e <= Q_t / tau rules out.  Lists are in block order,
 // which varies; no face's flux depends on it.
-__device__ __forceinline__ void d_face_list(const Geo& g, const double* __restrict__ QT,
-                                            const double* __restrict__ m,
-                                            unsigned char* __restrict__ fact,
-                                            int* __restrict__ flist, int* __restrict__ fcount,
+//
+// With `rows` the same kernel settles the cells whose own Q_t and six
+// neighbours' are 0: nothing flows into them and they have no source, so their
+// update is a copy of the row (predictor) or nothing (corrector).  The others
+// are listed for the update, which so runs on full warps, and without the
+// vacuum's memory traffic at its low occupancy: lists, faces and update took
+// 247 us per step on the 101x101x51 event and take 226 (the update 95 and 54),
+// 891 and 804 on 201x201x101.  One cell per thread: with two or four (an
+// atomic per 256 or 512 cells) 2 to 15 % slower.
+__device__ __forceinline__ void d_face_list(const Geo& g, const Fields& f, bool predict,
+                                            bool rows, bool viscous, double* __restrict__ nbB,
                                             const double* __restrict__ clk, long long blk) {
-  __shared__ int wcnt[3][4], base[3];
+  __shared__ int wcnt[4][4], base[4];
+  const double* __restrict__ QT = predict ? f.Q : f.Qh;
+  const double* __restrict__ m = f.m2;
+  int* fcount = f.fcount + (predict ? 0 : 3);
+  int* ucount = f.fcount + (predict ? 7 : 8);
   const long long i = blk * blockDim.x + threadIdx.x;
   const long long N = g.N;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  unsigned act = 0;
+  unsigned act = 0;  // bit 3: the update list
   if (i < N) {
     int ix, iy, iz;
     coords(g, i, ix, iy, iz);
     const int cc[3] = {ix, iy, iz}, nn[3] = {g.nx, g.ny, g.nz};
     const long long ss[3] = {1, g.nx, (long long)g.nx * g.ny};
     const double x1 = QT[i], huge = 0.9e10 * clk[0];
-    double up[3];
-#pragma unroll
-    for (int d = 0; d < 3; d++) up[d] = cc[d] < nn[d] - 1 ? QT[i + ss[d]] : 0.;
+    double up[3], dn[3];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-      const double x2 = up[d];
-      // two empty cells have two empty edges (a slope takes the smaller side)
-      if (cc[d] >= nn[d] - 1 || (x1 == 0. && x2 == 0.)) continue;
-      const long long st = ss[d];
-      const double x0 = cc[d] > 0 ? QT[i - st] : x1, x3 = cc[d] < nn[d] - 2 ? QT[i + 2 * st] : x2;
-      const double el = x1 + minmod((x2 - x1) / 2., (x1 - x0) / 2.);
-      const double er = x2 - minmod((x3 - x2) / 2., (x2 - x1) / 2.);
-      if (el <= 0. && er <= 0.) continue;
-      if (m[d * N + i] < 1. && m[d * N + i + st] < 1. && el <= huge) continue;
-      act |= 1u << d;
+      up[d] = cc[d] < nn[d] - 1 ? QT[i + ss[d]] : 0.;
+      dn[d] = cc[d] > 0 ? QT[i - ss[d]] : 0.;
     }
-    fact[i] = (unsigned char)act;
-  }
-  unsigned bal[3];
+    const bool far = rows && x1 == 0. && up[0] == 0. && up[1] == 0. && up[2] == 0. && dn[0] == 0. &&
+                     dn[1] == 0. && dn[2] == 0. && QT[3 * N + i] == 0.;
+    if (far) {
+      const bool ghost = is_ghost(g, ix, iy, iz);
+      if (predict) {
 #pragma unroll
-  for (int d = 0; d < 3; d++) {
+        for (int k = 0; k < 7; k++) {
+          const double q = QT[k * N + i];
+          f.Qprev[k * N + i] = q;
+          f.Qh[k * N + i] = q;
+        }
+        // pB (the predictor's state at rest) is read of cells with matter at
+        // the half step: not of this one, unless the ghost copy puts it there
+        if (viscous && ghost) {
+          f.pBC[i] = 1.;
+#pragma unroll
+          for (int k = 1; k < 5; k++) f.pBC[k * N + i] = 0.;
+          if (nbB) nbB[i] = 0.;
+        }
+      } else if (viscous && !ghost) {
+        empty_prims(f.pA, f.pD, N, i);
+      }
+    } else {
+      act = rows ? 8u : 0u;
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        const double x2 = up[d];
+        // two empty cells have two empty edges (a slope takes the smaller side)
+        if (cc[d] >= nn[d] - 1 || (x1 == 0. && x2 == 0.)) continue;
+        const long long st = ss[d];
+        const double x0 = cc[d] > 0 ? dn[d] : x1, x3 = cc[d] < nn[d] - 2 ? QT[i + 2 * st] : x2;
+        const double el = x1 + minmod((x2 - x1) / 2., (x1 - x0) / 2.);
+        const double er = x2 - minmod((x3 - x2) / 2., (x2 - x1) / 2.);
+        if (el <= 0. && er <= 0.) continue;
+        if (m[d * N + i] < 1. && m[d * N + i + st] < 1. && el <= huge) continue;
+        act |= 1u << d;
+      }
+    }
+    f.fact[i] = (unsigned char)(act & 7u);
+  }
+  unsigned bal[4];
+#pragma unroll
+  for (int d = 0; d < 4; d++) {
     bal[d] = __ballot_sync(0xffffffffu, (act >> d) & 1u);
     if (lane == 0) wcnt[d][warp] = __popc(bal[d]);
   }
   __syncthreads();
-  if (threadIdx.x < 3) {
+  if (threadIdx.x < 4) {
     int n = 0;
     for (int w = 0; w < nw; w++) n += wcnt[threadIdx.x][w];
-    base[threadIdx.x] = n ? atomicAdd(fcount + threadIdx.x, n) : 0;
+    base[threadIdx.x] = n ? atomicAdd(threadIdx.x < 3 ? fcount + threadIdx.x : ucount, n) : 0;
   }
   __syncthreads();
 #pragma unroll
-  for (int d = 0; d < 3; d++) {
+  for (int d = 0; d < 4; d++) {
     if (!((act >> d) & 1u)) continue;
     int at = base[d] + __popc(bal[d] & ((1u << lane) - 1u));
     for (int w = 0; w < warp; w++) at += wcnt[d][w];
-    flist[d * N + at] = (int)i;
+    if (d < 3)
+      f.flist[d * N + at] = (int)i;
+    else
+      f.ulist[at] = (int)i;
   }
 }
-__global__ void __launch_bounds__(128) k_face_list(Geo g, const double* __restrict__ QT,
-                                                   const double* __restrict__ m,
-                                                   unsigned char* __restrict__ fact,
-                                                   int* __restrict__ flist,
-                                                   int* __restrict__ fcount,
+__global__ void __launch_bounds__(128) k_face_list(Geo g, Fields f, bool predict, bool rows,
+                                                   bool viscous, double* nbB,
                                                    const double* __restrict__ clk) {
-  d_face_list(g, QT, m, fact, flist, fcount, clk, blockIdx.x);
+  d_face_list(g, f, predict, rows, viscous, nbB, clk, blockIdx.x);
 }
 
 // ------------------------------------------------------------ face flux
@@ -278,54 +366,6 @@ __global__ void __launch_bounds__(128, kFaceMinBlocks) k_face(
 }
 
 
-// ------------------------------------------------------- cells with matter
-// i joins the list: one atomic for the lanes that arrive together
-__device__ __forceinline__ void append(int* __restrict__ list, int* __restrict__ n, int i) {
-  const unsigned with = __activemask();
-  const int lane = threadIdx.x & 31, first = __ffs((int)with) - 1;
-  int base = 0;
-  if (lane == first) base = atomicAdd(n, __popc(with));
-  base = __shfl_sync(with, base, first);
-  list[base + __popc(with & ((1u << lane) - 1u))] = i;
-}
-// The same for the whole block (every thread calls it): one atomic, and the
-// block's entries in thread order, so that a list keeps the grid's runs (with
-// one atomic per warp the relaxation over the list took 112 instead of 101 us
-// at 101x101x51).
-__device__ __forceinline__ void append_block(int* __restrict__ list, int* __restrict__ n, int i,
-                                             bool with) {
-  __shared__ int cnt[4], first;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  const unsigned bal = __ballot_sync(0xffffffffu, with);
-  __syncthreads();  // an earlier call's reads
-  if (lane == 0) cnt[warp] = __popc(bal);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int c = 0;
-    for (int w = 0; w < nw; w++) c += cnt[w];
-    first = c ? atomicAdd(n, c) : 0;
-  }
-  __syncthreads();
-  if (!with) return;
-  int at = first + __popc(bal & ((1u << lane) - 1u));
-  for (int w = 0; w < warp; w++) at += cnt[w];
-  list[at] = i;
-}
-// the cells the ghost copy writes (Fluid::correctImagCells: the two outermost
-// of every side)
-__device__ __forceinline__ bool is_ghost(const Geo& g, int ix, int iy, int iz) {
-  return ix < 2 || ix >= g.nx - 2 || iy < 2 || iy >= g.ny - 2 || iz < 2 || iz >= g.nz - 2;
-}
-// what the viscous stages read of an empty cell: e and v at the half step, e
-// at the full one
-__device__ __forceinline__ void empty_prims(double* __restrict__ pA, double* __restrict__ pD,
-                                            long long N, long long i) {
-  pA[i] = 0.;
-#pragma unroll
-  for (int k = 5; k < 8; k++) pA[k * N + i] = 0.;
-  pD[i] = 0.;
-}
-
 // --------------------------------------------------- ideal cell update
 // Gathers the six face fluxes and the Milne source (Hydro::source_step,
 // src/hdo.cpp:307-353), then Cell::updateQtoQhByFlux (predictor) or
@@ -341,11 +381,10 @@ __device__ __forceinline__ void d_update(const Geo& g, const EosDev& E, double* 
                                          double* __restrict__ pB, double* __restrict__ pA,
                                          double* __restrict__ nbB, double* __restrict__ pD,
                                          int* __restrict__ wet, int* __restrict__ nwet,
-                                         long long blk) {
+                                         long long i) {
   const double tau = clk[0], dt = clk[1];  // the step's clock (device)
-  const long long i = blk * blockDim.x + threadIdx.x;
   const long long N = g.N;
-  const bool in = i < N;
+  const bool in = i < N;  // (the whole block calls)
   int ix = 0, iy = 0, iz = 0;
   if (in) coords(g, i, ix, iy, iz);
   const bool ghost = is_ghost(g, ix, iy, iz);
@@ -468,22 +507,28 @@ __device__ __forceinline__ void d_update(const Geo& g, const EosDev& E, double* 
     }
   }
 }
-template <bool PRED, int EK>
-__global__ void __launch_bounds__(128, kUpdateMinBlocks) k_update(Geo g, EosDev E, double* __restrict__ Q,
-                                                double* __restrict__ Qh,
-                                                double* __restrict__ Qprev,
-                                                const double* __restrict__ Fx,
-                                                const double* __restrict__ Fy,
-                                                const double* __restrict__ Fz,
-                                                const unsigned char* __restrict__ fact,
-                                                const double* __restrict__ clk, unsigned* err,
-                                                double* __restrict__ pB, double* __restrict__ pA,
-                                                double* __restrict__ nbB, double* __restrict__ pD,
-                                                int* __restrict__ wet, int* __restrict__ nwet) {
-  d_update<PRED, EK>(g, E, Q, Qh, Qprev, Fx, Fy, Fz, fact, clk, err, pB, pA, nbB, pD, wet, nwet,
-                     blockIdx.x);
+// LIST: the cells d_face_list listed; else every cell
+template <bool PRED, int EK, bool LIST>
+__global__ void __launch_bounds__(128, LIST ? kUpdateMinBlocks : kUpdateFewMinBlocks)
+k_update(Geo g, EosDev E, double* __restrict__ Q, double* __restrict__ Qh,
+         double* __restrict__ Qprev, const double* __restrict__ Fx, const double* __restrict__ Fy,
+         const double* __restrict__ Fz, const unsigned char* __restrict__ fact,
+         const double* __restrict__ clk, unsigned* err, double* __restrict__ pB,
+         double* __restrict__ pA, double* __restrict__ nbB, double* __restrict__ pD,
+         int* __restrict__ wet, int* __restrict__ nwet, const int* __restrict__ ulist,
+         const int* __restrict__ ucount) {
+  if (!LIST) {
+    d_update<PRED, EK>(g, E, Q, Qh, Qprev, Fx, Fy, Fz, fact, clk, err, pB, pA, nbB, pD, wet, nwet,
+                       (long long)blockIdx.x * blockDim.x + threadIdx.x);
+    return;
+  }
+  const int n = *ucount;
+  for (int b = blockIdx.x * blockDim.x; b < n; b += gridDim.x * blockDim.x) {
+    const int idx = b + threadIdx.x;
+    d_update<PRED, EK>(g, E, Q, Qh, Qprev, Fx, Fy, Fz, fact, clk, err, pB, pA, nbB, pD, wet, nwet,
+                       idx < n ? ulist[idx] : g.N);
+  }
 }
-
 
 // ------------------------------------------------------------- ghosts
 // Fluid::correctImagCells (HALF: Q and Qh) and correctImagCellsFull (FULL:
@@ -1892,7 +1937,12 @@ static int launch_step_ek(const StepArgs& a, cudaStream_t s, LaunchMarker* mk) {
   const long long fblocks = face_blocks(g, bs), resident = face_resident(bs);
   const bool lists = face_lists(g, bs);
   const unsigned nface = (unsigned)std::min(fblocks, resident);
-  const unsigned char* fact = lists ? a.f.fact : nullptr;
+  const unsigned rset = 148 * kUpdateMinBlocks * (128u / bs);
+  // the update runs on a list where its blocks do not fit one resident set:
+  // 101x101x51, 4065 blocks of 888, 446 us a step with the list and 463
+  // without; 47x61x23, 516 blocks, 169 with and 161 without
+  const bool rows = lists && nb > rset;
+  const unsigned nupd = rows ? rset : nb;
   const bool vort = a.vort && a.viscous;
   const unsigned wide = 128 / bs;
   const unsigned nprims = std::min(2 * nb, 148 * kPrimsMinBlocks * wide);
@@ -1912,20 +1962,19 @@ static int launch_step_ek(const StepArgs& a, cudaStream_t s, LaunchMarker* mk) {
     const double* QQ = pred ? F.Q : F.Qh;
     int* fcount = lists ? F.fcount + 3 * pass : nullptr;
     if (lists) {
-      k_face_list<<<nb, bs, 0, s>>>(g, QQ, m, F.fact, F.flist, fcount, a.clk);
+      k_face_list<<<nb, bs, 0, s>>>(g, F, pred, rows, a.viscous, vort ? a.vort->TB : nullptr, a.clk);
       launches++;
     }
     k_face<EK><<<nface, bs, 0, s>>>(g, a.eos, pred, QQ, m, F.Fx, F.Fy, F.Fz,
                                     lists ? F.flist : nullptr, fcount, a.clk, F.err);
     done(KK_FACE);
-    if (pred)
-      k_update<true, EK><<<nb, bs, 0, s>>>(g, a.eos, F.Q, F.Qh, F.Qprev, F.Fx, F.Fy, F.Fz, fact, a.clk,
-                                           F.err, a.viscous ? F.pBC : nullptr, nullptr,
-                                           vort ? a.vort->TB : nullptr, nullptr, nullptr, nullptr);
-    else
-      k_update<false, EK><<<nb, bs, 0, s>>>(g, a.eos, F.Q, F.Qh, F.Qprev, F.Fx, F.Fy, F.Fz, fact, a.clk,
-                                            F.err, nullptr, a.viscous ? F.pA : nullptr, nullptr, F.pD,
-                                            F.wet, F.fcount + 6);
+    auto update = pred ? (rows ? k_update<true, EK, true> : k_update<true, EK, false>)
+                       : (rows ? k_update<false, EK, true> : k_update<false, EK, false>);
+    update<<<nupd, bs, 0, s>>>(g, a.eos, F.Q, F.Qh, F.Qprev, F.Fx, F.Fy, F.Fz, lists ? F.fact : nullptr,
+                               a.clk, F.err, pred && a.viscous ? F.pBC : nullptr,
+                               !pred && a.viscous ? F.pA : nullptr,
+                               pred && vort ? a.vort->TB : nullptr, F.pD, F.wet, F.fcount + 6,
+                               F.ulist, F.fcount + 7 + pass);
     done(KK_UPDATE);
   }
   if (!a.viscous) {
@@ -2027,12 +2076,10 @@ __global__ void k_clock_set(double* clk, double tau, double dt) {
   clk[0] = tau;
   clk[1] = dt;
 }
-// tau += dt (src/hdo.cpp:1095), the substep divide (dt / n) and restore
-// (dt * n) of the driver loop (src/main.cpp:411,415), in the host's order
+// the substep divide (dt / n) and restore (dt * n) of the driver loop
+// (src/main.cpp:411,415), in the host's order
 __global__ void k_clock_op(double* clk, int op, int n) {
-  if (op == 0)
-    clk[0] += clk[1];
-  else if (op == 1)
+  if (op == 1)
     clk[1] = clk[1] / n;
   else
     clk[1] = clk[1] * n;
@@ -2060,8 +2107,7 @@ __global__ void __launch_bounds__(128) kb_face_list(const StepDev* __restrict__ 
                                                     const BItem* __restrict__ items,
                                                     bool predict) {
   VH_ITEM
-  d_face_list(g, predict ? A.f.Q : A.f.Qh, A.f.m2, A.f.fact, A.f.flist,
-              A.f.fcount + (predict ? 0 : 3), A.clk, blk);
+  d_face_list(g, A.f, predict, true, A.viscous, nullptr, A.clk, blk);
 }
 
 // a work item of kBatchBlock cells stands for six blocks (grid.y) of its
@@ -2088,8 +2134,12 @@ __global__ void __launch_bounds__(128, kUpdateMinBlocks) kb_update(const StepDev
   const EosDev E = A.eos;
   double* pB = PRED && A.viscous ? A.f.pBC : nullptr;
   double* pA = !PRED && A.viscous ? A.f.pA : nullptr;
+  const int n = A.f.fcount[PRED ? 7 : 8];
+  const long long idx = blk * blockDim.x + threadIdx.x;
+  if (blk * blockDim.x >= n) return;
   d_update<PRED, EK>(g, E, A.f.Q, A.f.Qh, A.f.Qprev, A.f.Fx, A.f.Fy, A.f.Fz, A.f.fact, A.clk,
-                     A.f.err, pB, pA, nullptr, A.f.pD, A.f.wet, A.f.fcount + 6, blk);
+                     A.f.err, pB, pA, nullptr, A.f.pD, A.f.wet, A.f.fcount + 6,
+                     idx < n ? A.f.ulist[idx] : g.N);
 }
 
 template <bool HALF, bool FULL>
@@ -2143,9 +2193,7 @@ __global__ void kb_clock_op(const StepDev* __restrict__ evs, int nev, int op,
   if (e >= nev) return;
   double* clk = evs[e].clk;
   const int n = ns ? ns[e] : 1;
-  if (op == 0)
-    clk[0] += clk[1];
-  else if (op == 1)
+  if (op == 1)
     clk[1] = clk[1] / n;
   else
     clk[1] = clk[1] * n;

@@ -91,8 +91,9 @@ struct Fields {
                                  // fact has the direction's bit
   unsigned char *fact;           // [N] bit d: the +d face may carry a flux
   int *flist;                    // [3][N] the cells whose +d face may
-  int *fcount;                   // [7] their numbers: predictor, corrector;
-                                 // the number of wet cells
+  int *fcount;                   // [9] their numbers: predictor, corrector;
+                                 // of wet cells; of ulist, per pass
+  int *ulist;                    // [N] the cells the ideal update works on
   int *wet;                      // [N] cells with Qh_t > 0 (viscous steps)
   double *flux;                  // [4][N] viscous flux accumulator
   double *pA;                    // [8][N] prims of Qh at tau_{n+1} - dt/2
@@ -105,7 +106,6 @@ struct Fields {
                                  // relaxation, those next to vacuum
                                  // complemented, and their count ([1])
   int *gsrc;                     // [nx+ny+nz] ghost-cell source map
-  unsigned char *gdst;           // [nx+ny+nz] ghost-cell destination flags
   unsigned *err;                 // device error word
 };
 
@@ -161,7 +161,7 @@ int step_ek(const EosDev& E);
 int launch_step_batched(int ek, bool viscous, const StepDev* evs, int nev, const BItem* items,
                         int nitems, cudaStream_t s);
 // launch_clock_op on the clocks of nev events at once (ns: device, each
-// event's n for ops 1 and 2)
+// event's n)
 void launch_clock_op_batched(const StepDev* evs, int nev, int op, const int* ns, cudaStream_t s);
 
 // ISformal's dbeta for every cell (after k_visc_prims, before the viscous
@@ -194,7 +194,7 @@ bool face_lists(const Geo& g, int bs);
 // Leaves the updated fill fractions in f.m2 (the caller swaps m and m2).
 int launch_step(const StepArgs& a, cudaStream_t s, LaunchMarker* mk = nullptr);
 void launch_clock_set(double* clk, double tau, double dt, cudaStream_t s);
-// op 0: tau += dt; 1: dt = dt / n; 2: dt = dt * n
+// op 1: dt = dt / n; 2: dt = dt * n
 void launch_clock_op(double* clk, int op, int n, cudaStream_t s);
 // gathers ncomp planes of the x2 resized grid from src into dst
 void launch_resize_gather(const Geo& g, const double* src, double* dst, int ncomp,

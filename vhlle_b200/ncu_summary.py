@@ -9,7 +9,7 @@ table of the launch list.
 CSV is ncu's `--csv --log-file` output of a capture of bench.py's timed
 region (`--nvtx --nvtx-include timed/`); GRID is the workload's nx,ny,nz.
 Launches are grouped under the kernel names bench.py's per-kernel profile
-uses (k_relax_list counted with k_is_relax, the
+uses (k_face_list counted with k_face, the
 freeze-out kernels as "surface"), each kind's values in launch order.
 """
 from __future__ import annotations
@@ -33,8 +33,8 @@ def kind_of(name: str) -> str:
     base = re.sub(r"^void\s+", "", name).split("(")[0]
     base = base.replace("vh::", "")
     short = base.split("<")[0]
-    if short == "k_relax_list":
-        return "k_is_relax"
+    if short == "k_face_list":
+        return "k_face"
     if any(short.startswith(p) for p in SURFACE):
         return "surface"
     return short
@@ -62,10 +62,10 @@ def read_rows(path: str):
     return [(lid, k, m) for lid, (k, m) in launches.items()]
 
 
-def per_launch(rows, value, merge=("k_is_relax",)):
+def per_launch(rows, value, merge=("k_face",)):
     """{kind: [value per launch]}; for the kinds in `merge`, consecutive
-    launches of that kind with no other kernel between them (k_relax_list
-    then k_is_relax) count as one launch."""
+    launches of that kind with no other kernel between them (k_face_list
+    then k_face) count as one launch."""
     out = collections.OrderedDict()
     prev = None
     for _, k, m in rows:
