@@ -46,16 +46,22 @@ __device__ __forceinline__ void d_update_m(const Geo& g, const double* __restric
   const long long N = g.N;
   double d0 = 0., d1 = 0., d2 = 0.;
   if (maxM(m, N, i) < 1.) {
-    if (m[cidx(g, ix + 1, iy, iz)] >= 1. || m[cidx(g, ix - 1, iy, iz)] >= 1.) d0 = dt / g.dx;
-    if (m[N + cidx(g, ix, iy + 1, iz)] >= 1. || m[N + cidx(g, ix, iy - 1, iz)] >= 1.)
-      d1 = dt / g.dy;
-    if (m[2 * N + cidx(g, ix, iy, iz + 1)] >= 1. || m[2 * N + cidx(g, ix, iy, iz - 1)] >= 1.)
-      d2 = dt / g.dz / tau;
+    // the loads of a stage together: as short-circuits they were a chain (us
+    // per step, 101x101x51 18.4 and 15.8, 201x201x101 91.8 and 66.2)
+    auto full = [&](int dx, int dy, int dz, int k) {
+      return m[k * N + cidx(g, ix + dx, iy + dy, iz + dz)] >= 1.;
+    };
+    const bool fx = full(1, 0, 0, 0) | full(-1, 0, 0, 0);
+    const bool fy = full(0, 1, 0, 1) | full(0, -1, 0, 1);
+    const bool fz = full(0, 0, 1, 2) | full(0, 0, -1, 2);
+    if (fx) d0 = dt / g.dx;
+    if (fy) d1 = dt / g.dy;
+    if (fz) d2 = dt / g.dz / tau;
     if (d0 == 0. && d1 == 0.) {
-      if (maxM(m, N, cidx(g, ix + 1, iy + 1, iz)) >= 1. ||
-          maxM(m, N, cidx(g, ix + 1, iy - 1, iz)) >= 1. ||
-          maxM(m, N, cidx(g, ix - 1, iy + 1, iz)) >= 1. ||
-          maxM(m, N, cidx(g, ix - 1, iy - 1, iz)) >= 1.) {
+      auto most = [&](int dx, int dy) {
+        return maxM(m, N, cidx(g, ix + dx, iy + dy, iz)) >= 1.;
+      };
+      if (most(1, 1) | most(1, -1) | most(-1, 1) | most(-1, -1)) {
         d0 = 0.707 * dt / g.dx;
         d1 = 0.707 * dt / g.dy;
       }
@@ -1819,13 +1825,15 @@ __device__ __forceinline__ void d_visc_update(const Geo& g, const double* __rest
   const int cc[3] = {ix, iy, iz};
   const int nn[3] = {g.nx, g.ny, g.nz};
   if (empty) {
+    // (the nine loads together, as in d_update_m: 201x201x101 133 -> 123 us)
     bool any = false;
 #pragma unroll
     for (int d = 0; d < 3; d++) {
       const double* md = m + d * N;
+      const bool in0 = cc[d] > 0, in1 = cc[d] < nn[d] - 1;
+      const double m0 = md[in0 ? i - st[d] : i], m1 = md[in1 ? i + st[d] : i];
       const bool own = !(md[i] < 1.);
-      any |= cc[d] > 0 && (own || !(md[i - st[d]] < 1.));
-      any |= cc[d] < nn[d] - 1 && (own || !(md[i + st[d]] < 1.));
+      any |= (in0 & (own | !(m0 < 1.))) | (in1 & (own | !(m1 < 1.)));
     }
     if (!any) return;
   }
