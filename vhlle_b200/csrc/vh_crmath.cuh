@@ -364,15 +364,21 @@ VH_CRM double exp_cr(double x) {
   return exp_long(x);
 }
 
+// x^y for y not 0 or 2, |y| <= 8, with L = pow_base(x): the log of x once
+// for all its powers (NaN where the short form does not apply)
+VH_CRM dd pow_base(double x) {
+  if (x >= 0x1p-1022 && x <= 0x1.fffffffffffffp1023 && x != 1.) return log_short(x);
+  return {(double)NAN, 0.};
+}
+VH_CRM double pow_of(double x, dd L, double y) {
+  const dd p = two_prod(y, L.hi);
+  const dd t = fast_two_sum(p.hi, fma(y, L.lo, p.lo));
+  double r;
+  if (fabs(t.hi) <= 700. && exp_try(t, &r)) return r;
+  return pow_long(x, y);
+}
 VH_CRM double pow_cr(double x, double y) {
-  if (x >= 0x1p-1022 && x <= 0x1.fffffffffffffp1023 && x != 1. && fabs(y) <= 8. && y != 2. &&
-      y != 0.) {
-    const dd L = log_short(x);
-    const dd p = two_prod(y, L.hi);
-    const dd t = fast_two_sum(p.hi, fma(y, L.lo, p.lo));
-    double r;
-    if (fabs(t.hi) <= 700. && exp_try(t, &r)) return r;
-  }
+  if (fabs(y) <= 8. && y != 2. && y != 0.) return pow_of(x, pow_base(x), y);
   return pow_long(x, y);
 }
 

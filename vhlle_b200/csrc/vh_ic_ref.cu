@@ -10,6 +10,7 @@
 // step) of every cell once per normalisation pass and once more at the end.
 // Those run here:
 //
+//   k_gliss_tr    the sources' Gaussians (trSmear) on their +-ns stencils
 //   k_gliss_rho   one thread per transverse cell and 8 eta cells: the
 //                 sources in file order (staged through shared memory),
 //                 each within its +-ns stencil adding the reference's
@@ -61,27 +62,29 @@ constexpr int kNormMaxIt = 10000;  // likewise its normalisation loops
 // exponentials, and the Newton loop around it would otherwise be tens of KB
 // of straight-line code per kernel
 __device__ __noinline__ double pw(double x, double y) { return crm::pow_cr(x, y); }
+__device__ __noinline__ double pwl(double x, crm::dd L, double y) { return crm::pow_of(x, L, y); }
 __device__ __noinline__ double ex(double x) { return crm::exp_cr(x); }
 
-// s95p::s95p_s, src/s95p.cpp:14-32 (the s95p-PCE fit of s(e))
-__device__ double s95p_s(double e) {
+// s95p::s95p_s, src/s95p.cpp:14-32 (the s95p-PCE fit of s(e)), L =
+// pow_base(e).  The FP64 pipe bounds it, and a warp's lanes take several of
+// the fit's ranges: its powers share the log of e, and the ranges their first
+// power (k_ic_terms on 520,251 cells 259 -> 163 us).
+__device__ double s95p_s(double e, crm::dd L) {
+  const bool low = e < 1.9402832534193788, a = e < 0.1270769021427449, b = e < 0.4467079524674040;
+  const double y = a ? 1.16849 : b ? 1.15635 : low ? 1.16187 : 4.54886;
+  const double p0 = pwl(e, L, y);
   double val;
-  if (e < 0.1270769021427449)
-    val = 12.2304 * pw(e, 1.16849);
-  else if (e < 0.4467079524674040)
-    val = 11.9279 * pw(e, 1.15635);
-  else if (e < 1.9402832534193788)
-    val = 0.0580578 + 11.833 * pw(e, 1.16187);
-  else if (e < 3.7292474570977285)
-    val = 18.202 * e - 62.021814 - 4.85479 * ex(-2.72407e-11 * pw(e, 4.54886)) +
-          65.1272 * pw(e, -0.128012) * ex(-0.00369624 * pw(e, 1.18735)) -
-          4.75253 * pw(e, -1.18423);
-  else
-    val = 18.202 * e - 63.0218 - 4.85479 * ex(-2.72407e-11 * pw(e, 4.54886)) +
-          65.1272 * pw(e, -0.128012) * ex(-0.00369624 * pw(e, 1.18735));
+  if (low) {
+    val = (a ? 12.2304 : b ? 11.9279 : 11.833) * p0;
+    if (!b) val = 0.0580578 + val;
+  } else {
+    const bool mid = e < 3.7292474570977285;
+    val = 18.202 * e - (mid ? 62.021814 : 63.0218) - 4.85479 * ex(-2.72407e-11 * p0) +
+          65.1272 * pwl(e, L, -0.128012) * ex(-0.00369624 * pwl(e, L, 1.18735));
+    if (mid) val = val - 4.75253 * pwl(e, L, -1.18423);
+  }
   return pw(val, 3. / 4.);
 }
-
 // s95p::s95p_e, src/s95p.cpp:34-41; *bad gets bit 1 if kS95pMaxIt steps
 // did not converge (the reference would not return)
 __device__ double s95p_e(double s, unsigned* bad) {
@@ -89,7 +92,8 @@ __device__ double s95p_e(double s, unsigned* bad) {
   int it = 0;
   do {
     e0 = e;
-    e = e0 - (s95p_s(e0) - s) / (6.608681233 * pw(e0, -0.25));
+    const crm::dd L = crm::pow_base(e0);
+    e = e0 - (s95p_s(e0, L) - s) / (6.608681233 * pwl(e0, L, -0.25));
     if (++it > kS95pMaxIt) {
       atomicOr(bad, 1u);
       break;
@@ -153,12 +157,45 @@ struct GlissArgs {
   const double* tilt;   // [2][nz] (code > 0, else)
   const double* bg;     // [nev][2][nz] baryon Gaussian / (nsigma sqrt(2 pi))
   double *rho, *nrho;   // [N] grid order
+  int k0, k1;           // the launch's sources
+  int bw, bh;           // the columns a source reaches, as an array
+  double* tr;           // [k1 - k0][bh][bw] their Gaussians there
+  // a source's first column and row of that array (the whole side where it
+  // reaches further)
+  __device__ int x0(int ixc) const { return ns <= (bw - 1) / 2 ? ixc - ns : 0; }
+  __device__ int y0(int iyc) const { return ns <= (bh - 1) / 2 ? iyc - ns : 0; }
 };
 
-// IcGlissando::makeSmoothTable over every event, src/icGlissando.cpp:187-228
+// The sources' Gaussians, a thread per source and column: in k_gliss_rho each
+// of a column's threads took the exponential of every source in turn.
+__global__ void __launch_bounds__(kTpb) k_gliss_tr(GlissArgs a) {
+  const ColGeo& g = a.g;
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int box = a.bw * a.bh;
+  if (t >= (long long)box * (a.k1 - a.k0)) return;
+  const int k = a.k0 + (int)(t / box), b = (int)(t % box);
+  const double norm_gauss = 2.0 * kCPi * a.Rg * a.Rg;
+  const double inv_norm = 1.0 / norm_gauss;
+  const double two_rg2 = 2. * a.Rg * a.Rg;
+  const double xs = a.sx[k], ys = a.sy[k];
+  const int ix = a.x0((int)((xs - g.xmin) / g.dx)) + b % a.bw;
+  const int iy = a.y0((int)((ys - g.ymin) / g.dy)) + b / a.bw;
+  const double xdiff = xs - (g.xmin + ix * g.dx), ydiff = ys - (g.ymin + iy * g.dy);
+  double tr = inv_norm * crm::exp_cr(-xdiff * xdiff / two_rg2 - ydiff * ydiff / two_rg2);
+  if (tr != tr || fabs(tr) > DBL_MAX) tr = 0.0;
+  a.tr[t] = tr;
+}
+
+// IcGlissando::makeSmoothTable over every event, src/icGlissando.cpp:187-228.
+// A source reaches the cells within 3 Rg of its own, about a tenth of the rows:
+// a block finds the sources' cells once and keeps, in file order, those that
+// reach its rows.  A column near the middle is a chain of several hundred
+// sources, which a warp mostly waits for: with the exponentials in the chain
+// and every source tested by every cell it took 974 us (101x101x51, 2403
+// sources), with the test once per block 631, with the exponentials apart 405,
+// with four sources' loads at a time about 300.
 __global__ void __launch_bounds__(kTpb) k_gliss_rho(GlissArgs a) {
-  __shared__ double shx[kTpb], shy[kTpb];
-  __shared__ int shc[kTpb], she[kTpb];
+  __shared__ int shk[kTpb], shc[kTpb], she[kTpb], shi[kTpb], shj[kTpb], wcnt[kTpb / 32];
   const ColGeo& g = a.g;
   const int ncol = g.nx * g.ny;
   const int nch = (g.nz + kKz - 1) / kKz;
@@ -169,43 +206,76 @@ __global__ void __launch_bounds__(kTpb) k_gliss_rho(GlissArgs a) {
   const bool open = in && ix > 0 && iy > 0;  // the loop's ix > 0 && iy > 0
   double r[kKz], nr[kKz];
 #pragma unroll
-  for (int k = 0; k < kKz; k++) r[k] = nr[k] = 0.0;
-  const double norm_gauss = 2.0 * kCPi * a.Rg * a.Rg;
-  const double inv_norm = 1.0 / norm_gauss;
-  const double two_rg2 = 2. * a.Rg * a.Rg;
-  const double xc = g.xmin + ix * g.dx, yc = g.ymin + iy * g.dy;
-  for (int base = 0; base < a.nsrc; base += kTpb) {
-    __syncthreads();
+  for (int k = 0; k < kKz; k++) {
+    const int iz = ch * kKz + k;
+    const bool more = a.k0 > 0 && in && iz < g.nz;  // after an earlier launch's
+    r[k] = more ? a.rho[col + (long long)ncol * iz] : 0.0;
+    nr[k] = more ? a.nrho[col + (long long)ncol * iz] : 0.0;
+  }
+  // the rows of the block's columns (all, where they run into the next chunk)
+  const long long t0 = (long long)blockIdx.x * blockDim.x, t1 = t0 + blockDim.x - 1;
+  const bool one = t0 / ncol == t1 / ncol;
+  const int row0 = one ? (int)(t0 % ncol) / g.nx : 0;
+  const int row1 = one ? (int)(t1 % ncol) / g.nx : g.ny - 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int base = a.k0; base < a.k1; base += kTpb) {
     const int k = base + threadIdx.x;
-    if (k < a.nsrc) {
-      shx[threadIdx.x] = a.sx[k];
-      shy[threadIdx.x] = a.sy[k];
-      shc[threadIdx.x] = a.sc[k];
-      she[threadIdx.x] = a.sev[k];
+    int iyc = 0;
+    bool near = k < a.k1;
+    if (near) {
+      iyc = (int)((a.sy[k] - g.ymin) / g.dy);
+      near = row1 >= iyc - a.ns && row0 <= iyc + a.ns;
+    }
+    const unsigned bal = __ballot_sync(0xffffffffu, near);
+    __syncthreads();  // the last sources are added
+    if (lane == 0) wcnt[warp] = __popc(bal);
+    __syncthreads();
+    int at = 0, n = 0;
+#pragma unroll
+    for (int w = 0; w < kTpb / 32; w++) {
+      if (w < warp) at += wcnt[w];
+      n += wcnt[w];
+    }
+    at += __popc(bal & ((1u << lane) - 1u));
+    if (near) {
+      shk[at] = k - a.k0;
+      shi[at] = (int)((a.sx[k] - g.xmin) / g.dx);
+      shj[at] = iyc;
+      shc[at] = a.sc[k];
+      she[at] = a.sev[k];
     }
     __syncthreads();
     if (!open) continue;
-    const int n = min(kTpb, a.nsrc - base);
-    for (int j = 0; j < n; j++) {
-      const double xs = shx[j], ys = shy[j];
-      const int ixc = (int)((xs - g.xmin) / g.dx);
-      const int iyc = (int)((ys - g.ymin) / g.dy);
-      if (ix < ixc - a.ns || ix > ixc + a.ns || iy < iyc - a.ns || iy > iyc + a.ns) continue;
-      const double xdiff = xs - xc, ydiff = ys - yc;
-      double tr = inv_norm * crm::exp_cr(-xdiff * xdiff / two_rg2 - ydiff * ydiff / two_rg2);
-      if (tr != tr || fabs(tr) > DBL_MAX) tr = 0.0;
-      const int c = shc[j], ev = she[j];
-      const double w = (1.0 - a.alphaMix) + abs(c) * a.alphaMix;
-      const int sg = c > 0 ? 0 : 1;
-      const double* fe = a.fEta + (long long)ev * g.nz;
-      const double* tl = a.tilt + sg * g.nz;
-      const double* bgp = a.bg + ((long long)ev * 2 + sg) * g.nz;
+    for (int j0 = 0; j0 < n; j0 += 4) {
+      double tr[4];
+      bool reach[4];
 #pragma unroll
-      for (int kz = 0; kz < kKz; kz++) {
-        const int iz = ch * kKz + kz;
-        if (iz < g.nz) {
-          r[kz] += tr * fe[iz] * tl[iz] * w;
-          if (a.baryon) nr[kz] += tr * w * bgp[iz];
+      for (int q = 0; q < 4; q++) {  // the loads of four sources together
+        const int j = j0 + q;
+        reach[q] = false;
+        if (j < n) {
+          const int bx = ix - shi[j], by = iy - shj[j];
+          reach[q] = bx >= -a.ns && bx <= a.ns && by >= -a.ns && by <= a.ns;
+        }
+        if (reach[q])
+          tr[q] = a.tr[((long long)shk[j] * a.bh + (iy - a.y0(shj[j]))) * a.bw + (ix - a.x0(shi[j]))];
+      }
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        if (!reach[q]) continue;
+        const int c = shc[j0 + q], ev = she[j0 + q];
+        const double w = (1.0 - a.alphaMix) + abs(c) * a.alphaMix;
+        const int sg = c > 0 ? 0 : 1;
+        const double* fe = a.fEta + (long long)ev * g.nz;
+        const double* tl = a.tilt + sg * g.nz;
+        const double* bgp = a.bg + ((long long)ev * 2 + sg) * g.nz;
+#pragma unroll
+        for (int kz = 0; kz < kKz; kz++) {
+          const int iz = ch * kKz + kz;
+          if (iz < g.nz) {
+            r[kz] += tr[q] * fe[iz] * tl[iz] * w;
+            if (a.baryon) nr[kz] += tr[q] * w * bgp[iz];
+          }
         }
       }
     }
@@ -344,8 +414,11 @@ __global__ void __launch_bounds__(kTpb) k_ic_terms(TermArgs a) {
 // (the 256 terms of a warp) with a tie, a negative or non-finite term, or
 // the step into the next binade is added term by term; over n terms of one
 // size that happens about ln n times for ties and log2 n times for binades.
-// One block, since each tile needs the sum before it; 520,251 terms took
-// 977 us as a chain of additions.
+// One block, since each tile needs the sum before it.  A warp whose terms are
+// all zeros skips the arithmetic, and a chain takes the non-zero terms only.
+// 520,251 terms take 148 us, and 977 as a chain of additions (181 with the
+// zeros treated as any term; 4 terms per thread and tile instead of 8 made a
+// call 15 % slower).
 constexpr int kSumThreads = 1024;
 constexpr int kSumPer = 8;                       // terms per thread and tile
 constexpr int kSumRun = 32 * kSumPer;            // a sub-tile
@@ -353,7 +426,7 @@ constexpr int kSumTile = kSumThreads * kSumPer;  // 32 sub-tiles
 
 __global__ void __launch_bounds__(kSumThreads) k_seq_sum(const double* __restrict__ t, long long n,
                                                          double* __restrict__ out) {
-  __shared__ double wsum[32];
+  __shared__ double wsum[32], chain[kSumRun];
   __shared__ int wbad[32];
   __shared__ double s_sh;
   __shared__ int pos_sh;
@@ -372,6 +445,10 @@ __global__ void __launch_bounds__(kSumThreads) k_seq_sum(const double* __restric
   for (long long tile = 0; tile < ntile; tile++) {
     double next[kSumPer];
     load(tile + 1, next);  // (zeros past the end)
+    bool with = false;
+#pragma unroll
+    for (int r = 0; r < kSumPer; r++) with |= v[r] != 0.0;
+    with = __any_sync(0xffffffffu, with);
     int pos = 0;           // the first sub-tile not added yet
     while (pos < 32) {
       // s in whole numbers of its last bit; s = 0 takes zero terms only
@@ -381,14 +458,16 @@ __global__ void __launch_bounds__(kSumThreads) k_seq_sum(const double* __restric
       const double u = fit ? crm::pow2i(ex - 1023 - 52) : 0.0;
       double sum = 0.0;
       bool bad = !fit && s != 0.0;
+      if (with) {  // (the warp's terms are not all zeros)
 #pragma unroll
-      for (int r = 0; r < kSumPer; r++) {
-        const double x = v[r] * scale, w = rint(x);
-        sum += w;
-        bad |= fit ? !(v[r] >= 0.0 && x < 0x1p51) || fabs(x - w) == 0.5 : v[r] != 0.0;
+        for (int r = 0; r < kSumPer; r++) {
+          const double x = v[r] * scale, w = rint(x);
+          sum += w;
+          bad |= fit ? !(v[r] >= 0.0 && x < 0x1p51) || fabs(x - w) == 0.5 : v[r] != 0.0;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
       }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
       const unsigned any = __ballot_sync(0xffffffffu, bad);
       if (lane == 0) {
         wsum[warp] = sum;
@@ -409,20 +488,31 @@ __global__ void __launch_bounds__(kSumThreads) k_seq_sum(const double* __restric
         const double before = __shfl_sync(0xffffffffu, run, f > 0 ? f - 1 : 0);
         if (f > pos) s = fit ? (S + before) * u : s;
         if (lane == 0) {
-          if (f < 32) {
-            const long long b = tile * kSumTile + (long long)f * kSumRun;
-            const int m = (int)(n - b < kSumRun ? (n - b > 0 ? n - b : 0) : kSumRun);
-#pragma unroll 8
-            for (int j = 0; j < m; j++) s += t[b + j];
-          }
           s_sh = s;
-          pos_sh = f < 32 ? f + 1 : 32;
+          pos_sh = f;
+        }
+      }
+      __syncthreads();
+      pos = pos_sh;
+      if (warp == pos) {  // its own sub-tile, from its registers
+        int m = 0;  // without the zeros, which leave any sum as it is (s = -0 cannot be)
+#pragma unroll
+        for (int r = 0; r < kSumPer; r++) {
+          const unsigned b = __ballot_sync(0xffffffffu, v[r] != 0.0);
+          if (v[r] != 0.0) chain[m + __popc(b & ((1u << lane) - 1u))] = v[r];
+          m += __popc(b);
+        }
+        __syncwarp();
+        if (lane == 0) {
+          s = s_sh;
+#pragma unroll 16
+          for (int j = 0; j < m; j++) s += chain[j];
+          s_sh = s;
         }
       }
       __syncthreads();
       s = s_sh;
-      pos = pos_sh;
-      __syncthreads();
+      pos++;
     }
 #pragma unroll
     for (int r = 0; r < kSumPer; r++) v[r] = next[r];
@@ -714,6 +804,7 @@ struct Scratch {
     if (err == cudaSuccess) bufs.push_back(p);
     return static_cast<T*>(p);
   }
+  size_t left() const { return end - next; }
   template <class T>
   T* upload(const T* h, size_t n, cudaStream_t s) {
     T* d = alloc<T>(n);
@@ -939,7 +1030,22 @@ extern "C" vh_status vh_init_glissando(vh_ctx* ctx, const vh_glissando_ic* ic, d
   if (sc.err != cudaSuccess) return ic_cuda(ctx, sc.err, who);
   const long long ncol = (long long)g.nx * g.ny;
   const long long nch = (nz + vh::icr::kKz - 1) / vh::icr::kKz;
-  vh::icr::k_gliss_rho<<<blocks(ncol * nch), kTpb, 0, s>>>(a);
+  // the Gaussians of as many sources at a time as the staging memory left (at
+  // least 4 MB) holds
+  a.bw = (int)std::min(2LL * a.ns + 1, (long long)g.nx);
+  a.bh = (int)std::min(2LL * a.ns + 1, (long long)g.ny);
+  const long long box = (long long)a.bw * a.bh;
+  const size_t room = std::max(sc.left(), (size_t)(4 << 20) + 256) - 256;
+  const long long some =
+      std::min(nsrc, std::max(1LL, (long long)(room / sizeof(double)) / box));
+  a.tr = sc.alloc<double>((size_t)(box * some));
+  if (sc.err != cudaSuccess) return ic_cuda(ctx, sc.err, who);
+  for (long long k0 = 0; k0 < nsrc; k0 += some) {
+    a.k0 = (int)k0;
+    a.k1 = (int)std::min(nsrc, k0 + some);
+    vh::icr::k_gliss_tr<<<blocks(box * (a.k1 - a.k0)), kTpb, 0, s>>>(a);
+    vh::icr::k_gliss_rho<<<blocks(ncol * nch), kTpb, 0, s>>>(a);
+  }
 
   // sNorm, nNorm (src/icGlissando.cpp:164-181) against np_tot / nevents
   double h_sum = 0.;
