@@ -74,46 +74,42 @@ EVENT_SEED = 20260001  # the Glauber event of the timed run (rank r: EVENT_SEED 
 COMPULSORY_B = 288  # bytes per cell-update: Q[7] + pi[10] + Pi, read + write
 
 # Algorithmic bytes of each kernel: the fields a launch must read and write
-# once (stencil neighbours come from cache), per grid cell, or for the
-# relaxation and the advection per cell on the packed list of cells with
-# matter (nactive, read from the device every step).
-KERNEL_BYTES = {
-    "k_update_m": 48,       # m[3] in, m[3] out
-    "k_face": 360,          # per direction Q or Qh [7] + m in, face flux [7] out
-    "k_update": 336,        # 3 face fluxes [21] + Q/Qh [7] in, 2 x [7] out
-    "k_ghost": 0,           # boundary planes only
-    "k_visc_prims": 152,    # Qh [7] in, prims [8] + [4] out
-    "k_visc_update": 288,   # prims [4], piH [10], PiH, m [3], flux [4], Q [7] in; Q [7] out
+# once (stencil neighbours come from cache), per cell with matter (the packed
+# list's count, nactive, read from the device every step) and per grid cell:
+# the vacuum costs the face list Q_t and, in the predictor, its rows' copies.
+KERNEL_BYTES = {  # (per listed cell, per grid cell)
+    "k_update_m": (0, 48),      # m[3] in, m[3] out
+    "k_face": (360, 8),         # per direction Q or Qh [7] + m in, face flux [7] out; Q_t
+    "k_update": (336, 0),       # 3 face fluxes [21] + Q/Qh [7] in, 2 x [7] out
+    "k_ghost": (0, 0),          # boundary planes only
+    "k_visc_prims": (152, 0),   # Qh [7] in, prims [8] + [4] out
+    "k_visc_update": (288, 8),  # prims [4], piH [10], PiH, m [3], flux [4], Q [7] in; Q [7] out; e
+    "k_is_relax": (492, 0),     # index, e and v [4], thermodynamics [6], B and C [9], u [5],
+                                # pi, Pi [11] in; pi0, piH0, Pi0, PiH0 [22], flux [4] out
+    "k_is_advect": (496, 0),    # prims [5], pi0, piH0, Pi0, PiH0 [22], flux [4] in;
+                                # pi, piH, Pi, PiH, vcc [23], flux [4] out
 }
-RELAX_ACTIVE_B = 528  # per listed cell: Q, Qprev [14], m [3], prims [12], pi, Pi [11] in;
-                      # pi0, piH0, Pi0, PiH0 [22], flux [4] out
-RELAX_VACUUM_B = 208  # per empty cell, by the list kernel: pi0, piH0, Pi0, PiH0, flux [26] out
-RELAX_LIST_B = 12     # per cell: e of the half-step prims in, per listed cell its index out
-ADVECT_ACTIVE_B = 496  # per listed cell: prims [5], pi0, piH0, Pi0, PiH0 [22], flux [4] in;
-                       # pi, piH, Pi, PiH, vcc [23], flux [4] out
-KERNEL_BYTES_RULE = {
-    "k_is_relax": "%d B x listed cells + %d B x empty cells + %d B x cells (k_relax_list + k_is_relax)"
-                  % (RELAX_ACTIVE_B, RELAX_VACUUM_B, RELAX_LIST_B),
-    "k_is_advect": "%d B x listed cells" % ADVECT_ACTIVE_B,
-}
-for _k, _b in KERNEL_BYTES.items():
-    KERNEL_BYTES_RULE[_k] = "%d B x cells" % _b
+VACUUM_COPY_B = 84  # per empty cell and pass: Q [7] in, Qh, Qprev [14] out, in one of the two
 
 
-def kernel_alg_bytes(prof, cells, nactive):
+def kernel_alg_bytes(prof, cells, steps, nactive):
     """Algorithmic bytes of every profiled kernel summed over its launches;
     nactive is the listed-cell count summed over the profiled steps."""
     out = {}
     for k, (n, _) in prof.items():
         if k in KERNEL_BYTES:
-            out[k] = float(KERNEL_BYTES[k]) * cells * n
-    if "k_is_relax" in prof:
-        n = prof["k_is_relax"][0]
-        out["k_is_relax"] = (RELAX_ACTIVE_B * nactive + RELAX_VACUUM_B * (n * cells - nactive)
-                             + RELAX_LIST_B * n * cells)
-    if "k_is_advect" in prof:
-        out["k_is_advect"] = float(ADVECT_ACTIVE_B) * nactive
+            listed, grid = KERNEL_BYTES[k]
+            out[k] = n * (listed * nactive / steps + float(grid) * cells)
+    if "k_face" in out:
+        out["k_face"] += prof["k_face"][0] * VACUUM_COPY_B * (cells - nactive / steps)
     return out
+
+
+def kernel_bytes_rule(k):
+    if k not in KERNEL_BYTES:
+        return ""
+    rule = "%d B x listed cells + %d B x cells" % KERNEL_BYTES[k]
+    return rule + (" + %d B x empty cells" % VACUUM_COPY_B if k == "k_face" else "")
 
 
 # the persistent per-cell state a step reads or leaves for the next one (the
@@ -221,8 +217,8 @@ def gpu_index_for(local_rank):
     return str(local_rank)
 
 
-# kernels whose work is the listed cells with matter (k_relax_list's list)
-ACTIVE_KERNELS = ("k_is_relax", "k_is_advect")
+# kernels whose work is the cells with matter
+ACTIVE_KERNELS = ("k_face", "k_update", "k_visc_prims", "k_is_relax", "k_is_advect", "k_visc_update")
 
 
 def ncu_per_launch(fname, field, kernel, grid, launches, warmup, active_per_step):
@@ -852,7 +848,7 @@ def main():
     # per-kernel algorithmic bytes over the timed steps and the dominant
     # kernel's roofline
     peak, peak_kind = measured_peaks()
-    alg_total = kernel_alg_bytes(prof, cells, nactive)
+    alg_total = kernel_alg_bytes(prof, cells, args.steps, nactive)
     dom = max(prof.items(), key=lambda kv: kv[1][1])
     dname, (dn, dms) = dom
     avg_s = dms / dn / 1e3
@@ -863,7 +859,7 @@ def main():
                 "traffic": None,
                 "alg_bytes_per_launch": alg, "avg_launch_ms": avg_s * 1e3,
                 "active_cells_per_step": nactive / args.steps,
-                "alg_bytes_rule": KERNEL_BYTES_RULE.get(dname, "")}
+                "alg_bytes_rule": kernel_bytes_rule(dname)}
     # FP64 co-roofline: the dominant kernel's and the whole step's FP64
     # operations (ncu counts of the same launches) over their CUDA-event
     # time, against a cuBLAS DGEMM measured now
