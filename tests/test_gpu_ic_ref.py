@@ -210,6 +210,51 @@ def test_gpu_urqmd_full_grid_equals_oracle(tmp_path):
     print(msg)
 
 
+@pytest.mark.parametrize("model", [5, 7, 4, 2, 3])
+def test_gpu_ic_keeps_no_device_memory(model, grid_setup, tmp_path):
+    """A context holds no more device memory after an initial state than
+    before it (42 MB are 10 doubles per cell at 101x101x51), and a step from
+    it, whose face fluxes the call may use for its buffers, is the oracle's."""
+    import dataclasses
+    torch = pytest.importorskip("torch")
+    path = str(tmp_path / "input.txt")
+    if model == 5:
+        F.write_glissando(path, F.synthetic_glissando_events(2, seed=5))
+        data, su = F.read_glissando(path), capi.ic_setup(capi.IC_GLISSANDO, "RHIC62")
+        init = lambda h: h.init_glissando(data, su)  # noqa: E731
+    elif model == 7:
+        F.write_trento(path, F.synthetic_trento_events(2, seed=7, n=60))
+        data, su = F.read_trento(path), capi.ic_setup(capi.IC_TRENTO, "RHIC62")
+        init = lambda h: h.init_trento(data, su)  # noqa: E731
+    elif model == 2:
+        F.synthetic_song_table().write(path)
+        data, su = F.read_song_table(path), None
+        init = lambda h: h.init_table(data, 1.0, 1)  # noqa: E731
+    elif model == 3:
+        F.write_urqmd(path, F.synthetic_urqmd_events(2, seed=5, nmean=300))
+        data, su = F.read_urqmd(path), None
+        init = lambda h: h.init_urqmd(data, 1.0, 1.0)  # noqa: E731
+    else:
+        data, su = None, None
+        init = lambda h: h.init_gubser()  # noqa: E731
+    small = W.glauber3d_setup(nx=21, ny=21, nz=9, xmax=12.0, etamax=6.0)
+    h = capi.GpuHydro(small, upload=False)
+    init(h)  # loads the kernels
+    o, _ = P.oracle_ic(small, model, data, su, crmath=True)
+    h.step(1)
+    run = P.OracleRun(dataclasses.replace(small, Q=o["Q"], m=o["m"][0].copy()))
+    assert run.step(1) == 0
+    assert np.array_equal(h.get_state(("Q",))["Q"], run.get_state()["Q"].reshape(7, -1))
+    h.close()
+    h = capi.GpuHydro(W.glauber3d_setup(), upload=False)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    init(h)
+    after = torch.cuda.mem_get_info()[0]
+    h.close()
+    assert before - after < 8 << 20, (before, after)
+
+
 def test_gpu_ic_refused_on_a_slab(grid_setup):
     h = capi.GpuHydro(grid_setup, upload=False)
     try:

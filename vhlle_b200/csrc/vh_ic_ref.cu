@@ -770,41 +770,43 @@ const SetupEntry kSetups[] = {
     {7, "RHIC27", {27, 0, 0, 1.0, 3.36, 0.123, 0.4, 0.0, 0, 0}},
 };
 
-// A call's device buffers: from the context's resize staging (10 doubles per
-// cell, kept; the call's use of it is ordered by the context's stream), and
-// allocated where that is full.  Allocating and freeing thirteen buffers took
-// 1.9 of a call's 7.0 ms (101 x 101 x 51 cells, 10 sources).
+// A call's device buffers: from the context's face fluxes (3 x 7 doubles per
+// cell, which hold nothing between steps; the call's use of them is ordered
+// by the context's stream), and allocated, and freed when it returns, where
+// those are full.  Allocating and freeing thirteen buffers took 1.9 of a
+// call's 7.0 ms (101 x 101 x 51 cells, 10 sources).
 struct Scratch {
   std::vector<void*> bufs;
   cudaError_t err = cudaSuccess;
-  char *next = nullptr, *end = nullptr;
+  struct Span {
+    char *next, *end;
+    size_t left() const { return end - next; }
+  } spans[3];
   explicit Scratch(vh_ctx* ctx) {
-    const size_t bytes = sizeof(double) * 10 * ctx->g.N;
-    if (!ctx->resize_tmp) {
-      err = cudaMalloc(&ctx->resize_tmp, bytes);
-      if (err == cudaSuccess) ctx->allocs.push_back(ctx->resize_tmp);
-    }
-    if (err == cudaSuccess) {
-      next = reinterpret_cast<char*>(ctx->resize_tmp);
-      end = next + bytes;
-    }
+    double* const f[3] = {ctx->f.Fx, ctx->f.Fy, ctx->f.Fz};
+    for (int k = 0; k < 3; k++)
+      spans[k] = {reinterpret_cast<char*>(f[k]), reinterpret_cast<char*>(f[k] + 7 * ctx->g.N)};
   }
   Scratch(const Scratch&) = delete;
   Scratch& operator=(const Scratch&) = delete;
   template <class T>
   T* alloc(size_t n) {
     const size_t bytes = (sizeof(T) * (n ? n : 1) + 255) / 256 * 256;
-    if (err == cudaSuccess && bytes <= (size_t)(end - next)) {
-      T* p = reinterpret_cast<T*>(next);
-      next += bytes;
-      return p;
-    }
+    for (Span& sp : spans)
+      if (bytes <= sp.left()) {
+        T* p = reinterpret_cast<T*>(sp.next);
+        sp.next += bytes;
+        return p;
+      }
     void* p = nullptr;
     if (err == cudaSuccess) err = cudaMalloc(&p, bytes);
     if (err == cudaSuccess) bufs.push_back(p);
     return static_cast<T*>(p);
   }
-  size_t left() const { return end - next; }
+  // the largest buffer to be had without an allocation
+  size_t left() const {
+    return std::max(spans[0].left(), std::max(spans[1].left(), spans[2].left()));
+  }
   template <class T>
   T* upload(const T* h, size_t n, cudaStream_t s) {
     T* d = alloc<T>(n);
@@ -1030,8 +1032,8 @@ extern "C" vh_status vh_init_glissando(vh_ctx* ctx, const vh_glissando_ic* ic, d
   if (sc.err != cudaSuccess) return ic_cuda(ctx, sc.err, who);
   const long long ncol = (long long)g.nx * g.ny;
   const long long nch = (nz + vh::icr::kKz - 1) / vh::icr::kKz;
-  // the Gaussians of as many sources at a time as the staging memory left (at
-  // least 4 MB) holds
+  // the Gaussians of as many sources at a time as the memory left (at least
+  // 4 MB) holds
   a.bw = (int)std::min(2LL * a.ns + 1, (long long)g.nx);
   a.bh = (int)std::min(2LL * a.ns + 1, (long long)g.ny);
   const long long box = (long long)a.bw * a.bh;
