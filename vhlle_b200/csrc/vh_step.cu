@@ -561,6 +561,40 @@ __host__ __device__ inline Shell ghost_shell(const Geo& g) {
   s.n = s.b + (long long)s.iz * s.iy * s.gx;
   return s;
 }
+// Row i becomes row s (read before), or zeros where its Q_t is negative.  A
+// cell that is its own source keeps its row, and may be read by other threads
+// meanwhile (sides of 4 or fewer, where the sources are copied into too):
+// zeroed, it stores Q_t last.  So a reader that finds a negative Q_t stores
+// zeros whatever else it found, one that finds another Q_t but 0 has a row
+// that nobody writes, and one that finds 0 beside anything but zeros reads
+// again, behind a fence, what was stored before that 0.
+__device__ __forceinline__ void ghost_read(const double* F, long long N, long long s, double q[7]) {
+  q[0] = *(const volatile double*)(F + s);
+#pragma unroll
+  for (int k = 1; k < 7; k++) q[k] = F[k * N + s];
+}
+__device__ __forceinline__ void ghost_store(double* F, long long N, long long i, long long s,
+                                            double q[7]) {
+  const bool neg = q[0] < 0.;
+  if (s == i) {
+    if (!neg) return;
+#pragma unroll
+    for (int k = 1; k < 7; k++) F[k * N + i] = 0.;
+    __threadfence();
+    *(volatile double*)(F + i) = 0.;
+    return;
+  }
+  bool rest = false;
+#pragma unroll
+  for (int k = 1; k < 7; k++) rest |= q[k] != 0.;
+  if (q[0] == 0. && rest) {
+    __threadfence();
+#pragma unroll
+    for (int k = 1; k < 7; k++) q[k] = *(const volatile double*)(F + k * N + s);
+  }
+#pragma unroll
+  for (int k = 0; k < 7; k++) F[k * N + i] = neg ? 0. : q[k];
+}
 __device__ __forceinline__ int ghost_index(int k, int n) { return k < 2 || n <= 4 ? k : n - 4 + k; }
 
 template <bool HALF, bool FULL>
@@ -595,36 +629,28 @@ __device__ __forceinline__ void d_ghost(const Geo& g, const int* __restrict__ sr
   const long long N = g.N;
   const long long i = (long long)ix + (long long)g.nx * (iy + (long long)g.ny * iz);
   const long long s = (long long)sx[ix] + (long long)g.nx * (sy[iy] + (long long)g.ny * sz[iz]);
-  {
-    double q[7];
+  double q[7], h[7], p[11];  // the loads of all rows together
+  ghost_read(f.Q, N, s, q);
+  if (HALF) ghost_read(f.Qh, N, s, h);
+  if (FULL) {
 #pragma unroll
-    for (int k = 0; k < 7; k++) q[k] = f.Q[k * N + s];
-    const bool neg = q[0] < 0.;
-#pragma unroll
-    for (int k = 0; k < 7; k++) f.Q[k * N + i] = neg ? 0. : q[k];
+    for (int k = 0; k < 10; k++) p[k] = f.pi[k * N + s];
+    p[10] = f.Pi[s];
   }
+  ghost_store(f.Q, N, i, s, q);
   if (HALF) {
-    double q[7];
-#pragma unroll
-    for (int k = 0; k < 7; k++) q[k] = f.Qh[k * N + s];
-    const bool neg = q[0] < 0.;
-#pragma unroll
-    for (int k = 0; k < 7; k++) f.Qh[k * N + i] = neg ? 0. : q[k];
+    ghost_store(f.Qh, N, i, s, h);
     if (wet) {
-      if (!(q[0] <= 0.))
+      if (!(h[0] <= 0.))
         append(wet, f.fcount + 6, (int)i);
       else
         empty_prims(f.pA, f.pD, N, i);
     }
   }
-  if (FULL) {
-    double p[10];
-#pragma unroll
-    for (int k = 0; k < 10; k++) p[k] = f.pi[k * N + s];
-    const double P = f.Pi[s];
+  if (FULL && s != i) {
 #pragma unroll
     for (int k = 0; k < 10; k++) f.pi[k * N + i] = p[k];
-    f.Pi[i] = P;
+    f.Pi[i] = p[10];
   }
 }
 template <bool HALF, bool FULL>
