@@ -258,3 +258,27 @@ def test_negative_rows_beside_the_edge_equal_oracle(nx, ny, nz, viscous):
         if found == 8:
             break
     assert found
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(9, 8, 1), (21, 20, 1), (9, 8, 7), (5, 6, 4), (12, 11, 10)])
+def test_root_finds_of_a_step(nx, ny, nz):
+    """Matter everywhere, moving, at a clock without rounding: a viscous step
+    solves two states per face and one per cell in each pass, then D and C of
+    every cell, and A of the cells that the ghost copy writes only, once."""
+    s = W.glauber3d_setup(nx=nx, ny=ny, nz=nz, xmax=5.0, etamax=3.0) if nz > 1 else W.gubser_setup(nx, ny)
+    s.tau0, s.dt = 1.0, 0.0625
+    s.eos = W.EosTable(kind=0)
+    N = s.grid.ncells
+    one = np.ones(N)
+    s.Q = W.conserved_from_primitive(s.tau0, 10. * one, 10. / 3 * one, 0. * one, 0.3 * one, 0.2 * one,
+                                     0.1 * one).reshape(7, -1)
+    s.m = one
+    s.tr = dict(s.tr, etaS0=0.1, zetaS0=0.0)
+    h = capi.GpuHydro(s)
+    h.con2prim_stats(True)
+    h.step(1)
+    calls = h.con2prim_stats(False)[0]
+    h.close()
+    faces = (nx - 1) * ny * nz + nx * (ny - 1) * nz + nx * ny * (nz - 1)
+    inner = max(nx - 4, 0) * max(ny - 4, 0) * max(nz - 4, 0)
+    assert calls == 2 * (2 * faces + N) + 2 * N + (N - inner)

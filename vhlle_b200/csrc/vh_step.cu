@@ -714,21 +714,32 @@ __device__ __forceinline__ void d_visc_prims(const Geo& g, const EosDev& E, cons
   double q[7], qh[7];
   const double tA = tau - dt / 2.;
   Prim a{0., 0., 0., 0., 0., 0., 0., 0.};
-  int gx = 0, gy = 0, gz = 0;
+  // the first half solves A, the second looks for vacuum beside the cell
+  __shared__ double ea[64];
+  __shared__ bool beside[64];
+  const int half = blockDim.x >> 1, slot = second ? threadIdx.x - half : threadIdx.x;
   bool vac = false;
   if (in) {
+    int gx, gy, gz;
     coords(g, i, gx, gy, gz);
-    // A is the corrector's con2prim (k_update<false> stored it in pA) when
-    // its divisor tau_n + dt/2 equals tA bit for bit and the ghost copy has
-    // not changed this cell's Qh since
-    if (tA == clk[0] + 0.5 * dt && !is_ghost(g, gx, gy, gz)) {
-      a = loadA(pA, N, i);
+    if (second) {
+      vac = maxM_at(g, m, gx + 1, gy, gz) <= 0.9 || maxM_at(g, m, gx, gy + 1, gz) <= 0.9 ||
+            maxM_at(g, m, gx - 1, gy, gz) <= 0.9 || maxM_at(g, m, gx, gy - 1, gz) <= 0.9 ||
+            maxM_at(g, m, gx + 1, gy + 1, gz) <= 0.9 ||
+            maxM_at(g, m, gx + 1, gy - 1, gz) <= 0.9 ||
+            maxM_at(g, m, gx - 1, gy + 1, gz) <= 0.9 || maxM_at(g, m, gx - 1, gy - 1, gz) <= 0.9;
+      beside[slot] = vac;
     } else {
+      // A is the corrector's con2prim (k_update<false> stored it in pA) when
+      // its divisor tau_n + dt/2 equals tA bit for bit and the ghost copy has
+      // not changed this cell's Qh since
+      if (tA == clk[0] + 0.5 * dt && !is_ghost(g, gx, gy, gz)) {
+        a = loadA(pA, N, i);
+      } else {
 #pragma unroll
-      for (int k = 0; k < 7; k++) qh[k] = Qh[k * N + i];
-      q_over(qh, tA, q);
-      transform_pv<EK>(E, q, a, c2p_guess(E, i));
-      if (!second) {
+        for (int k = 0; k < 7; k++) qh[k] = Qh[k * N + i];
+        q_over(qh, tA, q);
+        transform_pv<EK>(E, q, a, c2p_guess(E, i));
         pA[0 * N + i] = a.e;
         pA[1 * N + i] = a.p;
         pA[2 * N + i] = a.nb;
@@ -738,14 +749,12 @@ __device__ __forceinline__ void d_visc_prims(const Geo& g, const EosDev& E, cons
         pA[6 * N + i] = a.vy;
         pA[7 * N + i] = a.vz;
       }
+      ea[slot] = a.e;
     }
-    if (!(a.e <= 0.))
-      vac = maxM_at(g, m, gx + 1, gy, gz) <= 0.9 || maxM_at(g, m, gx, gy + 1, gz) <= 0.9 ||
-            maxM_at(g, m, gx - 1, gy, gz) <= 0.9 || maxM_at(g, m, gx, gy - 1, gz) <= 0.9 ||
-            maxM_at(g, m, gx + 1, gy + 1, gz) <= 0.9 ||
-            maxM_at(g, m, gx + 1, gy - 1, gz) <= 0.9 ||
-            maxM_at(g, m, gx - 1, gy + 1, gz) <= 0.9 || maxM_at(g, m, gx - 1, gy - 1, gz) <= 0.9;
   }
+  __syncthreads();
+  if (in && second) a.e = ea[slot];
+  if (in && !second) vac = beside[slot];
   {
     // the list of cells with matter, for the relaxation and the advection
     // (the complement of a cell next to vacuum, which NSquant leaves alone);
