@@ -69,3 +69,28 @@ def test_gpu_hadron_eos_is_only_a_surface_eos(name):
     s = W.glauber3d_nb_setup(9, 9, 5, eos=h)
     with pytest.raises(capi.VhError):
         capi.GpuHydro(s)
+
+
+@pytest.mark.parametrize("name", ["conformal", "table", "nb_table", "chiral", "eos3f", "hadron", "smash", "azh", "cmfe"])
+def test_totals_of_every_kind_equal_oracle(name):
+    """The totals' kernel is one per EoS kind; sums in another order than the
+    oracle's: 1e-12 relative to the sum of the terms' magnitudes, which 1e-10
+    of the sum itself bounds where the terms have one sign (all but the odd
+    moments, taken against the energy)."""
+    make = {"conformal": lambda: W.EosTable(kind=0), "table": W.make_cs2_table, "nb_table": lambda: W.nb_table(200, 20),
+            "chiral": W.chiral_eos, "eos3f": W.eos3f_table, "hadron": W.hadron_eos_table,
+            "smash": W.smash_eos_table, "azh": W.azh_eos_table, "cmfe": W.cmfe_eos_table}[name]
+    own = name in ("hadron", "smash")
+    s = W.glauber3d_nb_setup(21, 20, 11, eos=W.nb_table(200, 20) if own else make())
+    surf = make() if own else None
+    o, d = P.OracleRun(s, surface_eos=surf), capi.GpuHydro(s)
+    if own:
+        d.set_surface_eos(surf)
+    d.step(2)
+    assert o.step(2) == 0
+    to, td = o.totals(), d.totals()
+    e = abs(next(iter(to.values())))
+    for k in to:
+        both_nan = np.isnan(td[k]) and np.isnan(to[k])  # (an entropy where the table's sum has one)
+        assert both_nan or abs(td[k] - to[k]) <= 1e-10 * abs(to[k]) + 1e-12 * e, (k, td[k], to[k])
+    d.close()

@@ -172,14 +172,22 @@ int totals_blocks(const Geo& g) {
 void launch_totals(const Geo& g, const EosDev& E, const Fields& f, double tau, double ecrit,
                    double etamin, bool viscous, double* partial, double* out, cudaStream_t s) {
   const int nb = totals_blocks(g);
-  // the common table kinds alone, the others by kind at run time: with every
-  // kind's lookup compiled in, the kernel held 2 blocks per SM
-  if (E.kind <= 1)
-    k_totals<EK_TABLE><<<nb, kTotBlock, 0, s>>>(g, E, f.Q, f.pi, f.vcc, tau, ecrit, etamin, viscous,
-                                                partial);
-  else
-    k_totals<EK_ANY><<<nb, kTotBlock, 0, s>>>(g, E, f.Q, f.pi, f.vcc, tau, ecrit, etamin, viscous,
-                                              partial);
+  auto run = [&](auto kernel) {
+    kernel<<<nb, kTotBlock, 0, s>>>(g, E, f.Q, f.pi, f.vcc, tau, ecrit, etamin, viscous, partial);
+  };
+  // a kernel per kind (us a call at 101x101x51, with every kind's lookup in one
+  // kernel at 2 blocks per SM, and so: chiral 217 and 166, EoS3f 178 and 158,
+  // hadron 512 and 450, SMASH 179 and 152, AZH 165 and 143, CMFe 150 and 129)
+  switch (E.kind) {
+    case 0:
+    case 1: run(k_totals<EK_TABLE>); break;
+    case 2: run(k_totals<EK_CHIRAL>); break;
+    case 3: run(k_totals<EK_TABLE3>); break;
+    case 4: run(k_totals<EK_HADRON>); break;
+    case 5: run(k_totals<EK_SMASH>); break;
+    case 6: run(k_totals<EK_AZH>); break;
+    default: run(k_totals<EK_CMFE>); break;
+  }
   k_totals_final<<<1, kTotBlock, 0, s>>>(partial, nb, out);
 }
 
