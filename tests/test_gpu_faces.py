@@ -184,6 +184,25 @@ def test_listed_update_with_vorticity_equals_oracle():
     h.close()
 
 
+@pytest.mark.parametrize("viscous", [False, True])
+@pytest.mark.parametrize("nb", [0.0, 0.02])
+def test_full_listed_grid_equals_oracle(viscous, nb):
+    """Matter in every cell of a grid whose faces and cells are listed."""
+    s = W.glauber3d_setup(nx=54, ny=53, nz=55, xmax=9.0, etamax=5.0, eos=W.nb_table(400, 40) if nb else None)
+    N = s.grid.ncells
+    rng = np.random.default_rng(6)
+    e = 1. + rng.random(N)
+    s.Q = W.conserved_from_primitive(s.tau0, e, e / 4, nb * e, 0.2 + 0. * e, -0.1 + 0. * e, 0. * e).reshape(7, -1)
+    s.m = np.ones(N)
+    s.tr = dict(s.tr, etaS0=0.08 if viscous else 0.0, zetaS0=0.0)
+    h, o = capi.GpuHydro(s), P.OracleRun(s)
+    h.step(2)
+    assert o.step(2) == 0
+    bad = compare_states(gpu_state_as_oracle(h.get_state()), o.get_state())
+    assert not bad, bad
+    h.close()
+
+
 @pytest.mark.parametrize("form", ["ordinary", "tiny", "mixed", "zero", "no_shear", "bump", "large_dt"])
 def test_relaxation_ranges_equal_oracle(form):
     """Shear and bulk stresses inside and outside the ranges in which the

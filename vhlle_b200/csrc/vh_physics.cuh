@@ -947,33 +947,38 @@ __device__ __forceinline__ double eos_s(const EosDev& E, double e, double nb,
 // One loop holds the only EoS lookup: the start point's, each iterate's and
 // the final state's pressure are its trips, so the final lookup of a lane
 // that is done shares a trip with the others' next iterates, and the
-// kernels' code is a third of the unrolled form's (the face kernels spent
-// most of their issue slots waiting for instructions: 5.6 of 14 cycles per
-// issue, at 101x101x51).
-template <int EK = EK_ANY>
-__device__ __forceinline__ void transform_pv(const EosDev& E, double Q[7], Prim& o,
-                                             float g = -1.f) {
-  const int MAXIT = 100;
-  const double dpe = 1. / 3.;
+// kernels' code is a third of the unrolled form's (whose face kernels waited
+// for instructions 5.6 of the 14 cycles between two issues of a warp, at
+// 101x101x51).
+//
+// In three parts, so that a caller short of registers can put away what the
+// root find does not need (Q_i, Q_nq, Q_ns): c2p_start, c2p_root, c2p_state.
+
+// |Q_i|, and |Q_i| > Q_t cut back to corrf Q_t; false for vacuum (Q_t <= 0)
+__device__ __forceinline__ bool c2p_start(double Q[7], double& M) {
   const double corrf = 0.9999;
-  double M = sqrtz(Q[X_] * Q[X_] + Q[Y_] * Q[Y_] + Q[Z_] * Q[Z_]);
-  if (Q[T_] <= 0.) {
-    o.e = 0.; o.p = 0.;
-    o.vx = o.vy = o.vz = 0.;
-    o.nb = o.nq = o.ns = 0.;
-    return;
-  }
+  M = sqrtz(Q[X_] * Q[X_] + Q[Y_] * Q[Y_] + Q[Z_] * Q[Z_]);
+  if (Q[T_] <= 0.) return false;
   if (M > Q[T_]) {
     Q[X_] *= corrf * Q[T_] / M;
     Q[Y_] *= corrf * Q[T_] / M;
     Q[Z_] *= corrf * Q[T_] / M;
     M = Q[T_] * corrf;
   }
+  return true;
+}
+
+// v, e and p of the state with Q_t, Q_nb and |Q_i| = M
+template <int EK>
+__device__ __forceinline__ void c2p_root(const EosDev& E, double QT, double QNB, double M, float g,
+                                         double& v, double& e, double& p) {
+  const int MAXIT = 100;
+  const double dpe = 1. / 3.;
   const bool rest = M == 0.;  // v = 0: one trip, for p(Q_t, Q_nb)
   const bool guessed = g > 0.f && g < 1.f;
   double vl = 0., vh = 1., dvold = 1., dv = 1.;
-  double v = guessed ? (double)g : 0.5;
-  double e, p, nb = Q[NB_];
+  v = guessed ? (double)g : 0.5;
+  double nb = QNB;
   // The table-slope variant (ek_slope) takes f' = (Q_t + p) - v (M dp/de +
   // dp/dnb Q_nb v / sqrt(1 - v^2)) with the EoS's own derivatives, so the
   // Newton steps converge quadratically inside a table cell, and stops when
@@ -982,16 +987,16 @@ __device__ __forceinline__ void transform_pv(const EosDev& E, double Q[7], Prim&
   // only, where the result does not depend on the path to the root.
   constexpr bool SL = ek_slope(EK);
   // Q_nb = +-0 stays Q_nb times any square root of a number in [0, 1]
-  const bool nb0 = !SL && Q[NB_] == 0.;
+  const bool nb0 = !SL && QNB == 0.;
   bool done = rest, keep_nb = rest;
   int it = 0;
 #pragma unroll 1
   while (true) {
-    e = Q[T_] - M * v;
+    e = QT - M * v;
     double sq = 0.;
     if (!keep_nb && !(nb0 && fabs(v) <= 1.)) {
       sq = sqrt(1 - v * v);
-      nb = Q[NB_] * sq;
+      nb = QNB * sq;
     }
     if (!done && e < 0.) e = 0.;
     double dpde = 0., dpdn = 0.;
@@ -1001,17 +1006,17 @@ __device__ __forceinline__ void transform_pv(const EosDev& E, double Q[7], Prim&
       p = eos_p<EK>(E, e, nb);
     }
     if (done) break;  // p of the state at v, with the last iterate's nb, as the reference
-    const double f = (Q[T_] + p) * v - M;
+    const double f = (QT + p) * v - M;
     if (SL && f == 0.) {
       done = keep_nb = true;
       continue;
     }
     double df;
     if (SL) {
-      const double dn = sq > 0. ? dpdn * Q[NB_] * v / sq : 0.;
-      df = (Q[T_] + p) - v * (M * dpde + dn);
+      const double dn = sq > 0. ? dpdn * QNB * v / sq : 0.;
+      df = (QT + p) - v * (M * dpde + dn);
     } else {
-      df = (Q[T_] + p) - M * v * dpe;
+      df = (QT + p) - M * v * dpe;
     }
     if (it > 0 || guessed) {
       if (f > 0.)
@@ -1034,16 +1039,21 @@ __device__ __forceinline__ void transform_pv(const EosDev& E, double Q[7], Prim&
     keep_nb = fabs(dv) < E.tol;
     done = keep_nb || it == MAXIT;
   }
-  if (rest) {
+  if (E.stats && !rest) {
+    atomicAdd(&E.stats[0], 1ull);
+    atomicAdd(&E.stats[1], (unsigned long long)it);
+  }
+}
+
+// the primitives at that root
+__device__ __forceinline__ void c2p_state(const double Q[7], double M, double v, double e, double p,
+                                          Prim& o) {
+  o.p = p;
+  if (M == 0.) {
     o.e = Q[T_];
-    o.p = p;
     o.vx = 0.; o.vy = 0.; o.vz = 0.;
     o.nb = Q[NB_]; o.nq = Q[NQ_]; o.ns = Q[NS_];
     return;
-  }
-  if (E.stats) {
-    atomicAdd(&E.stats[0], 1ull);
-    atomicAdd(&E.stats[1], (unsigned long long)it);
   }
   {
     // v Q_i / M, i = x, y, z: one divide for RN(1/M) and crm::mk_div
@@ -1061,11 +1071,24 @@ __device__ __forceinline__ void transform_pv(const EosDev& E, double Q[7], Prim&
     }
   }
   o.e = e;
-  o.p = p;
   const double sq = sqrt(1 - o.vx * o.vx - o.vy * o.vy - o.vz * o.vz);
   o.nb = Q[NB_] * sq;
   o.nq = Q[NQ_] * sq;
   o.ns = Q[NS_] * sq;
+}
+
+template <int EK = EK_ANY>
+__device__ __forceinline__ void transform_pv(const EosDev& E, double Q[7], Prim& o,
+                                             float g = -1.f) {
+  double M, v, e, p;
+  if (!c2p_start(Q, M)) {
+    o.e = 0.; o.p = 0.;
+    o.vx = o.vy = o.vz = 0.;
+    o.nb = o.nq = o.ns = 0.;
+    return;
+  }
+  c2p_root<EK>(E, Q[T_], Q[NB_], M, g, v, e, p);
+  c2p_state(Q, M, v, e, p, o);
 }
 
 // ------------------------------------------------- transport coefficients

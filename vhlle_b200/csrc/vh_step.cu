@@ -22,8 +22,8 @@
 namespace vh {
 
 // resident blocks of 128 threads per SM, from sweeps (us per step at the
-// stated counts): the face kernel 5 / 6 / 8 blocks 161 / 160 / 153 on the
-// 101x101x51 event; the update on a list 5 / 6 / 7 / 8: 64 / 54 / 56 / 58
+// stated counts): the face kernel 5 / 6 / 7 / 8 blocks 151 / 149 / 146 / 143 on
+// the 101x101x51 event; the update on a list 5 / 6 / 7 / 8: 64 / 54 / 56 / 58
 // there, 149 / 145 / 148 / 156 on 201x201x101, and on every cell of the 2+1D
 // grid of 101x101 4 / 5 / 6: 36 / 37 / 40; the viscous primitives 6 / 7 / 8:
 // 30.8 / 31.5 / 33.1
@@ -211,11 +211,16 @@ __device__ __forceinline__ void d_face_list(const Geo& g, const Fields& f, bool 
         // two empty cells have two empty edges (a slope takes the smaller side)
         if (cc[d] >= nn[d] - 1 || (x1 == 0. && x2 == 0.)) continue;
         const long long st = ss[d];
+        const bool dry = m[d * N + i] < 1. && m[d * N + i + st] < 1.;
+        if (x1 > 0. && x2 > 0. && !dry) {  // matter on both sides: edges > 0
+          act |= 1u << d;
+          continue;
+        }
         const double x0 = cc[d] > 0 ? dn[d] : x1, x3 = cc[d] < nn[d] - 2 ? QT[i + 2 * st] : x2;
         const double el = x1 + minmod((x2 - x1) / 2., (x1 - x0) / 2.);
         const double er = x2 - minmod((x3 - x2) / 2., (x2 - x1) / 2.);
         if (el <= 0. && er <= 0.) continue;
-        if (m[d * N + i] < 1. && m[d * N + i + st] < 1. && el <= huge) continue;
+        if (dry && el <= huge) continue;
         act |= 1u << d;
       }
     }
@@ -268,7 +273,17 @@ __global__ void __launch_bounds__(128) k_face_list(Geo g, Fields f, bool predict
 // warps) spent 5.6 of 14 cycles per issue waiting for instructions; in this
 // form it is 0.5 of 9.  101x101x51, two passes, 20 % of the cells with
 // matter: 492 us a step in that form, 280 in this one over the whole grid,
-// 153 over the lists (with the list kernels).
+// 144 over the lists (with the list kernels).
+//
+// A state's 21 loads go out together, also for vacuum edges (with Q_t first
+// and the rest behind its test 147 us), and what the root find does not need
+// waits in shared memory (640 / 896 bytes of spills without, 532 / 792 so).
+// A grid without any empty cell gains least from this form: lists, faces and
+// hlle_flux of 101x101x51 cells 570 us a step in the three kernels, 553 here,
+// but with charge 590 and 640, and 3950 and 4240, 4190 and 4900 of 201x201x101.
+// Tried for those: both states of a face by one thread in turn (no barrier)
+// even without charge, 4 % slower with; the flux one component at a time (324
+// / 304 bytes of spills) 4 % slower; 5, 6 and 7 blocks per SM 3 to 8 % slower.
 struct FaceBatch {
   int cnt[3], blocks[3];  // listed faces, and blocks of B / 2 of them, per direction
 };
@@ -315,21 +330,29 @@ __device__ __forceinline__ void d_face(const Geo& g, const EosDev& E, bool predi
     if (right) c++;
     const long long cell = i + (right ? st : 0);
     const long long lo = cell - (c > 0 ? st : 0), hi = cell + (c < n - 1 ? st : 0);
-    // the reconstructed state, then divided by tau as one batch; the state
-    // of vacuum (Q_t <= 0, transform_pv's first test) needs no more than Q_t
-    double q[7];
-    auto edge = [&](int k) {
+    // the reconstructed state, then divided by tau as one batch
+    double q[7], M;
+#pragma unroll
+    for (int k = 0; k < 7; k++) {
       const double x0 = QQ[k * N + lo], x1 = QQ[k * N + cell], x2 = QQ[k * N + hi];
       const double dQ = minmod((x2 - x1) / 2., (x1 - x0) / 2.);
-      return x1 + (right ? -dQ : dQ);
-    };
+      q[k] = x1 + (right ? -dQ : dQ);
+    }
     Prim p{0., 0., 0., 0., 0., 0., 0., 0.};
-    q[0] = edge(0);
-    if (!(q[0] <= 0.)) {
-#pragma unroll
-      for (int k = 1; k < 7; k++) q[k] = edge(k);
+    if (!(q[T_] <= 0.)) {
       div_batch<7>(q, tau, 1.0 / tau, crm::mk_den_ok(tau));
-      transform_pv<EK>(E, q, p, c2p_guess(E, cell));
+      if (c2p_start(q, M)) {
+        // what the root find does not need waits in the thread's own slots of sp
+        volatile double* park = &sp[0][t];
+        const int keep[5] = {X_, Y_, Z_, NQ_, NS_};
+#pragma unroll
+        for (int k = 0; k < 5; k++) park[128 * k] = q[keep[k]];
+        double v, e, pr;
+        c2p_root<EK>(E, q[T_], q[NB_], M, c2p_guess(E, cell), v, e, pr);
+#pragma unroll
+        for (int k = 0; k < 5; k++) q[keep[k]] = park[128 * k];
+        c2p_state(q, M, v, e, pr, p);
+      }
     }
     sp[0][t] = p.e;
     sp[1][t] = p.p;
@@ -339,6 +362,11 @@ __device__ __forceinline__ void d_face(const Geo& g, const EosDev& E, bool predi
     sp[5][t] = p.vx;
     sp[6][t] = p.vy;
     sp[7][t] = p.vz;
+  }
+  double mL = 0., mR = 0.;  // before the barrier, whose wait covers the loads
+  if (face && !right) {
+    mL = m[(dir - 1) * N + i];
+    mR = m[(dir - 1) * N + i + st];
   }
   __syncthreads();
   if (right || !face) return;
@@ -350,7 +378,7 @@ __device__ __forceinline__ void d_face(const Geo& g, const EosDev& E, bool predi
   double fl[7];
   unsigned e = 0;
   const bool ok = hlle_face(dir, predict, tau, dt, dxdir, prim(t), prim(t + half),
-                            m[(dir - 1) * N + i], m[(dir - 1) * N + i + st], fl, e);
+                            mL, mR, fl, e);
   if (e) atomicOr(err, e);
 #pragma unroll
   for (int k = 0; k < 7; k++) F[k * N + i] = ok ? fl[k] : 0.;
