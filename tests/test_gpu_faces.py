@@ -163,16 +163,18 @@ def test_listed_faces_equal_oracle(nx, ny, nz, nb):
     h.close()
 
 
-# the ideal update runs on a list above 888 blocks of 128 cells: sizes on both
-# sides of the line, the list's blocks of 512 with and without a remainder,
-# and the temperatures that the vorticity takes from it
-@pytest.mark.parametrize("nx,ny,nz", [(48, 48, 49), (49, 49, 48), (64, 64, 28), (337, 339, 1)])
+# the ideal update runs on a list above 1184 blocks of 128 cells: sizes on both
+# sides of the line, the last block with and without a remainder, and the
+# temperatures that the vorticity takes from it
+@pytest.mark.parametrize("nx,ny,nz", [(48, 48, 49), (49, 49, 48), (64, 64, 28), (337, 339, 1), (64, 64, 37),
+                                      (54, 53, 53), (64, 64, 38), (390, 391, 1)])
 def test_listed_updates_equal_oracle(nx, ny, nz):
     test_listed_faces_equal_oracle(nx, ny, nz, 0.0)
 
 
-def test_listed_update_with_vorticity_equals_oracle():
-    s = W.glauber3d_setup(nx=49, ny=49, nz=48, xmax=14.0, etamax=7.0, b=9.0, nb_peak=0.3)
+@pytest.mark.parametrize("nx,ny,nz", [(49, 49, 48), (54, 53, 54)])
+def test_listed_update_with_vorticity_equals_oracle(nx, ny, nz):
+    s = W.glauber3d_setup(nx=nx, ny=ny, nz=nz, xmax=14.0, etamax=7.0, b=9.0, nb_peak=0.3)
     h, o = capi.GpuHydro(s), P.OracleRun(s, vorticity=True)
     h.enable_vorticity()
     for _ in range(2):

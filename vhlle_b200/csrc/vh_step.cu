@@ -23,11 +23,12 @@ namespace vh {
 
 // resident blocks of 128 threads per SM, from sweeps (us per step at the
 // stated counts): the face kernel 5 / 6 / 7 / 8 blocks 151 / 149 / 146 / 143 on
-// the 101x101x51 event; the update on a list 5 / 6 / 7 / 8: 64 / 54 / 56 / 58
-// there, 149 / 145 / 148 / 156 on 201x201x101, and on every cell of the 2+1D
-// grid of 101x101 4 / 5 / 6: 36 / 37 / 40; the viscous primitives 6 / 7 / 8:
-// 30.8 / 31.5 / 33.1
-constexpr int kFaceMinBlocks = 8, kUpdateMinBlocks = 6, kUpdateFewMinBlocks = 4, kPrimsMinBlocks = 6;
+// the 101x101x51 event; the update on a list 6 / 8 / 10 / 12: 79 / 64 / 75 / 83
+// there (two passes, 30 steps in), 49 / 51 / 60 / 66 early in it, 170 / 156 /
+// 198 / 204 on 201x201x101, 155 / 139 / 150 / 181 on 101x101x51 cells full of
+// matter; on every cell of the 2+1D grid of 101x101 4 / 5 / 6: 36 / 37 / 40;
+// the viscous primitives 6 / 7 / 8: 30.8 / 31.5 / 33.1
+constexpr int kFaceMinBlocks = 8, kUpdateMinBlocks = 8, kUpdateFewMinBlocks = 4, kPrimsMinBlocks = 6;
 
 // -------------------------------------------------------------- updateM
 // Fluid::updateM, src/fld.cpp:384-423 (both passes; out of place).
@@ -2009,9 +2010,10 @@ static int launch_step_ek(const StepArgs& a, cudaStream_t s, LaunchMarker* mk) {
   const bool lists = face_lists(g, bs);
   const unsigned nface = (unsigned)std::min(fblocks, resident);
   const unsigned rset = 148 * kUpdateMinBlocks * (128u / bs);
-  // the update runs on a list where its blocks do not fit one resident set:
-  // 101x101x51, 4065 blocks of 888, 446 us a step with the list and 463
-  // without; 47x61x23, 516 blocks, 169 with and 161 without
+  // the update runs on a list where its blocks do not fit one resident set
+  // (1184): 101x101x51, 4065 blocks, 446 us a step with the list and 463
+  // without; 47x61x23, 516 blocks, 169 with and 161 without; 61x61x31, 902
+  // blocks, 80 to 100 % matter, 152 and 173 with, 148 and 156 without
   const bool rows = lists && nb > rset;
   const unsigned nupd = rows ? rset : nb;
   const bool vort = a.vort && a.viscous;
