@@ -137,7 +137,8 @@ def test_root_find_equals_oracle(eos):
 # the faces that can carry a flux are listed where they fill the chip (more
 # than 1184 blocks of 64 faces): sizes on both sides of the line, mostly
 # vacuum, with a filled event and with cells not filled yet (m < 1)
-@pytest.mark.parametrize("nx,ny,nz", [(29, 30, 29), (31, 29, 29), (33, 64, 32), (197, 191, 1), (200, 199, 1)])
+@pytest.mark.parametrize("nx,ny,nz", [(29, 29, 29), (29, 30, 29), (31, 29, 29), (33, 64, 32), (197, 191, 1),
+                                      (200, 199, 1)])
 @pytest.mark.parametrize("nb", [0.0, 0.3])
 def test_listed_faces_equal_oracle(nx, ny, nz, nb):
     if nz > 1:

@@ -59,7 +59,7 @@ def test_gpu_dbeta_equals_reference_fixture(name):
 @pytest.mark.parametrize("case", [
     ("glauber_41x41x21", lambda: W.small_glauber3d(41, 21, seed=3, b=6.0), 5),
     ("glauber_nb_33x33x17", lambda: W.glauber3d_nb_setup(33, 33, 17, eos=W.nb_table(200, 20)), 4),
-    # EoSChiral: the k_vort_T / k_vort_ops instantiations of the chiral class
+    # EoSChiral: k_visc_prims keeps the temperatures that the rows divide by, per EoS class
     ("glauber_nb_chiral_25x25x13", lambda: W.glauber3d_nb_setup(25, 25, 13, eos=W.chiral_eos()), 4),
 ], ids=lambda c: c[0])
 def test_gpu_dbeta_equals_oracle(case):

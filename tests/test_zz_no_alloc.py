@@ -74,8 +74,13 @@ def _noalloc_step(L, setup, eos_d, dev, tau):
 
 @pytest.mark.parametrize("make", [lambda: W.small_glauber3d(21, 11),
                                   lambda: W.gubser_setup(nx=31, ny=31),
-                                  lambda: W.glauber3d_nb_setup(17, 17, 9, eos=W.chiral_eos())],
-                         ids=["viscous_21x21x11", "gubser_31x31", "chiral_nb_17x17x9"])
+                                  lambda: W.glauber3d_nb_setup(17, 17, 9, eos=W.chiral_eos()),
+                                  # the faces are listed above 25,216 cells in 3D: just below, above, the most
+                                  lambda: W.glauber3d_setup(29, 29, 29),
+                                  lambda: W.glauber3d_setup(29, 30, 29),
+                                  lambda: W.glauber3d_nb_setup(32, 32, 32, eos=W.chiral_eos())],
+                         ids=["viscous_21x21x11", "gubser_31x31", "chiral_nb_17x17x9", "viscous_29x29x29",
+                              "viscous_29x30x29", "chiral_nb_32x32x32"])
 def test_noalloc_step_matches_the_context_step_twice(make):
     torch = pytest.importorskip("torch")
     setup = make()
