@@ -1743,13 +1743,20 @@ vh_status vh_enable_vorticity(vh_ctx* ctx, int on) {
   VH_CUDA(ctx, cudaSetDevice(ctx->device));
   vh::VortDev& v = ctx->vort;
   if (on && !v.dbeta) {
-    vh_status st;
-    if ((st = dalloc(ctx, &v.dbeta, (size_t)16 * N)) || (st = dalloc(ctx, &v.TD, (size_t)N)) ||
-        (st = dalloc(ctx, &v.TB, (size_t)N)) || (st = dalloc(ctx, &v.TC, (size_t)N)) ||
-        (st = dalloc(ctx, &v.val, (size_t)18 * N)) || (st = dalloc(ctx, &v.R, (size_t)2 * N)) ||
-        (st = dalloc(ctx, &v.flag, (size_t)N)) || (st = dalloc(ctx, &v.last, (size_t)5 * N)) ||
-        (st = dalloc(ctx, &v.agg, (size_t)5 * vh::vort_scan_blocks(N))))
-      return st;
+    // one allocation, so that a refused one leaves nothing half made
+    const size_t ints = 5 * (size_t)N + 5 * (size_t)vh::vort_scan_blocks(N);
+    double* buf = nullptr;
+    const vh_status st = dalloc(ctx, &buf, 39 * (size_t)N + (ints + 1) / 2 + ((size_t)N + 7) / 8);
+    if (st) return st;
+    v.dbeta = buf;
+    v.TD = v.dbeta + 16 * N;
+    v.TB = v.TD + N;
+    v.TC = v.TB + N;
+    v.val = v.TC + N;
+    v.R = v.val + 18 * N;
+    v.last = reinterpret_cast<int*>(v.R + 2 * N);
+    v.agg = v.last + 5 * N;
+    v.flag = reinterpret_cast<unsigned char*>(v.R + 2 * N + (ints + 1) / 2);
     // Cell::enableVorticity, src/cll.h:167-170: dbeta starts at zero
     VH_CUDA(ctx, cudaMemsetAsync(v.dbeta, 0, sizeof(double) * 16 * N, ctx->stream));
   }
