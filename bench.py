@@ -76,13 +76,15 @@ COMPULSORY_B = 288  # bytes per cell-update: Q[7] + pi[10] + Pi, read + write
 # Algorithmic bytes of each kernel: the fields a launch must read and write
 # once (stencil neighbours come from cache), per cell with matter (the packed
 # list's count, nactive, read from the device every step) and per grid cell:
-# the vacuum costs the face list Q_t and, in the predictor, its rows' copies.
+# the vacuum costs the face list Q_t and, in the predictor, its rows' copies,
+# which the face list makes where the update runs on a list, else the update.
 KERNEL_BYTES = {  # (per listed cell, per grid cell)
     "k_update_m": (0, 48),      # m[3] in, m[3] out
     "k_face": (360, 8),         # per direction Q or Qh [7] + m in, face flux [7] out; Q_t
     "k_update": (336, 0),       # 3 face fluxes [21] + Q/Qh [7] in, 2 x [7] out
     "k_ghost": (0, 0),          # boundary planes only
-    "k_visc_prims": (152, 0),   # Qh [7] in, prims [8] + [4] out
+    "k_visc_prims": (352, 0),   # index, Q, Qh [14], prims [8], m [3] in; e, u [5],
+                                # thermodynamics [9], u [4], index out
     "k_visc_update": (288, 8),  # prims [4], piH [10], PiH, m [3], flux [4], Q [7] in; Q [7] out; e
     "k_is_relax": (492, 0),     # index, e and v [4], thermodynamics [6], B and C [9], u [5],
                                 # pi, Pi [11] in; pi0, piH0, Pi0, PiH0 [22], flux [4] out
@@ -90,6 +92,11 @@ KERNEL_BYTES = {  # (per listed cell, per grid cell)
                                 # pi, piH, Pi, PiH, vcc [23], flux [4] out
 }
 VACUUM_COPY_B = 84  # per empty cell and pass: Q [7] in, Qh, Qprev [14] out, in one of the two
+UPDATE_LIST_BLOCKS = 148 * 8  # the update runs on a list above this many blocks of 128 cells
+
+
+def vacuum_copier(cells):
+    return "k_face" if -(-cells // 128) > UPDATE_LIST_BLOCKS else "k_update"
 
 
 def kernel_alg_bytes(prof, cells, steps, nactive):
@@ -100,16 +107,17 @@ def kernel_alg_bytes(prof, cells, steps, nactive):
         if k in KERNEL_BYTES:
             listed, grid = KERNEL_BYTES[k]
             out[k] = n * (listed * nactive / steps + float(grid) * cells)
-    if "k_face" in out:
-        out["k_face"] += prof["k_face"][0] * VACUUM_COPY_B * (cells - nactive / steps)
+    k = vacuum_copier(cells)
+    if k in out:
+        out[k] += prof[k][0] * VACUUM_COPY_B * (cells - nactive / steps)
     return out
 
 
-def kernel_bytes_rule(k):
+def kernel_bytes_rule(k, cells):
     if k not in KERNEL_BYTES:
         return ""
     rule = "%d B x listed cells + %d B x cells" % KERNEL_BYTES[k]
-    return rule + (" + %d B x empty cells" % VACUUM_COPY_B if k == "k_face" else "")
+    return rule + (" + %d B x empty cells" % VACUUM_COPY_B if k == vacuum_copier(cells) else "")
 
 
 # the persistent per-cell state a step reads or leaves for the next one (the
@@ -403,7 +411,7 @@ def run_reference_arm(args):
         "config": {"workload": WORKLOAD % ("x".join(map(str, args.grid))),
                    "path": "reference C++ Hydro::performStep + Fluid::outputSurface every %d steps"
                            % SURF_EVERY},
-        "cpu_baseline": {"value": value, "unit": UNIT, "cores": nproc, "kind": kind,
+        "cpu_baseline": {"value": value, "unit": UNIT, "cores": nproc, "kind": "reference",
                          "cpu_model": cpu_model(),
                          "sample": "%d processes, each stepping its own copy of the event (seed %d, "
                                    "surface every %d steps) for up to %d steps or %.0f s; %.1f s wall"
@@ -864,7 +872,7 @@ def main():
                 "traffic": None,
                 "alg_bytes_per_launch": alg, "avg_launch_ms": avg_s * 1e3,
                 "active_cells_per_step": nactive / args.steps,
-                "alg_bytes_rule": kernel_bytes_rule(dname)}
+                "alg_bytes_rule": kernel_bytes_rule(dname, cells)}
     # FP64 co-roofline: the dominant kernel's and the whole step's FP64
     # operations (ncu counts of the same launches) over their CUDA-event
     # time, against a cuBLAS DGEMM measured now
@@ -1011,7 +1019,7 @@ def main():
                        "parallelism": "events%d" % ws,
                        "vorticity": bool(args.vorticity),
                        "l2": "inputs larger than L2 (%.0f MB of resident fields)" % (
-                           cells * 8 * 127 / 1e6)},
+                           cells * 1049 / 1e6)},
             "roofline": roofline, "step_roofline": step_roofline, "fp64_roofline": fp64_roofline,
             "kernels": kernels,
             "e2e": e2e, "cpu_baseline": cpu, "batched_mlp": bmlp, "batch_2d": batch2d,
