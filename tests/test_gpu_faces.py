@@ -135,8 +135,9 @@ def test_root_find_equals_oracle(eos):
 
 
 # the faces that can carry a flux are listed where they fill the chip (more
-# than 1184 blocks of 64 faces): sizes on both sides of the line, mostly
-# vacuum, with a filled event and with cells not filled yet (m < 1)
+# than 1184 blocks of 64 faces, 1776 in 2+1D, and there with a table only):
+# sizes on both sides of the line, mostly vacuum, with a filled event and with
+# cells not filled yet (m < 1)
 @pytest.mark.parametrize("nx,ny,nz", [(29, 29, 29), (29, 30, 29), (31, 29, 29), (33, 64, 32), (197, 191, 1),
                                       (200, 199, 1)])
 @pytest.mark.parametrize("nb", [0.0, 0.3])
@@ -144,9 +145,9 @@ def test_listed_faces_equal_oracle(nx, ny, nz, nb):
     if nz > 1:
         s = W.glauber3d_setup(nx=nx, ny=ny, nz=nz, xmax=14.0, etamax=7.0, b=9.0, nb_peak=nb)
     else:
-        if nb:
-            pytest.skip("one 2+1D form")
         s = W.gubser_setup(nx, ny)
+        if nb:  # the conformal flow's state under a table
+            s.eos = W.nb_table(400, 40)
         s.dt = 0.2 * min(s.grid.dx, s.grid.dy)
         x, y, _ = s.grid.coords()
         far = (np.hypot(*np.meshgrid(x, y)) > 2.5).reshape(-1)
@@ -171,6 +172,11 @@ def test_listed_faces_equal_oracle(nx, ny, nz, nb):
                                       (54, 53, 53), (64, 64, 38), (390, 391, 1)])
 def test_listed_updates_equal_oracle(nx, ny, nz):
     test_listed_faces_equal_oracle(nx, ny, nz, 0.0)
+
+
+@pytest.mark.parametrize("nx,ny", [(238, 238), (239, 238), (337, 339), (390, 391)])
+def test_listed_faces_and_updates_in_2d_equal_oracle(nx, ny):
+    test_listed_faces_equal_oracle(nx, ny, 1, 0.3)
 
 
 @pytest.mark.parametrize("nx,ny,nz", [(49, 49, 48), (54, 53, 54)])

@@ -1333,7 +1333,7 @@ vh_status vh_launches_per_step(vh_ctx* ctx, int* n) {
   // update_m, 2 x (face list, faces, update), a ghost copy; the viscous four
   // (prims, relaxation, advection, update) and their ghost copy, the five of
   // the vorticity; the MLP guess
-  int k = 1 + 2 * (vh::face_lists(ctx->g, 128) ? 3 : 2) + 1 + (ctx->viscous ? 5 : 0) +
+  int k = 1 + 2 * (vh::face_lists(ctx->g, 128, ctx->eos.kind) ? 3 : 2) + 1 + (ctx->viscous ? 5 : 0) +
           (ctx->viscous && ctx->vort_on ? 5 : 0) + (ctx->mlp ? 1 : 0);
   *n = k;
   return VH_OK;

@@ -1989,8 +1989,21 @@ static long long face_resident(int bs) { return 148LL * kFaceMinBlocks * (128 / 
 // of latencies, and the lists (a kernel more in it, and the emptiest warps
 // of a grid that leaves the chip idle anyway) do not pay: 101x101x1, 320
 // blocks of 1184, 48 us a step with lists and 39 without; 47x61x23, 3093
-// blocks, 192 with and 223 without.
-bool face_lists(const Geo& g, int bs) { return face_blocks(g, bs) > face_resident(bs); }
+// blocks, 192 with and 223 without.  Two directions in place of three gain
+// less for the same two list kernels: on 201x201x1, 1264 blocks, an event takes
+// 120 us viscous and 50.5 ideal with lists, 119 and 47.8 without, on 251x251x1,
+// 1970 blocks, 129 and 54, 141 and 63.
+// A grid without empty cells is slower with lists in every case, and the host
+// cannot tell.  The conformal EoS in 2+1D, whose root finds are the cheapest,
+// is used for such flow (Gubser's): without lists full grids of 251x251 and
+// 401x401 take 63 and 134 us and not 71 and 154 (79 and 137 were 301's and
+// 401's before there were lists), events, mostly vacuum, 56 and 101 and not 48
+// and 75 (69 and 106).
+bool face_lists(const Geo& g, int bs, int eos_kind) {
+  if (g.nz == 1)
+    return eos_kind != 0 && face_blocks(g, bs) > face_resident(bs) * 3 / 2;
+  return face_blocks(g, bs) > face_resident(bs);
+}
 
 
 const char* const kKernelNames[KK_COUNT] = {
@@ -2007,7 +2020,7 @@ static int launch_step_ek(const StepArgs& a, cudaStream_t s, LaunchMarker* mk) {
   const unsigned nb128 = nblk(g.N, 128);
   // one resident set of blocks for the faces
   const long long fblocks = face_blocks(g, bs), resident = face_resident(bs);
-  const bool lists = face_lists(g, bs);
+  const bool lists = face_lists(g, bs, a.eos.kind);
   const unsigned nface = (unsigned)std::min(fblocks, resident);
   const unsigned rset = 148 * kUpdateMinBlocks * (128u / bs);
   // the update runs on a list where its blocks do not fit one resident set
