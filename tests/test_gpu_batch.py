@@ -132,6 +132,45 @@ def test_gpu_stage_batched_equals_events_alone(with_mlp):
         mlp.close()
 
 
+@pytest.mark.parametrize("viscous", [False, True])
+def test_gpu_stage_batched_conformal_2d_equals_events_alone(viscous):
+    """The conformal EoS in 2+1D takes no face lists in the stage-batched form:
+    full flow, flow with empty cells, and an event of a table class beside
+    them, at sides that leave remainders of a block."""
+    from vhlle_b200.capi import Batch, GpuHydro
+
+    def events():
+        out = []
+        for nx, ny, cut in ((21, 21, None), (33, 31, 2.5), (5, 6, None), (64, 4, 1.0), (29, 37, 2.0)):
+            s = W.gubser_setup(nx, ny)
+            s.dt = 0.2 * min(s.grid.dx, s.grid.dy)
+            if cut is not None:
+                x, y, _ = s.grid.coords()
+                far = (np.hypot(*np.meshgrid(x, y)) > cut).reshape(-1)
+                s.Q = s.Q.reshape(7, -1).copy()
+                s.Q[:, far] = 0.
+                s.m = np.where(far, 0., s.m.reshape(-1))
+            s.tr = dict(s.tr, etaS0=0.1 if viscous else 0.0, zetaS0=0.0)
+            out.append(s)
+        out[-1].eos = W.make_cs2_table()
+        return out
+    hs = [GpuHydro(s) for s in events()]
+    b = Batch(hs)
+    b.set_mode(True)
+    for _ in range(3):
+        b.advance()
+    assert b.sync() == 0
+    for k, s in enumerate(events()):
+        h = GpuHydro(s)
+        h.step(3)
+        bad = compare_states(hs[k].get_state(), h.get_state())
+        assert not bad, (k, bad)
+        h.close()
+    b.close()
+    for h in hs:
+        h.close()
+
+
 def test_gpu_stage_batched_needs_one_class():
     """Events of different viscosity (the ideal Gubser flow beside viscous
     ones) cannot share stage launches: set_mode(True) is refused and the

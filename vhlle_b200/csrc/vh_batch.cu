@@ -211,7 +211,7 @@ vh_status capture_stages(vh_batch* b, const std::vector<int>& nsub, cudaGraphExe
       d.eos = c->eos;
       d.eos.vguess = c->mlp ? c->vguess : nullptr;
       d.tr = c->tr;
-      d.f = c->f;
+      d.f = vh::batch_fields(c->f, c->g, c->eos.kind);
       if (j & 1) std::swap(d.f.m, d.f.m2);
       d.clk = c->clk;
       d.viscous = c->viscous;

@@ -189,6 +189,9 @@ cudaError_t step_kernels_setup();
 // Whether launch_step lists the faces that can carry a flux (two launches
 // more) on this grid, with bs threads per block.
 bool face_lists(const Geo& g, int bs, int eos_kind);
+// An event's fields in the stage-batched form, without its lists where it
+// takes none.
+Fields batch_fields(const Fields& f, const Geo& g, int eos_kind);
 // Enqueues one performStep on stream s, and tau += dt on a.tick; returns the
 // number of launches.
 // Leaves the updated fill fractions in f.m2 (the caller swaps m and m2).
