@@ -1996,9 +1996,8 @@ static long long face_resident(int bs) { return 148LL * kFaceMinBlocks * (128 / 
 // A grid without empty cells is slower with lists in every case, and the host
 // cannot tell.  The conformal EoS in 2+1D, whose root finds are the cheapest,
 // is used for such flow (Gubser's): without lists full grids of 251x251 and
-// 401x401 take 63 and 134 us and not 71 and 154 (79 and 137 were 301's and
-// 401's before there were lists), events, mostly vacuum, 56 and 101 and not 48
-// and 75 (69 and 106).
+// 401x401 take 63 and 134 us and not 71 and 154 (70 and 137 in the form before
+// the lists), events, mostly vacuum, 56 and 101 and not 48 and 75 (69 and 106).
 bool face_lists(const Geo& g, int bs, int eos_kind) {
   if (g.nz == 1)
     return eos_kind != 0 && face_blocks(g, bs) > face_resident(bs) * 3 / 2;
